@@ -420,7 +420,6 @@ struct mgp_solver {
     double* gm_red = nullptr;
     int gm_m = 0;
     size_t gm_vec = 0, gm_ld = 0;
-    std::vector<SweepTma> tma;   // per level, for the fused sweep
     // MGP_FLAG_MIXED: FP32 copies of the grid-path levels 0 .. dc-1
     struct Lv32 {
         int nx = 0, ny = 0;
@@ -428,7 +427,7 @@ struct mgp_solver {
         DF32 e{}, e2{}, r{}, w{}, invd{};
     };
     std::vector<Lv32> lv32;
-    std::vector<SweepTma> tma32;
+    std::vector<LevelMaps> maps, maps32;   // per grid-path level, for the sweeps of large levels
     Arena32 fixed32, state32;
     // V-cycles captured as CUDA graphs, keyed by their arguments and by which
     // buffer holds e on each grid-path level when the cycle starts
@@ -649,7 +648,7 @@ int build_fp32_levels(mgp_solver* s) {
     }
     RC(s->fixed32.commit(st));
     RC(s->state32.commit(st));
-    s->tma32.assign(s->dc, SweepTma{});
+    s->maps32.assign(s->dc, LevelMaps{});
     for (int d = 0; d < s->dc; ++d) {
         const Lv& L = s->lv[d];
         auto& M = s->lv32[d];
@@ -667,7 +666,7 @@ int build_fp32_levels(mgp_solver* s) {
             CK(launch_round_bf16(M.g.yy, L.nx, L.ny + 1, 0, st));
             CK(launch_round_bf16(M.invd, L.nx, L.ny, 0, st));
         }
-        sweep_tma_prepare(&s->tma32[d], M.e, M.e2, M.r, M.invd, M.g, M.nx, M.ny);
+        sweep_maps_prepare(&s->maps32[d], M.e, M.e2, M.r, M.invd, M.g, M.nx, M.ny);
     }
     return MGP_OK;
 }
@@ -885,10 +884,10 @@ int solver_build(mgp_solver* s, const mgp_box* valid, const mgp_geo* geo, const 
             s->gctl.wait_ns = kGridWaitNsDefault;
         }
     }
-    s->tma.assign(md + 1, SweepTma{});
+    s->maps.assign(s->dc, LevelMaps{});
     for (int d = 0; d < s->dc; ++d) {
         Lv& L = s->lv[d];
-        if (L.e2.p) sweep_tma_prepare(&s->tma[d], L.e, L.e2, L.r, L.invd, L.g, L.nx, L.ny);
+        if (L.e2.p) sweep_maps_prepare(&s->maps[d], L.e, L.e2, L.r, L.invd, L.g, L.nx, L.ny);
     }
     if (mixed(s)) RC(build_fp32_levels(s));
     std::vector<int> ref(2 * (md + 1), 0);
@@ -938,22 +937,11 @@ int smooth_body(mgp_solver* s, int d, int nu) {
             CK(launch_dd_colour(L.e, L.w, L.invd, L.g, L.nx, L.ny, 4.0 / 5.0, 1, st));
         }
     } else if (L.e2.p && sweep_fusable(L.bc)) {
-        // on small levels two sweeps per launch where the level allows it
-        // (the same bits as two launches)
-        const bool pairs = sweep_pair_ok(&s->tma[d], L.bc);
         for (int k = 0; k < nu;) {
-            if (pairs && nu - k >= 2) {
-                CK(launch_sweep9_pair(L.e, L.e2, L.r, L.invd, L.g, L.bc, 1, L.nx, L.ny, 1.0, &s->tma[d], s->d_status,
-                                      st));
-                k += 2;
-            } else {
-                CK(launch_sweep9(L.e, L.e2, L.r, L.invd, L.g, L.bc, 1, L.nx, L.ny, 1.0, &s->tma[d], s->d_status,
-                                 st));
-                k += 1;
-            }
-            const DF t = L.e;
-            L.e = L.e2;
-            L.e2 = t;
+            const SweepPlan p = sweep_plan<double>(L.nx, L.ny, L.bc, nu - k, &s->maps[d]);
+            CK(launch_sweep9(L.e, L.e2, L.r, L.invd, L.g, L.bc, 1, L.nx, L.ny, 1.0, p, 1, &s->maps[d], s->d_status, st));
+            k += p.k;
+            std::swap(L.e, L.e2);
         }
     } else {
         for (int k = 0; k < nu; ++k) CK(launch_gs_sweep(L.e, L.r, L.invd, L.g, L.bc, 1, L.nx, L.ny, 1.0, st));
@@ -1079,19 +1067,15 @@ int vcycle32(mgp_solver* s, int d, int numcycles, int nd, int nu, int nb) {
                 }
                 return MGP_OK;
             }
-            // on small levels two sweeps per launch where the level allows it
-            // (the same bits as two launches; half the launches and loads)
-            const bool pairs = sweep_pair_ok(&s->tma32[d], F.bc);
             for (int k = 0; k < nu_;) {
-                if (pairs && nu_ - k >= 2) {
-                    CK(launch_sweep9_pair(L.e, L.e2, L.r, L.invd, L.g, F.bc, 1, L.nx, L.ny, 1.0, &s->tma32[d],
-                                          s->d_status, st));
-                    k += 2;
-                } else {
-                    CK(launch_sweep9(L.e, L.e2, L.r, L.invd, L.g, F.bc, 1, L.nx, L.ny, 1.0, &s->tma32[d],
-                                     s->d_status, st));
-                    k += 1;
-                }
+                // the BF16 study rounds what a kernel writes: after two sweeps
+                // where 32 x 32 tiles are at most two an SM, else after each
+                const long t32 = (long)((L.nx + 31) / 32) * ((L.ny + 31) / 32);
+                const int left = !(b16 && d >= 1) ? nu_ - k : std::min(nu_ - k, t32 <= 296 ? 2 : 1);
+                const SweepPlan p = sweep_plan<float>(L.nx, L.ny, F.bc, left, &s->maps32[d]);
+                CK(launch_sweep9(L.e, L.e2, L.r, L.invd, L.g, F.bc, 1, L.nx, L.ny, 1.0, p, 1, &s->maps32[d],
+                                 s->d_status, st));
+                k += p.k;
                 std::swap(L.e, L.e2);
                 CK(round16(L.e, d, L.nx, L.ny, 1));
             }
@@ -1557,7 +1541,7 @@ int solver_solve(mgp_solver* s, int which, mgp_array* phi, mgp_array* rhs, const
     CK(cudaEventRecord(s->ev1, st));
     CK(cudaStreamSynchronize(st));
     if (status == MGP_OK && dstat)
-        status = (dstat == DST_TIMEOUT) ? MGP_ETIMEOUT : (dstat == DST_MISALIGNED) ? MGP_ECUDA : MGP_EDIVERGED;
+        status = (dstat == DST_TIMEOUT) ? MGP_ETIMEOUT : MGP_EDIVERGED;
     if (status == MGP_OK && (s->flags & MGP_FLAG_REPORT_MAXITER) && !diverged && !(relres[iters] <= tol))
         status = MGP_EMAXITER;
     if (rep) {
@@ -1582,7 +1566,6 @@ int solver_solve(mgp_solver* s, int which, mgp_array* phi, mgp_array* rhs, const
             for (int k = 0; k <= iters; ++k) rep->relres[k] = relres[k];
     }
     if (status == MGP_ETIMEOUT) return set_err(status, "a device wait ran out of its iteration limit");
-    if (status == MGP_ECUDA) return set_err(status, "misaligned shared-memory window in the sweep");
     if (status == MGP_EMAXITER) return set_err(status, "maxiters reached before the tolerance");
     if (status) return set_err(status, "non-finite residual");
     return MGP_OK;
@@ -1816,20 +1799,21 @@ bool fill_one_phase(const BCd& b, int do_neum) {   // no side's fill reads anoth
     return true;
 }
 
+// A level's sweep jobs: one sweep per launch, two per launch, and levels of a
+// single tile, whose launch makes the whole smoothing call in place.
 template <class T>
-struct SweepGroups {   // a level's sweep jobs by tile width, and those that sweep twice per launch
-    Table<SweepJobT<T>> w32, w64, w32k2;
+struct SweepGroups {
+    Table<SweepJobT<T>> one, two, all;
 };
 
 template <class T>
-void add_sweep_job(SweepGroups<T>& sg, const SweepTma& t, const DFT<T>& e, const DFT<T>& e2, const DFT<T>& r,
-                   const DFT<T>& invd, const GeoT<T>& g, const BCd& b, int nx, int ny, bool pairs) {
+void add_sweep_job(SweepGroups<T>& sg, const LevelMaps& m, const DFT<T>& e, const DFT<T>& e2, const DFT<T>& r, const DFT<T>& invd,
+                   const GeoT<T>& g, const BCd& b, int nx, int ny, bool pairs) {
     SweepJobT<T> J;
     std::memset(&J, 0, sizeof J);
-    const bool a_is_e = (const void*)e.p == t.pa;
-    const bool k2 = pairs && t.ok2;   // the level's two-sweep descriptors exist
-    J.m[0] = k2 ? (a_is_e ? t.ma2 : t.mb2) : (a_is_e ? t.ma : t.mb);
-    J.m[1] = k2 ? (a_is_e ? t.mb2 : t.ma2) : (a_is_e ? t.mb : t.ma);
+    const bool a_is_e = (const void*)e.p == m.pa;
+    J.m[0] = a_is_e ? m.a : m.b;
+    J.m[1] = a_is_e ? m.b : m.a;
     J.buf[0] = e;
     J.buf[1] = e2;
     J.rhs = r;
@@ -1838,11 +1822,18 @@ void add_sweep_job(SweepGroups<T>& sg, const SweepTma& t, const DFT<T>& e, const
     J.b = b;
     J.nx = nx;
     J.ny = ny;
-    J.gx = cdiv(nx, t.tx);
-    J.gy = cdiv(ny, 32);
-    J.part = make_int4(nx / J.gx, nx % J.gx, ny / J.gy, ny % J.gy);
-    J.s0 = 0;
-    (k2 ? sg.w32k2 : t.tx == 64 ? sg.w64 : sg.w32).push(J, J.gx * J.gy);
+    // one tile: the whole call in a launch; `pairs`: two sweeps a launch on small
+    // levels; else one sweep with the large shape's tiles
+    const SweepPlan p = sweep_plan<T>(nx, ny, b, 2, &m);
+    J.in_place = p.gx * p.gy == 1;
+    if (J.in_place || (pairs && p.k == 2)) {
+        J.gx = p.gx;
+        J.gy = p.gy;
+        (J.in_place ? sg.all : sg.two).push(J, J.gx * J.gy);
+    } else {
+        J.tiles = sweep_large_tiles<T>(nx, ny);
+        sg.one.push(J, J.tiles.total);
+    }
 }
 
 // Everything one V-cycle iteration launches, for one set of active problems.
@@ -1923,7 +1914,7 @@ void build_plan(Plan& P, const std::vector<mgp_solver*>& ss, const std::vector<i
             const int cbx = cdiv(C.nx, 32), cby = cdiv(C.ny, 8);
             if (mx) {
                 auto& L = s->lv32[d];
-                add_sweep_job(P.sw32[d], s->tma32[d], L.e, L.e2, L.r, L.invd, L.g, F.bc, L.nx, L.ny, pairs);
+                add_sweep_job(P.sw32[d], s->maps32[d], L.e, L.e2, L.r, L.invd, L.g, F.bc, L.nx, L.ny, pairs);
                 P.fpre32[d].push(FillJob<float>{L.e, L.g, F.bc, L.nx, L.ny, 1, 0}, fblk);
                 if (next_grid) {
                     auto& N = s->lv32[d + 1];
@@ -1940,7 +1931,7 @@ void build_plan(Plan& P, const std::vector<mgp_solver*>& ss, const std::vector<i
                     P.pro3264[d].push(ProlongJob<float, double>{L.e, C.e, C.nx, C.ny, rx, ry, cbx}, cbx * cby);
                 }
             } else {
-                add_sweep_job(P.sw64[d], s->tma[d], F.e, F.e2, F.r, F.invd, F.g, F.bc, F.nx, F.ny, pairs);
+                add_sweep_job(P.sw64[d], s->maps[d], F.e, F.e2, F.r, F.invd, F.g, F.bc, F.nx, F.ny, pairs);
                 P.fpre64[d].push(FillJob<double>{F.e, F.g, F.bc, F.nx, F.ny, 1, 0}, fblk);
                 P.res64[d].push(ResidJob<double, double>{F.e, F.r, F.g, F.bc, C.r, C.e, C.invd, F.nx, F.ny, C.nx, C.ny,
                                                          rx, ry, gbx},
@@ -1979,8 +1970,8 @@ void build_plan(Plan& P, const std::vector<mgp_solver*>& ss, const std::vector<i
 
 template <class F>
 void for_tables(Plan& P, F f) {
-    for (auto& g : P.sw64) { f(g.w32); f(g.w64); f(g.w32k2); }
-    for (auto& g : P.sw32) { f(g.w32); f(g.w64); f(g.w32k2); }
+    for (auto& g : P.sw64) { f(g.one); f(g.two); f(g.all); }
+    for (auto& g : P.sw32) { f(g.one); f(g.two); f(g.all); }
     for (auto& t : P.fpre64) f(t);
     for (auto& t : P.fpre32) f(t);
     for (auto& t : P.fpost64) f(t);
@@ -2034,13 +2025,13 @@ int upload_plan(Plan& P, Lockstep* ls, cudaStream_t st) {
 // 4, so every job's correction ends in its first buffer).
 template <class T>
 int sweeps(SweepGroups<T>& g, int n, Lockstep* ls, cudaStream_t st) {
-    for (int k = 0; k < n; ++k) {
-        CK(launch_sweep9_jobs<T>(g.w32.dj, g.w32.dp, g.w32.n(), g.w32.blocks(), 32, 1, k & 1, ls->status, st));
-        CK(launch_sweep9_jobs<T>(g.w64.dj, g.w64.dp, g.w64.n(), g.w64.blocks(), 64, 1, k & 1, ls->status, st));
-    }
-    for (int k = 0; k < n / 2; ++k)
-        CK(launch_sweep9_jobs<T>(g.w32k2.dj, g.w32k2.dp, g.w32k2.n(), g.w32k2.blocks(), 32, 2, k & 1, ls->status,
+    for (int k = 0; k < n; ++k)
+        CK(launch_sweep9_jobs<T>(g.one.dj, g.one.dp, g.one.n(), g.one.blocks(), 1, 0, k & 1, ls->status,
                                  st));
+    for (int k = 0; k < n / 2; ++k)
+        CK(launch_sweep9_jobs<T>(g.two.dj, g.two.dp, g.two.n(), g.two.blocks(), 2, 1, k & 1, ls->status,
+                                 st));
+    if (n > 0) CK(launch_sweep9_jobs<T>(g.all.dj, g.all.dp, g.all.n(), g.all.blocks(), n, 1, 0, ls->status, st));
     return MGP_OK;
 }
 
@@ -2100,8 +2091,8 @@ void lockstep_free(Lockstep* ls) {
 // Whether the lockstep path serves these solvers with these counts: the MG
 // stationary V-cycle (no Krylov or GMRES flags), one coarse visit per level,
 // even smoothing counts (so every phase but the sweeps finds each level's
-// correction in its first buffer), every level swept with TMA descriptors, no
-// periodic side and a Dirichlet side (no mean removal), bottoms that fit one
+// correction in its first buffer), every level's sweep descriptors, no periodic
+// side and a Dirichlet side (no mean removal), bottoms that fit one
 // CTA, and one precision for all.
 bool lockstep_ok(const std::vector<mgp_solver*>& ss, int numcycles, int nd, int nu) {
     if (ss.empty() || numcycles != 1 || (nd & 1) || (nu & 1) || nd < 0 || nu < 0) return false;
@@ -2118,8 +2109,7 @@ bool lockstep_ok(const std::vector<mgp_solver*>& ss, int numcycles, int nd, int 
         }
         if (!diri) return false;
         for (int d = 0; d < s->dc; ++d) {
-            const SweepTma& t = mx ? s->tma32[d] : s->tma[d];
-            if (!t.ok || !s->lv[d].e2.p || !sweep_fusable(s->lv[d].bc)) return false;
+            if (!(mx ? s->maps32[d] : s->maps[d]).ok || !s->lv[d].e2.p || !sweep_fusable(s->lv[d].bc)) return false;
         }
     }
     return true;
@@ -2285,7 +2275,7 @@ int lockstep_vcycle(const std::vector<mgp_solver*>& ss, Lockstep* ls, mgp_array*
         CK(cudaMemcpy(&dstat, ss[p]->d_status, sizeof(int), cudaMemcpyDeviceToHost));
         if (!dstat) dstat = sweep_status;
         if (status[p] == MGP_OK && dstat)
-            status[p] = (dstat == DST_TIMEOUT) ? MGP_ETIMEOUT : (dstat == DST_MISALIGNED) ? MGP_ECUDA : MGP_EDIVERGED;
+            status[p] = (dstat == DST_TIMEOUT) ? MGP_ETIMEOUT : MGP_EDIVERGED;
         if (status[p] == MGP_OK && (ss[p]->flags & MGP_FLAG_REPORT_MAXITER) && !diverged[p] &&
             !(hist[p][iters[p]] <= tol))
             status[p] = MGP_EMAXITER;
@@ -2307,7 +2297,6 @@ int lockstep_vcycle(const std::vector<mgp_solver*>& ss, Lockstep* ls, mgp_array*
         if (status[p] && !first) first = status[p];
     }
     if (first == MGP_ETIMEOUT) return set_err(first, "a device wait ran out of its iteration limit");
-    if (first == MGP_ECUDA) return set_err(first, "misaligned shared-memory window in the sweep");
     if (first == MGP_EMAXITER) return set_err(first, "maxiters reached before the tolerance");
     if (first) return set_err(first, "non-finite residual");
     return MGP_OK;
@@ -2647,14 +2636,15 @@ int mgp_relax_gs(const mgp_box* valid, mgp_array* phi, const mgp_array* rhs, con
         if (rscale == 0.0) rscale = 1.0;
     }
     const bool fused = sweep_fusable(b);
-    for (int it = 1; it <= maxiters; ++it) {
-        if (fused) {
-            CK(launch_sweep9(p, p2, f, d, g, b, homog, nx, ny, omega, nullptr, nullptr, c.st));
-            const DF t = p;
-            p = p2;
-            p2 = t;
+    for (int it = 0; it < maxiters;) {
+        if (fused) {   // several sweeps a launch where no norm is wanted between them
+            const SweepPlan sp = sweep_plan<double>(nx, ny, b, tol > 0.0 ? 1 : maxiters - it, nullptr);
+            CK(launch_sweep9(p, p2, f, d, g, b, homog, nx, ny, omega, sp, 0, nullptr, nullptr, c.st));
+            it += sp.k;
+            std::swap(p, p2);
         } else {
             CK(launch_gs_sweep(p, f, d, g, b, homog, nx, ny, omega, c.st));
+            ++it;
         }
         if (tol > 0.0) {
             RC(resnorm(&h));

@@ -19,9 +19,8 @@ enum RedKind { RED_SUMSQ = 0, RED_MAXABS = 1, RED_DOT = 2, RED_JSUM = 3, RED_ABS
 // sees the cause, not a later consequence.
 enum DevStatus {
     DST_OK = 0,
-    DST_TIMEOUT = 2,      // a bounded device wait (TMA tile barrier, grid barrier) ran out
+    DST_TIMEOUT = 2,      // a bounded device wait (tile loads, grid barrier) ran out
     DST_NONFINITE = 3,    // a non-finite residual in a device-side solve (bottom BiCGStab)
-    DST_MISALIGNED = 4,   // the sweep's shared-memory window was not 128-byte aligned
 };
 #ifdef __CUDACC__
 __device__ __forceinline__ void set_status(int* s, int v) {
@@ -136,29 +135,39 @@ cudaError_t launch_apply(const DF& out, const DF& phi, const DF& rhs, const Geo&
                          int nx, int ny, int mode, int jscale, cudaStream_t st);
 cudaError_t launch_gs_sweep(const DF& phi, const DF& rhs, const DF& invd, const Geo& g, const BCd& b, int homog,
                             int nx, int ny, double omega, cudaStream_t st);
-// One sweep in a single launch, reading pin and writing pout (mgp_sweep.cu).
-// Sides must be DIRI, NEUM or PERIODIC (sweep_fusable).
+// Whether the one-launch sweep serves these sides: DIRI, NEUM or PERIODIC.
 bool sweep_fusable(const BCd& b);
-// TMA descriptors of the seven fields one sweep stages; phi element (i,j) is
-// map coordinate (i - pcb, j - prb), the operands' (i,j) is (i,j).
-struct SweepMaps {
-    CUtensorMap pin, rhs, invd, xx, xy, yx, yy;
-    int pcb, prb;
-};
 // ---- lockstep batches -------------------------------------------------- //
 // One launch runs the same phase of many problems.  Each launch has a job
 // table and pre[0..njobs]: job k owns blocks [pre[k], pre[k + 1]) of a 1-D
 // grid of pre[njobs] blocks (a block finds its job by binary search).
-// One level's sweep: phi in buf[s0 ^ flip] (descriptors m[s0 ^ flip]),
-// written to the other buffer.
+// One sweep's tiles of a large level: regions of gx x gy tiles (a balanced
+// partition in pairs of cells), numbered from `first`; inner: away from the
+// domain's sides.
+struct SweepTiles {
+    struct Region {
+        int x0, x1, y0, y1, gx, gy, first, inner;
+        int px, rx, py, ry;   // pairs of cells a tile, and tiles with one more, along x and y
+    };
+    int n, total;
+    Region r[5];
+};
+// TMA descriptors of the seven fields a large sweep stages; element (i,j) at
+// coordinates (i,j).
+struct SweepMaps {
+    CUtensorMap phi, rhs, invd, xx, xy, yx, yy;
+};
+// One level's sweep: phi in buf[flip], written to the other buffer; in_place
+// (a level that is one tile): phi in buf[0], swept there.  gx x gy tiles of the
+// small shape, or the large shape's tiles.
 template <class T>
 struct alignas(64) SweepJobT {
     SweepMaps m[2];
     DFT<T> buf[2], rhs, invd;
     GeoT<T> g;
     BCd b;
-    int4 part;   // (nx / gx, nx % gx, ny / gy, ny % gy)
-    int nx, ny, gx, gy, s0;
+    SweepTiles tiles;
+    int nx, ny, gx, gy, in_place;
 };
 // fill_ghosts of one field.
 template <class T>
@@ -212,44 +221,44 @@ struct DirectJob {
     int nx, ny;
 };
 
-// Descriptors for sweeping one level with phi in either of its two buffers.
-struct SweepTma {
-    SweepMaps ma, mb;
-    const void *pa = nullptr, *pb = nullptr, *rhs = nullptr, *invd = nullptr, *xx = nullptr;
-    int tx = 32;   // tile width the descriptors' boxes are cut for
-    bool ok = false;
-    SweepMaps ma2, mb2;   // boxes for two sweeps per launch (small FP32 levels)
-    bool ok2 = false;
+// How one launch sweeps a level: k sweeps over gx x gy tiles of the small
+// shape, or one sweep in the large shape (mgp_sweep.cu).
+struct SweepPlan {
+    int k, gx, gy;
+    bool small;
 };
-// Builds the descriptors when the arrays allow it (16-byte aligned bases and
-// pitches, phi with a ghost layer and pitch >= nx + 3); else t->ok = false
-// and the sweep stages with cp.async.
-void sweep_tma_prepare(SweepTma* t, const DF& ea, const DF& eb, const DF& rhs, const DF& invd, const Geo& g, int nx,
-                       int ny);
-void sweep_tma_prepare(SweepTma* t, const DF32& ea, const DF32& eb, const DF32& rhs, const DF32& invd,
-                       const Geo32& g, int nx, int ny);
-// status (nullable) receives DST_TIMEOUT if a CTA's staging never completed,
-// DST_MISALIGNED if the shared-memory window was not 128-byte aligned
-// (neither is expected).
+template <class T>
+SweepTiles sweep_large_tiles(int nx, int ny);
+// A level's descriptors with phi in either of its two buffers.  Built when the
+// arrays allow it (16-byte aligned bases and pitches), else ok stays false.
+struct LevelMaps {
+    SweepMaps a, b;
+    const void *pa = nullptr, *pb = nullptr, *rhs = nullptr, *invd = nullptr, *xx = nullptr;
+    bool ok = false;
+};
+void sweep_maps_prepare(LevelMaps* m, const DF& ea, const DF& eb, const DF& rhs, const DF& invd, const Geo& g, int nx,
+                        int ny);
+void sweep_maps_prepare(LevelMaps* m, const DF32& ea, const DF32& eb, const DF32& rhs, const DF32& invd,
+                        const Geo32& g, int nx, int ny);
+// The next launch's sweeps when `left` are still to do: 1 <= k <= left.  maps:
+// the level's, or nullptr (a caller's arrays).
+template <class T>
+SweepPlan sweep_plan(int nx, int ny, const BCd& b, int left, const LevelMaps* maps);
+// p.k sweeps of a level in one launch, reading pin and writing pout (two
+// buffers; the same one is fine when the plan is one tile), with ghosts filled
+// at the start of each sweep.  The bits of p.k launches of one sweep.
+// dependent: launch as a programmatic dependent of the kernel ahead; the faces
+// and invd must not be written by that kernel.  maps as for sweep_plan.  status
+// (nullable) receives DST_TIMEOUT if a tile's loads never arrived (not expected).
 cudaError_t launch_sweep9(const DF& pin, const DF& pout, const DF& rhs, const DF& invd, const Geo& g, const BCd& b,
-                          int homog, int nx, int ny, double omega, const SweepTma* tma, int* status,
-                          cudaStream_t st);
+                          int homog, int nx, int ny, double omega, const SweepPlan& p, int dependent,
+                          const LevelMaps* maps, int* status, cudaStream_t st);
 cudaError_t launch_sweep9(const DF32& pin, const DF32& pout, const DF32& rhs, const DF32& invd, const Geo32& g,
-                          const BCd& b, int homog, int nx, int ny, double omega, const SweepTma* tma, int* status,
-                          cudaStream_t st);
-// Two sweeps in one launch on a level whose descriptors allow it
-// (sweep_pair_ok: small levels of 32-wide tiles, no periodic side): the
-// result of two launch_sweep9 calls, bit for bit, written to pout.
-bool sweep_pair_ok(const SweepTma* tma, const BCd& b);
-cudaError_t launch_sweep9_pair(const DF32& pin, const DF32& pout, const DF32& rhs, const DF32& invd, const Geo32& g,
-                               const BCd& b, int homog, int nx, int ny, double omega, const SweepTma* tma,
-                               int* status, cudaStream_t st);
-cudaError_t launch_sweep9_pair(const DF& pin, const DF& pout, const DF& rhs, const DF& invd, const Geo& g,
-                               const BCd& b, int homog, int nx, int ny, double omega, const SweepTma* tma,
-                               int* status, cudaStream_t st);
+                          const BCd& b, int homog, int nx, int ny, double omega, const SweepPlan& p, int dependent,
+                          const LevelMaps* maps, int* status, cudaStream_t st);
 // Lockstep launches: jobs and pre in device memory (pre[njobs] blocks in all).
 template <class T>
-cudaError_t launch_sweep9_jobs(const SweepJobT<T>* jobs, const int* pre, int njobs, int nblocks, int tx, int k,
+cudaError_t launch_sweep9_jobs(const SweepJobT<T>* jobs, const int* pre, int njobs, int nblocks, int k, int small,
                                int flip, int* status, cudaStream_t st);
 template <class T>
 cudaError_t launch_fill_jobs(const FillJob<T>* jobs, const int* pre, int njobs, int nblocks, int phases,

@@ -1,50 +1,49 @@
-// mgp_sweep.cu -- one Gauss-Seidel sweep of the mapped 9-point operator in a
-// single launch (relax_gs, poisson2d.f90:1460-1988, in the device order).
+// mgp_sweep.cu -- Gauss-Seidel sweeps of the mapped 9-point operator, one or
+// several per launch (relax_gs, poisson2d.f90:1460-1988, in the device order).
 //
-// The sweep reads phi from `pin` and writes the swept field to `pout` (two
-// buffers), so no CTA ever reads a value another CTA has already replaced.
-// Each CTA owns one tile of a balanced partition of the grid (tiles at most
-// TX x TY and, when there is more than one, at least TX/2 x TY/2, so every
-// corner's neighbourhood lies inside the tile that owns the corner: with
-// g = ceil(n / TX) tiles along a side, n / g lies in [TX/2, TX] for n > TX
-// and equals TX only when g divides n).
+// A launch reads phi from `pin` and writes the swept field to `pout` (two
+// buffers), so no CTA reads a value another CTA has already replaced; a level
+// that one CTA covers may be swept in place.  A CTA owns a tile of a balanced
+// partition of the grid and works on a window of cells around it.  A sweep's
+// sub-passes are
+//   * the sweep-start ghost fill (P2:1556);
+//   * the four colours (0,0),(1,1),(1,0),(0,1) over interior cells;
+//   * along the domain's non-periodic sides the edge cells colour by colour,
+//     then the four corners.
+// Every pass runs on the whole window: what it computes near the window's rim
+// from cells the window does not hold is wrong, and moves inward by a known
+// number of cells a pass, never into the tile.  With K sweeps a window has 4 K +
+// 2 columns left of its tile, 4 K right and 4 K + 2 rows below and above (tiles
+// start at even cells; tests/test_sweep_halo.py walks the dependences of every
+// partition shape).  So K sweeps in a launch give the bits of K launches, and
+// the result depends on neither the tiling nor K.
 //
-// A CTA first stages everything its tile's update reads -- phi with its
-// halo, rhs, the inverse diagonal and the four metric face arrays, each on
-// exactly the region the sub-passes touch -- into shared memory with
-// coalesced loads, applies the sweep-start ghost fill there (P2:1556), then
-// runs the sweep's sub-passes from shared memory only, on shrinking regions:
-//   * the four colours (0,0),(1,1),(1,0),(0,1) over interior cells -- the
-//     stencil reaches one cell, so pass c is exact on the tile grown by
-//     (3 - c + E) cells;
-//   * on tiles that touch a non-periodic side, the boundary pass: edge cells
-//     colour by colour (away from corners a colour along an edge reads only
-//     neighbours of the colour updated just before it, so one extra cell of
-//     halo suffices, E = 2), then the four corners in turn.
-// The halo cells are recomputed by every CTA that needs them, with the same
-// operations in the same order, so the result is bit-identical to running the
-// sub-passes over the whole grid one after another.  The same argument lets
-// one launch run K sweeps (K = 2 on small levels, whose sweeps last about
-// one CTA's latency): with a halo of K times the one-sweep halo, sweep s of K
-// works on the tile grown by (K - 1 - s)(4 + E) cells, and the tile comes out
-// as after K launches, bit for bit.
+// The operator lives in registers.  A thread owns a 2 x 2 block of cells -- one
+// of each colour -- and keeps their face coefficients, inverse diagonals and
+// right-hand sides (36 values) through all K sweeps.  Shared memory holds phi
+// alone, as four planes, one per colour (i mod 2, j mod 2), so a colour pass
+// reads its five neighbours outside the block with consecutive lanes on
+// consecutive words.  (With the whole operator in shared memory at one word a
+// cell, a colour reads 19 values an update at stride two: 640 of the ~900
+// cycles of a pass with one CTA on the SM were replayed wavefronts, and the
+// edge cells, one generic routine for four sides, another 0.5 us a colour.)
 //
-// Staging: on the solver's own arrays (aligned, with spare columns) one
-// thread issues seven TMA tile loads (five on the wide FP32 tiles;
-// cp.async.bulk.tensor.2d) of the CTA's
-// window of each field, completing on one mbarrier; elsewhere (caller arrays
-// of any pitch and alignment) the threads stage with cp.async.
-//
-// The kernel is compiled for FP64 fields (the solver's arithmetic; the
-// update is gs9's, bit for bit) and for FP32 fields (the grid levels of the
-// mixed-precision V-cycle), where each thread updates two interior cells at
-// once in packed FP32x2 arithmetic with fused multiply-adds (gs9_pair).  The
-// result depends on neither the tiling nor the launch: the same inputs give
-// the same bits.
+// Two shapes, chosen by sweep_plan.  Levels whose sweeps last one CTA's latency
+// take several sweeps a launch, with four warps of their own for the sides:
+// measured per sweep of an n^2 level, FP32 / FP64, before (operator in shared
+// memory, two sweeps a launch) and now: 128^2 8.4 / 8.3 -> 2.7 / 3.7 us, 256^2
+// 8.5 / 8.3 -> 2.9 / 5.3 us, 512^2 8.7 / 11 -> 5.7 / 10 us.  Large levels take
+// one sweep a launch by persistent CTAs that load the next tile while they
+// sweep one: 1024^2 17.2 / 32 -> 13.5 / 22 us, 2048^2 41 / 88 -> 38 / 72 us
+// (0.55 / 0.58 of the copy rate by the 8 words a cell of a sweep).  They are
+// bound by the barriers between colour passes (5 of 18 cycles between a warp's
+// issues), not by the bytes.
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
+#include <algorithm>
 #include <mutex>
+#include <type_traits>
 
 #include "mgp_kernels.cuh"
 
@@ -52,123 +51,647 @@ namespace mgp {
 
 namespace {
 
-constexpr int kTY = 32;
-constexpr int kH1 = 6;   // phi halo of one sweep: 4 for the colour passes + E = 2 for the boundary pass
-// A CTA gives up on its tile loads after kWaitLimit polls or kWaitNs, far
-// above any real wait (microseconds); each poll sleeps up to kSuspendNs.
-constexpr long kWaitLimit = 1L << 22;
-constexpr unsigned long long kWaitNs = 200000000ull;
-constexpr unsigned kSuspendNs = 20000;
-
-// Tile and shared-memory window of one field type and tile width: 32 x 32
-// tiles (FP64: two CTAs of 114 KB per SM; FP32: three of 59 KB) and, for
-// FP32 levels large enough to fill the GPU, 64 x 32 tiles, which spread each
-// thread's fixed work over more cells and recompute a smaller share of halo.
-// The wide tiles stage five arrays, not seven: rhs and the inverse diagonal,
-// read once per update and only at the updated cell, come from global memory
-// there, so the window (70 KB) leaves room for three CTAs per SM -- a tile's
-// colour passes are latency-bound, and more CTAs in flight hide it.  All
-// staged arrays share one
-// window -- origin (pox, poy) with pox the column at or below tile corner - kH
-// that is a multiple of kAlign (a 16-byte boundary, as TMA needs), pitch PW --
-// so one offset addresses a cell in every array: phi and the cell operands
-// at o, the west/east x-faces at o and o + 1, the south/north y-faces at o
-// and o + PW.  The operands are needed on tile + (3 + E) <= tile + 5 cells
-// (faces one further), inside the phi footprint tile + kH.
-template <class T, int TX_, int K_ = 1>
-struct Win {
-    static constexpr int TX = TX_;
-    static constexpr int kH = K_ * kH1;   // phi halo of K_ sweeps per launch
-    static constexpr int kAlign = 16 / (int)sizeof(T);   // 2 doubles, 4 floats
-    static constexpr int PW = (TX + 2 * kH + (kAlign - 1) + kAlign - 1) / kAlign * kAlign;   // 46 / 48 / 80
-    static constexpr int PH = kTY + 2 * kH;                                                        // 44
-    static constexpr int kA = (PW * PH * (int)sizeof(T) + 127) / 128 * 128 / (int)sizeof(T);     // 128-B aligned
-    static constexpr bool kRI = !(sizeof(T) == 4 && TX_ == 64);   // rhs and inverse diagonal staged
-    static constexpr int NA = kRI ? 7 : 5;                          // staged arrays
-    static constexpr int oF = kA, oD = 2 * kA;                      // (when kRI)
-    static_assert(oD == oF + kA, "rhs and inverse diagonal adjacent");
-    static constexpr int oXX = (kRI ? 3 : 1) * kA, oXY = oXX + kA, oYX = oXX + 2 * kA, oYY = oXX + 3 * kA;
-    static constexpr int oBarBytes = NA * kA * (int)sizeof(T);   // the TMA mbarrier (8 bytes)
-    static constexpr size_t kSmemBytes = (size_t)oBarBytes + 16;
-    static constexpr unsigned kBoxBytes = PW * PH * sizeof(T);
-    // threads: the wide tiles' colour passes hold 256 to 333 cell pairs (up to
-    // 389 on tiles at the domain edge), so 12 warps cover them, and three
-    // CTAs of 384 threads leave 56 registers a thread
-    static constexpr int kThreads = kRI ? 512 : 384;
-    static_assert(K_ == 1 || TX_ == 32, "two sweeps per launch: 32-wide tiles only");
-    // CTAs per SM the window and the thread count allow
-    static constexpr int kMinBlocks = (int)((228 * 1024) / (kSmemBytes + 1024)) < 2048 / kThreads
-                                          ? (int)((228 * 1024) / (kSmemBytes + 1024))
-                                          : 2048 / kThreads;
+// A CTA's shape: NI warps own the window's blocks, LB blocks (2 LB columns) a
+// row, 32 / LB rows a warp; with kSep four more warps serve the domain's sides.
+template <class T_, int NI_, int LB_, bool kSep_, int kMinBlocks_>
+struct Shape {
+    using T = T_;
+    static constexpr int NI = NI_, LB = LB_, kMinBlocks = kMinBlocks_;
+    static constexpr bool kSep = kSep_;
+    static constexpr int RB = 32 / LB;                       // block rows a warp
+    static constexpr int kThreads = 32 * (NI + (kSep ? 4 : 0));
+    static constexpr int WX = 2 * LB, WY = 2 * NI * RB;      // window
+    static constexpr int P = LB + 2;                         // blocks per plane row, one spare either side
+    static constexpr int PS = P * (NI * RB + 2);             // one plane
+    static_assert(WX <= 64 && WY <= 64 && NI >= 4, "a warp holds a side, two cells a lane");
+    // largest tile for K sweeps a launch
+    static constexpr int tx(int k) { return WX - (8 * k + 2); }
+    static constexpr int ty(int k) { return WY - (8 * k + 4); }
 };
 
-static_assert(Win<double, 32>::PW == 46 && Win<float, 32>::PW == 48 && Win<float, 64>::PW == 80, "window pitch");
-static_assert(Win<double, 32>::kMinBlocks == 2 && Win<float, 32>::kMinBlocks == 3 && Win<float, 64>::kMinBlocks == 3,
-              "CTAs per SM");
-static_assert(Win<float, 32, 2>::PW == 60 && Win<float, 32, 2>::PH == 56 && Win<float, 32, 2>::kMinBlocks == 2,
-              "two-sweep window");
-static_assert(Win<double, 32, 2>::PW == 58 && Win<double, 32, 2>::kMinBlocks == 1, "two-sweep FP64 window");
+// Programmatic dependent launch: a grid launched with the programmatic
+// serialization attribute may start before the grid ahead of it in the stream
+// has finished; griddepcontrol.wait returns once that grid has completed and
+// its writes are visible (at once when there is none), and launch_dependents
+// lets the next such grid start as SM resources free up.
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void allow_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// Barrier of the four warps that serve the sides, and of the whole CTA (the
+// two roles reach it at different places in the code).
+__device__ __forceinline__ void boundary_sync() {
+    __syncwarp();
+    asm volatile("bar.sync 1, 128;" ::: "memory");
+}
+__device__ __forceinline__ void cta_sync() {
+    __syncwarp();
+    asm volatile("bar.sync 0;" ::: "memory");
+}
 
 template <class T>
-struct SLoadT {
-    const T* c;
-    int ld;
-    __device__ __forceinline__ T operator()(int di, int dj) const { return c[di + dj * ld]; }
+struct Pair;
+template <>
+struct Pair<float> {
+    using type = float2;
+};
+template <>
+struct Pair<double> {
+    using type = double2;
 };
 
-// phi at the start of the sweep: the staged copy where it holds (i,j), else
-// global memory (the far side of a periodic domain).
-template <class T, int PW>
-struct PinLoad {
+// Elements p[0] (if a) and p[1] (if b; b implies a).  kVec: p is aligned to a
+// pair.  kConst: the memory is not written while the kernel runs or by the
+// kernel ahead of it.
+template <bool kVec, bool kConst, class T>
+__device__ __forceinline__ void load_pair(const T* p, bool a, bool b, T& v0, T& v1) {
+    using V = typename Pair<T>::type;
+    if (kVec && b) {
+        const V v = kConst ? __ldg(reinterpret_cast<const V*>(p)) : *reinterpret_cast<const V*>(p);
+        v0 = v.x;
+        v1 = v.y;
+    } else {
+        if (a) v0 = kConst ? __ldg(p) : p[0];
+        if (b) v1 = kConst ? __ldg(p + 1) : p[1];
+    }
+}
+
+// A plane index is the sum of a term of the window column x and one of the row
+// y, -1 <= x <= WX, -1 <= y <= WY.
+template <class C>
+__device__ __forceinline__ int x_term(int x) {
+    return (x & 1) * C::PS + (x >> 1);
+}
+template <class C>
+__device__ __forceinline__ int y_term(int y) {
+    return (y & 1) * 2 * C::PS + (y >> 1) * C::P + C::P + 1;
+}
+
+// The part of the grid a CTA works on.
+struct Window {
+    int ox, oy, wx1, wy1;      // cells [ox, wx1) x [oy, wy1)
+    int X0, X1, Y0, Y1;        // its tile
+    bool xl, xh, yl, yh;       // sides of the domain in the window
+    __device__ __forceinline__ bool any() const { return xl || xh || yl || yh; }
+    // The tile and its halo (cells left, right, below, above), clipped to the grid.
+    __device__ __forceinline__ void set(int x0, int x1, int y0, int y1, int l, int r, int d, int u, int nx, int ny) {
+        X0 = x0, X1 = x1, Y0 = y0, Y1 = y1;
+        ox = max(0, X0 - l), wx1 = min(nx, X1 + r);
+        oy = max(0, Y0 - d), wy1 = min(ny, Y1 + u);
+        xl = ox == 0, xh = wx1 == nx, yl = oy == 0, yh = wy1 == ny;
+    }
+};
+
+// phi at the start of a sweep: the window where it holds (i,j), else global
+// memory (a stored ghost, or the far side of a periodic domain).
+template <class C>
+struct StartLoad {
+    using T = typename C::T;
     const T* s;
-    int pox, poy, pi0, pi1, pj0, pj1;
+    const Window& w;
     DFT<T> pin;
     __device__ __forceinline__ T operator()(int i, int j) const {
-        if (i >= pi0 && i < pi1 && j >= pj0 && j < pj1) return s[(j - poy) * PW + (i - pox)];
+        if (i >= w.ox && i < w.wx1 && j >= w.oy && j < w.wy1) return s[x_term<C>(i - w.ox) + y_term<C>(j - w.oy)];
         return AT(pin, i, j);
     }
 };
 
-// Copy rows [j0,j1) x columns [i0,i1) of a global field into a shared array
-// whose (0,0) is cell (ox, oy) and whose row pitch is w.  Warp w8 takes rows
-// j0 + w8, j0 + w8 + 8, ...; where a row's global and shared addresses have
-// the same 16-byte phase its lanes copy pairs of doubles, else single ones.
-__device__ __forceinline__ void stage(double* s, int w, int ox, int oy, const DF& f, int i0, int i1, int j0, int j1) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    const unsigned sbase = (unsigned)__cvta_generic_to_shared(s);
-    for (int j = j0 + warp; j < j1; j += nw) {
-        const double* g = f.p + (long)j * f.ld + i0;
-        unsigned sa = sbase + (unsigned)(((j - oy) * w + (i0 - ox)) * 8);
-        const int n = i1 - i0;
-        if (n <= 0) continue;
-        if (((unsigned)(uintptr_t)g ^ sa) & 8) {
-            for (int k = lane; k < n; k += 32) cp_async8s(sa + 8 * k, g + k);
-            continue;
-        }
-        int k0 = 0;
-        if (sa & 8) {   // leading single
-            if (lane == 0) cp_async8s(sa, g);
-            k0 = 1;
-        }
-        const int np = (n - k0) >> 1;
-        for (int k = lane; k < np; k += 32) cp_async16s(sa + 8 * (k0 + 2 * k), g + k0 + 2 * k);
-        if (((n - k0) & 1) && lane == 31) cp_async8s(sa + 8 * (n - 1), g + n - 1);   // trailing single
+// What a thread keeps of its 2 x 2 block: x-faces [row][face], y-faces
+// [face][column], inverse diagonal, right-hand side and phi [row][column].
+// FP64: Jgup_xy and Jgup_yx times 1/4 (the first product lap9f forms, so the
+// same bits).  FP32: every face value times its two grid factors (dx^-2, or
+// dx^-1 dy^-1 / 4), one rounding, and the inverse diagonal times omega.
+template <class T>
+struct Block {
+    T xx[2][3], xy[2][3], yx[3][2], yy[3][2], d[2][2], f[2][2], p[2][2];
+};
+
+// The update of the block's cell (CX, CY), an interior cell; s is the block's
+// place in plane 0.
+template <class C, int CX, int CY, class T>
+__device__ __forceinline__ T update(const Block<T>& k, const T* s, T idx, T idy, T om, T om1) {
+    const auto N = [&](int dx, int dy) -> T {   // compile-time dx, dy
+        const int x = CX + dx, y = CY + dy;
+        if (x >= 0 && x <= 1 && y >= 0 && y <= 1) return k.p[y][x];
+        return s[((y & 1) * 2 + (x & 1)) * C::PS + (y >> 1) * C::P + (x >> 1)];
+    };
+    const T p = k.p[CY][CX], pe = N(1, 0), pw = N(-1, 0), pn = N(0, 1), ps = N(0, -1);
+    const T ene = N(1, 1), enw = N(-1, 1), ese = N(1, -1), esw = N(-1, -1);
+    if constexpr (sizeof(T) == 8) {   // lap9f's operations in their order (P2:1768-1771 for the update)
+        const T xfe = k.xx[CY][CX + 1] * (pe - p) * idx + k.xy[CY][CX + 1] * (ene - ese + pn - ps) * idy;
+        const T xfw = k.xx[CY][CX] * (p - pw) * idx + k.xy[CY][CX] * (pn - ps + enw - esw) * idy;
+        const T yfn = k.yy[CY + 1][CX] * (pn - p) * idy + k.yx[CY + 1][CX] * (ene - enw + pe - pw) * idx;
+        const T yfs = k.yy[CY][CX] * (p - ps) * idy + k.yx[CY][CX] * (pe - pw + ese - esw) * idx;
+        const T lphi = (xfe - xfw) * idx + (yfn - yfs) * idy;
+        const T newphi = p + (k.f[CY][CX] - lphi) * k.d[CY][CX];
+        return om * newphi + om1 * p;
+    } else {
+        const T ty = pn - ps, tx = pe - pw;
+        T x = k.xx[CY][CX + 1] * (pe - p);
+        x = __fmaf_rn(k.xx[CY][CX], pw - p, x);
+        x = __fmaf_rn(k.xy[CY][CX + 1], (ene - ese) + ty, x);
+        x = __fmaf_rn(k.xy[CY][CX], (esw - enw) - ty, x);
+        T y = k.yy[CY + 1][CX] * (pn - p);
+        y = __fmaf_rn(k.yy[CY][CX], ps - p, y);
+        y = __fmaf_rn(k.yx[CY + 1][CX], (ene - enw) + tx, y);
+        y = __fmaf_rn(k.yx[CY][CX], (esw - ese) - tx, y);
+        return __fmaf_rn((k.f[CY][CX] - x) - y, k.d[CY][CX], p);
     }
 }
 
-// The same for FP32 fields, one element per copy.
-__device__ __forceinline__ void stage(float* s, int w, int ox, int oy, const DF32& f, int i0, int i1, int j0, int j1) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    const unsigned sbase = (unsigned)__cvta_generic_to_shared(s);
-    for (int j = j0 + warp; j < j1; j += nw) {
-        const float* g = f.p + (long)j * f.ld + i0;
-        const unsigned sa = sbase + (unsigned)(((j - oy) * w + (i0 - ox)) * 4);
-        for (int k = lane; k < i1 - i0; k += 32)
-            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(sa + 4 * k), "l"(g + k));
+// ---- the cells along the domain's sides ------------------------------------ //
+// A warp serves each side the window holds: its ghosts, its edge cells colour
+// by colour and one corner.  A side is described by its tangential direction t
+// (x on the y sides, y on the x sides) and its normal n; the cell formulas are
+// gather9's and lap9f's with t for x and n for y, which on the x sides are the
+// same operations by the symmetry of the operator under exchanging x and y.
+// A lane keeps two neighbouring cells of the side, one of each colour: their
+// operator and the sixteen plane addresses they read.  These passes are a
+// serial chain of single warps (about 4 cycles an instruction), so every
+// instruction that does not depend on phi is made once, before the sweeps.
+//
+// The operator at a side's cells comes from their owners through shared
+// memory: value q of cell a along side t at [(t * kStrip + q) * kAlong + a].
+constexpr int kStrip = 10, kAlong = 64;
+enum { Q_TT1, Q_TT0, Q_TN1, Q_TN0, Q_NN1, Q_NN0, Q_NT1, Q_NT0, Q_D, Q_F };   // 1: the high face, 0: the low face
+
+template <int CX, int CY, class T>
+__device__ __forceinline__ void strip_write(T* q, const Block<T>& k, bool yside) {
+    const T xe = k.xx[CY][CX + 1], xw = k.xx[CY][CX], ce = k.xy[CY][CX + 1], cw = k.xy[CY][CX];
+    const T yn = k.yy[CY + 1][CX], ys = k.yy[CY][CX], dn = k.yx[CY + 1][CX], ds = k.yx[CY][CX];
+    q[Q_TT1 * kAlong] = yside ? xe : yn;
+    q[Q_TT0 * kAlong] = yside ? xw : ys;
+    q[Q_TN1 * kAlong] = yside ? ce : dn;
+    q[Q_TN0 * kAlong] = yside ? cw : ds;
+    q[Q_NN1 * kAlong] = yside ? yn : xe;
+    q[Q_NN0 * kAlong] = yside ? ys : xw;
+    q[Q_NT1 * kAlong] = yside ? dn : ce;
+    q[Q_NT0 * kAlong] = yside ? ds : cw;
+    q[Q_D * kAlong] = k.d[CY][CX];
+    q[Q_F * kAlong] = k.f[CY][CX];
+}
+
+// The corner (kHX, kHY) of the domain, its operator in a y side's strip at q; x
+// and y: plane terms of the ghosts, the side's cells and the next two inward.
+template <bool kHX, bool kHY, class T>
+__device__ __forceinline__ void corner_cell(T* S, const T* q, const int* x, const int* y, const GeoT<T>& g,
+                                            const BCd& b, int homog, int i, int j, T om, T om1) {
+    const T three = T(3.0), half = T(0.5);
+    const T p = S[x[1] + y[1]], a = S[x[2] + y[1]], c = S[x[1] + y[2]], ac = S[x[2] + y[2]];   // a, c: x, y inward
+    const T gx = S[x[0] + y[1]], gy = S[x[1] + y[0]];
+    const T o = three * (p - a) + S[x[3] + y[1]], u = three * (p - c) + S[x[1] + y[3]];   // outward in x, in y
+    const T oc = three * (c - ac) + S[x[3] + y[2]], au = three * (a - ac) + S[x[2] + y[3]];
+    const T ou = half * ((three * (u - au) + S[x[3] + y[0]]) + (three * (o - oc) + S[x[0] + y[3]]));
+    St9T<T> st;
+    st.p = p;
+    st.pe = kHX ? gx : a;
+    st.pw = kHX ? a : gx;
+    st.pn = kHY ? gy : c;
+    st.ps = kHY ? c : gy;
+    st.ee = kHX ? o : a;
+    st.ew = kHX ? a : o;
+    st.en = kHY ? u : c;
+    st.es = kHY ? c : u;
+    const T ni = kHY ? au : ac, si = kHY ? ac : au, no = kHY ? ou : oc, so = kHY ? oc : ou;   // x inward, outward
+    st.ene = kHX ? no : ni;
+    st.enw = kHX ? ni : no;
+    st.ese = kHX ? so : si;
+    st.esw = kHX ? si : so;
+    FacesT<T> fc;
+    fc.xxe = q[Q_TT1 * kAlong];
+    fc.xxw = q[Q_TT0 * kAlong];
+    fc.xye = q[Q_TN1 * kAlong];
+    fc.xyw = q[Q_TN0 * kAlong];
+    fc.yyn = q[Q_NN1 * kAlong];
+    fc.yys = q[Q_NN0 * kAlong];
+    fc.yxn = q[Q_NT1 * kAlong];
+    fc.yxs = q[Q_NT0 * kAlong];
+    const T lphi = lap9f(st, fc, T(g.idx), T(g.idy), i, j, kHX ? RHI : RLO, kHY ? RHI : RLO, b, homog);
+    const T newphi = p + (q[Q_F * kAlong] - lphi) * q[Q_D * kAlong];
+    S[x[1] + y[1]] = om * newphi + om1 * p;
+}
+
+// What a lane keeps of its side (kY: a y side; kHigh: at the high end).
+template <class C, bool kY, bool kHigh>
+struct SideLane {
+    using T = typename C::T;
+    static constexpr int sd = (kY ? S_YLO : S_XLO) + (kHigh ? 1 : 0);
+    bool on, plain, neum;      // the window holds the side; its ghosts follow from three rows; a Neumann side
+    bool ok[2], in[2];         // the lane's cells: edge cells to update, cells of the window
+    int ad[4][4];              // plane index of (column - 1, the two cells, column + 2; ghost, side, one, two inward)
+    int ph[2];                 // the colour in whose turn each cell is
+    T q[2][kStrip], nb[2];     // operators; the Neumann side's boundary fluxes
+    T idt, idn, om, om1;
+
+    __device__ __forceinline__ void place(const Window& w, const GeoT<T>& g, const BCd& b, int homog, int nx, int ny,
+                                          T om_, T om1_) {
+        const int lane = threadIdx.x & 31;
+        on = kY ? (kHigh ? w.yh : w.yl) : (kHigh ? w.xh : w.xl);
+        const Per pr = periodic_of(b);
+        const bool periodic = kY ? (kHigh ? pr.yh : pr.yl) : (kHigh ? pr.xh : pr.xl);
+        plain = !(pr.xl || pr.xh || pr.yl || pr.yh) &&
+                (b.type[sd] == T_NEUM || (b.type[sd] == T_DIRI && homog && b.mode[sd] != M_LAH));
+        neum = b.type[sd] == T_NEUM;
+        const int ot = kY ? w.ox : w.oy, et = kY ? w.wx1 : w.wy1, nt = kY ? nx : ny;
+        const int at = kHigh ? (kY ? ny : nx) - 1 : 0, in_ = kHigh ? -1 : 1;
+        const int n = at - (kY ? w.oy : w.ox), a = 2 * lane;
+        const int lo = (kY ? pr.xl : pr.yl) ? 0 : 1, hi = (kY ? pr.xh : pr.yh) ? nt : nt - 1;   // corners left out
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            const int t = ot + a + c;
+            in[c] = on && t < et;
+            ok[c] = in[c] && !periodic && t >= lo && t < hi;
+            // colours (0,0),(1,1),(1,0),(0,1): the one with this normal parity and tangential parity c
+            ph[c] = kY ? ((at & 1) ? (c ? 1 : 3) : (c ? 2 : 0)) : ((at & 1) ? (c ? 1 : 2) : (c ? 3 : 0));
+        }
+#pragma unroll
+        for (int t = 0; t < 4; ++t)
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                const int tt = a - 1 + t, nn = n + (r - 1) * in_;
+                ad[t][r] = kY ? x_term<C>(tt) + y_term<C>(nn) : x_term<C>(nn) + y_term<C>(tt);
+            }
+        idt = T(kY ? g.idx : g.idy);
+        idn = T(kY ? g.idy : g.idx);
+        om = om_;
+        om1 = om1_;
+    }
+    // The operators, once their owners have written the strips.
+    __device__ __forceinline__ void take(const T* strips, const Window& w, const BCd& b, int homog) {
+        const int lane = threadIdx.x & 31, side = (kY ? 0 : 2) + (kHigh ? 1 : 0);
+#pragma unroll
+        for (int c = 0; c < 2; ++c)
+#pragma unroll
+            for (int v = 0; v < kStrip; ++v) {
+                q[c][v] = T(0.0);
+                if (ok[c]) q[c][v] = strips[(side * kStrip + v) * kAlong + 2 * lane + c];
+                if (v == Q_TN1 || v == Q_TN0 || v == Q_NT1 || v == Q_NT0) q[c][v] = q[c][v] * T(0.25);
+            }
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            const int t = (kY ? w.ox : w.oy) + 2 * lane + c;
+            nb[c] = T(0.0);
+            if (neum && ok[c]) nb[c] = T(nbval(b, homog, sd, sd == S_YHI ? b.kyhi : t));
+        }
+    }
+    // A sweep's ghosts (fill_ghosts without do_neum, P2:1556).
+    __device__ __forceinline__ void fill(T* S, const DFT<T>& pin, const Window& w, const BCd& b, int homog, int nx,
+                                         int ny, int sw) const {
+        if (!on) return;
+        if (plain) {
+            if (neum) return;   // as stored
+#pragma unroll
+            for (int c = 0; c < 2; ++c)   // AU:1161-1177, homogeneous
+                if (in[c])
+                    S[ad[1 + c][0]] = -(T(3.0) * S[ad[1 + c][1]]) + S[ad[1 + c][2]] - T(1.0 / 5.0) * S[ad[1 + c][3]];
+        } else if (!(sw > 0 && neum)) {
+            const StartLoad<C> P{S, w, pin};
+            const int lo = kY ? (w.xl ? -1 : w.ox) : w.oy, hi = kY ? (w.xh ? nx + 1 : w.wx1) : w.wy1;
+            const int at = kHigh ? (kY ? ny : nx) : -1;
+            for (int v = lo + (threadIdx.x & 31); v < hi; v += 32) {
+                const int i = kY ? v : at, j = kY ? at : v;
+                S[x_term<C>(i - w.ox) + y_term<C>(j - w.oy)] = sweep_ghost(P, b, homog, nx, ny, i, j);
+            }
+        }
+    }
+    // gs9's update of the lane's cell c.
+    template <int c>
+    __device__ __forceinline__ void cell(T* S) const {
+        const T three = T(3.0);
+        const T p = S[ad[1 + c][1]], i1 = S[ad[1 + c][2]], i2 = S[ad[1 + c][3]], gh = S[ad[1 + c][0]];
+        const T pm = S[ad[c][1]], m1 = S[ad[c][2]], m2 = S[ad[c][3]];
+        const T pp = S[ad[2 + c][1]], p1 = S[ad[2 + c][2]], p2 = S[ad[2 + c][3]];
+        const T x0 = three * (p - i1) + i2, xm = three * (pm - m1) + m2, xp = three * (pp - p1) + p2;
+        const T N0 = kHigh ? x0 : i1, S0 = kHigh ? i1 : x0, Np = kHigh ? xp : p1, Sp = kHigh ? p1 : xp;
+        const T Nm = kHigh ? xm : m1, Sm = kHigh ? m1 : xm, gn = kHigh ? gh : i1, gs = kHigh ? i1 : gh;
+        const T t1 = q[c][Q_TT1] * (pp - p) * idt + q[c][Q_TN1] * (Np - Sp + N0 - S0) * idn;
+        const T t0 = q[c][Q_TT0] * (p - pm) * idt + q[c][Q_TN0] * (N0 - S0 + Nm - Sm) * idn;
+        T n1 = q[c][Q_NN1] * (gn - p) * idn + q[c][Q_NT1] * (Np - Nm + pp - pm) * idt;
+        T n0 = q[c][Q_NN0] * (p - gs) * idn + q[c][Q_NT0] * (pp - pm + Sp - Sm) * idt;
+        if (kHigh) n1 = neum ? nb[c] : n1;
+        else n0 = neum ? nb[c] : n0;
+        const T lphi = (t1 - t0) * idt + (n1 - n0) * idn;
+        const T newphi = p + (q[c][Q_F] - lphi) * q[c][Q_D];
+        S[ad[1 + c][1]] = om * newphi + om1 * p;
+    }
+    // The edge cells colour by colour, then the corners: warps y low, y high, x
+    // low, x high take the corners (low, low), (low, high), (high, low), (high,
+    // high); on a grid of at least 4 x 4 they do not read each other.
+    __device__ __forceinline__ void pass(T* S, const T* strips, const Window& w, const GeoT<T>& g, const BCd& b,
+                                         int homog, int nx, int ny) const {
+#pragma unroll 1
+        for (int c = 0; c < 4; ++c) {
+            if (c == ph[0]) {
+                if (ok[0]) cell<0>(S);
+            } else if (c == ph[1]) {
+                if (ok[1]) cell<1>(S);
+            }
+            boundary_sync();
+        }
+        constexpr bool hx = !kY, hy = kHigh;
+        const Per pr = periodic_of(b);
+        if ((threadIdx.x & 31) == 0 && (hx ? w.xh && !pr.xh : w.xl && !pr.xl) && (hy ? w.yh && !pr.yh : w.yl && !pr.yl)) {
+            const int i = hx ? nx - 1 : 0, j = hy ? ny - 1 : 0;
+            int x[4], y[4];
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                x[r] = x_term<C>(i - w.ox + (r - 1) * (hx ? -1 : 1));
+                y[r] = y_term<C>(j - w.oy + (r - 1) * (hy ? -1 : 1));
+            }
+            corner_cell<hx, hy>(S, strips + (hy ? kStrip * kAlong : 0) + i - w.ox, x, y, g, b, homog, i, j, om, om1);
+        }
+    }
+};
+
+// Calls f with the side of warp v (0-3: y low, y high, x low, x high).
+template <class C, class F>
+__device__ __forceinline__ void with_side(int v, F f) {
+    if (v == 0) f(SideLane<C, true, false>());
+    else if (v == 1) f(SideLane<C, true, true>());
+    else if (v == 2) f(SideLane<C, false, false>());
+    else if (v == 3) f(SideLane<C, false, true>());
+}
+
+// Ghosts no sweep changes, by warps 0-3: a Neumann side's, as stored, and the
+// corners' marker.
+template <class C, class T>
+__device__ __forceinline__ void fixed_ghosts(T* s, const Window& w, const DFT<T>& pin, const BCd& b, int nx, int ny) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (warp >= 4) return;
+    const bool yside = warp < 2, high = warp & 1;
+    const int sd = (warp + 2) & 3;
+    const bool on = warp == 0 ? w.yl : warp == 1 ? w.yh : warp == 2 ? w.xl : w.xh;
+    const int ot = yside ? w.ox : w.oy, et = yside ? w.wx1 : w.wy1;
+    const int at = high ? (yside ? ny : nx) : -1, gt = at - (yside ? w.oy : w.ox);
+    if (on && b.type[sd] == T_NEUM) {
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            const int a = 2 * lane + c;
+            if (ot + a < et) {
+                const T v = yside ? AT(pin, ot + a, at) : AT(pin, at, ot + a);
+                s[yside ? x_term<C>(a) + y_term<C>(gt) : x_term<C>(gt) + y_term<C>(a)] = v;
+            }
+        }
+    }
+    if (on && yside && lane < 2 && (lane ? w.xh : w.xl))
+        s[x_term<C>(lane ? nx - w.ox : -1) + y_term<C>(gt)] = bogus<T>();
+}
+
+// A freshly loaded block made ready: the sides' strips, the scaled coefficients,
+// phi into the planes.  Returns the
+// mask of interior cells (bit q: the block's cell q).
+template <class C, bool kInner, class T>
+__device__ __forceinline__ unsigned settle(Block<T>& k, T* s, T* strips, const Window& w, int kbx, int kby, T idx,
+                                           T idy, T om, const BCd& b, int nx, int ny) {
+    const int i0 = w.ox + 2 * kbx, j0 = w.oy + 2 * kby;
+    if (!kInner && w.any()) {
+        const int yh = ny - 1 - j0, xh = nx - 1 - i0;   // the high side's row / column in this block, if 0 or 1
+        const int sz = kStrip * kAlong;
+        if (w.yl && kby == 0) {
+            strip_write<0, 0>(strips + 2 * kbx, k, true);
+            strip_write<1, 0>(strips + 2 * kbx + 1, k, true);
+        }
+        if (w.yh && yh == 0) {
+            strip_write<0, 0>(strips + sz + 2 * kbx, k, true);
+            strip_write<1, 0>(strips + sz + 2 * kbx + 1, k, true);
+        } else if (w.yh && yh == 1) {
+            strip_write<0, 1>(strips + sz + 2 * kbx, k, true);
+            strip_write<1, 1>(strips + sz + 2 * kbx + 1, k, true);
+        }
+        if (w.xl && kbx == 0) {
+            strip_write<0, 0>(strips + 2 * sz + 2 * kby, k, false);
+            strip_write<0, 1>(strips + 2 * sz + 2 * kby + 1, k, false);
+        }
+        if (w.xh && xh == 0) {
+            strip_write<0, 0>(strips + 3 * sz + 2 * kby, k, false);
+            strip_write<0, 1>(strips + 3 * sz + 2 * kby + 1, k, false);
+        } else if (w.xh && xh == 1) {
+            strip_write<1, 0>(strips + 3 * sz + 2 * kby, k, false);
+            strip_write<1, 1>(strips + 3 * sz + 2 * kby + 1, k, false);
+        }
+    }
+    const T q = T(0.25);
+    if constexpr (sizeof(T) == 8) {
+#pragma unroll
+        for (int a = 0; a < 2; ++a)
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                k.xy[a][c] = k.xy[a][c] * q;
+                k.yx[c][a] = k.yx[c][a] * q;
+            }
+    } else {
+        const T sx = idx * idx, sy = idy * idy, sc = q * idx * idy;
+#pragma unroll
+        for (int a = 0; a < 2; ++a)
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                k.xx[a][c] = k.xx[a][c] * sx;
+                k.xy[a][c] = k.xy[a][c] * sc;
+                k.yx[c][a] = k.yx[c][a] * sc;
+                k.yy[c][a] = k.yy[c][a] * sy;
+            }
+#pragma unroll
+        for (int a = 0; a < 4; ++a) k.d[a >> 1][a & 1] = k.d[a >> 1][a & 1] * om;
+    }
+    T* own = s + (kby + 1) * C::P + kbx + 1;
+    if (kInner) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) own[c * C::PS] = k.p[c >> 1][c & 1];
+        return 15u;
+    }
+    const Per pr = periodic_of(b);
+    const int mi0 = pr.xl ? 0 : 1, mi1 = pr.xh ? nx : nx - 1;   // interior cells
+    const int mj0 = pr.yl ? 0 : 1, mj1 = pr.yh ? ny : ny - 1;
+    unsigned mask = 0;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        const int i = i0 + (c & 1), j = j0 + (c >> 1);
+        if (i < w.wx1 && j < w.wy1) own[c * C::PS] = k.p[c >> 1][c & 1];   // past them there may be ghosts
+        if (i >= mi0 && i < min(mi1, w.wx1) && j >= mj0 && j < min(mj1, w.wy1)) mask |= 1u << c;
+    }
+    return mask;
+}
+
+// The four interior colours, a CTA barrier after each.
+template <class C, class T>
+__device__ __forceinline__ void colours(Block<T>& k, T* own, unsigned mask, T idx, T idy, T om, T om1) {
+    if (mask & 1u) own[0] = k.p[0][0] = update<C, 0, 0>(k, own, idx, idy, om, om1);
+    cta_sync();
+    if (mask & 8u) own[3 * C::PS] = k.p[1][1] = update<C, 1, 1>(k, own, idx, idy, om, om1);
+    cta_sync();
+    if (mask & 2u) own[C::PS] = k.p[0][1] = update<C, 1, 0>(k, own, idx, idy, om, om1);
+    cta_sync();
+    if (mask & 4u) own[2 * C::PS] = k.p[1][0] = update<C, 0, 1>(k, own, idx, idy, om, om1);
+    cta_sync();
+}
+
+// phi of the thread's block, as the sides' passes and ghost fills left it.
+template <class C, class T>
+__device__ __forceinline__ void reload(Block<T>& k, const T* own) {
+#pragma unroll
+    for (int c = 0; c < 4; ++c) k.p[c >> 1][c & 1] = own[c * C::PS];
+}
+
+// The block's cells of the tile, to pout.
+template <bool kVec, class T>
+__device__ __forceinline__ void store_block(const Block<T>& k, const DFT<T>& pout, const Window& w, int i0, int j0) {
+    const bool w0 = i0 >= w.X0 && i0 < w.X1, w1 = w0 && i0 + 1 < w.X1;
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+        const int j = j0 + r;
+        if (j < w.Y0 || j >= w.Y1) continue;
+        T* o = &AT(pout, i0, j);
+        if (kVec && w1) {
+            typename Pair<T>::type v;
+            v.x = k.p[r][0];
+            v.y = k.p[r][1];
+            *reinterpret_cast<typename Pair<T>::type*>(o) = v;
+        } else {
+            if (w0) o[0] = k.p[r][0];
+            if (w1) o[1] = k.p[r][1];
+        }
     }
 }
 
-// ---- TMA staging ---------------------------------------------------------- //
+// The ghost cells next to the tile (the state fill_ghosts leaves: filled at the
+// start of the last sweep), by side warp v.
+template <class C, class T>
+__device__ __forceinline__ void store_ghosts(const T* s, const DFT<T>& pout, const Window& w, int v, int nx, int ny) {
+    if (v < 0 || v >= 4) return;
+    const bool yside = v < 2;
+    if (!(v == 0 ? w.Y0 == 0 : v == 1 ? w.Y1 >= ny : v == 2 ? w.X0 == 0 : w.X1 >= nx)) return;
+    const int lo = yside ? (w.X0 == 0 ? -1 : w.X0) : w.Y0, hi = yside ? (w.X1 >= nx ? nx + 1 : w.X1) : w.Y1;
+    const int at = v == 0 || v == 2 ? -1 : yside ? ny : nx;
+    for (int q = lo + (threadIdx.x & 31); q < hi; q += 32) {
+        const int i = yside ? q : at, j = yside ? at : q;
+        AT(pout, i, j) = s[x_term<C>(i - w.ox) + y_term<C>(j - w.oy)];
+    }
+}
+
+// K sweeps of tile (bx, by) of a level's gx x gy tiles, by one CTA of a shape
+// with kSep.  kVec: every array's rows are aligned to pairs of elements.
+template <class C, bool kVec, class T>
+__device__ __forceinline__ void sweep_tile(const DFT<T>& pin, const DFT<T>& pout, const DFT<T>& rhs,
+                                           const DFT<T>& invd, const GeoT<T>& g, const BCd& b, int homog, int nx,
+                                           int ny, int gx, int gy, double omega, int K, int bx, int by) {
+    __shared__ T s[4 * C::PS];
+    __shared__ T strips[4 * kStrip * kAlong];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    // tile bounds: even, so blocks do not straddle tiles
+    const int hx = (nx + 1) >> 1, hy = (ny + 1) >> 1;
+    Window w;
+    w.set(2 * (bx * hx / gx), min(nx, 2 * ((bx + 1) * hx / gx)), 2 * (by * hy / gy), min(ny, 2 * ((by + 1) * hy / gy)),
+          4 * K + 2, 4 * K, 4 * K + 2, 4 * K + 2, nx, ny);
+    const bool any_side = w.any();
+    const T idx = T(g.idx), idy = T(g.idy), om = T(omega), om1 = T(1.0 - omega);
+    if (warp >= C::NI) {   // the counterpart of the blocks' loop below, with the same CTA barriers
+        with_side<C>(warp - C::NI, [&](auto L) {
+            L.place(w, g, b, homog, nx, ny, om, om1);
+            cta_sync();   // phi and the strips are in place
+            if (any_side) {
+                L.take(strips, w, b, homog);
+                L.fill(s, pin, w, b, homog, nx, ny, 0);
+                cta_sync();
+            }
+#pragma unroll 1
+            for (int sw = 0; sw < K; ++sw) {
+                for (int c = 0; c < 4; ++c) cta_sync();   // the interior colours
+                if (!any_side) continue;
+                L.pass(s, strips, w, g, b, homog, nx, ny);
+                if (sw + 1 < K) {
+                    boundary_sync();
+                    L.fill(s, pin, w, b, homog, nx, ny, sw + 1);
+                }
+                cta_sync();
+            }
+        });
+        store_ghosts<C>(s, pout, w, warp - C::NI, nx, ny);
+        return;
+    }
+    const int kbx = lane % C::LB, kby = warp * C::RB + lane / C::LB;   // the thread's block
+    const int i0 = w.ox + 2 * kbx, j0 = w.oy + 2 * kby;
+    const bool c0 = i0 < w.wx1, c1 = i0 + 1 < w.wx1;
+    T* own = s + (kby + 1) * C::P + kbx + 1;
+    // 1. the operator, constant during a solve: requested before the wait for
+    //    the kernel ahead (the solver launches sweeps as programmatic dependents)
+    Block<T> k = {};
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+        const int j = j0 + r;
+        const bool in = j < w.wy1;
+        const bool f0 = in && i0 <= w.wx1, f1 = in && i0 + 1 <= w.wx1;
+        load_pair<kVec, true>(&AT(g.xx, i0, j), f0, f1, k.xx[r][0], k.xx[r][1]);
+        load_pair<kVec, true>(&AT(g.xy, i0, j), f0, f1, k.xy[r][0], k.xy[r][1]);
+        load_pair<kVec, true>(&AT(invd, i0, j), in && c0, in && c1, k.d[r][0], k.d[r][1]);
+        if (kbx == C::LB - 1 && in && c1) {   // the window's last face has no neighbour lane
+            k.xx[r][2] = __ldg(&AT(g.xx, i0 + 2, j));
+            k.xy[r][2] = __ldg(&AT(g.xy, i0 + 2, j));
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+        const int j = j0 + r;
+        const bool in = j <= w.wy1;
+        load_pair<kVec, true>(&AT(g.yy, i0, j), in && c0, in && c1, k.yy[r][0], k.yy[r][1]);
+        load_pair<kVec, true>(&AT(g.yx, i0, j), in && c0, in && c1, k.yx[r][0], k.yx[r][1]);
+    }
+    grid_dependency_wait();
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+        const int j = j0 + r;
+        const bool in = j < w.wy1;
+        load_pair<kVec, false>(&AT(pin, i0, j), in && c0, in && c1, k.p[r][0], k.p[r][1]);
+        load_pair<kVec, false>(&AT(rhs, i0, j), in && c0, in && c1, k.f[r][0], k.f[r][1]);
+    }
+    if (any_side) fixed_ghosts<C>(s, w, pin, b, nx, ny);
+    // a block's east faces are its neighbour lane's west faces
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+        const T a = __shfl_down_sync(0xffffffffu, k.xx[r][0], 1), c = __shfl_down_sync(0xffffffffu, k.xy[r][0], 1);
+        if (kbx < C::LB - 1) {
+            k.xx[r][2] = a;
+            k.xy[r][2] = c;
+        }
+    }
+    const unsigned mask = settle<C, false>(k, s, strips, w, kbx, kby, idx, idy, om, b, nx, ny);
+    cta_sync();
+    if (any_side) cta_sync();   // 2. the sides' warps fill the first sweep's ghosts
+#pragma unroll 1
+    for (int sw = 0; sw < K; ++sw) {
+        // the boundary pass of the sweep before changed cells their owners hold
+        // in registers, and a block may hold a ghost (an odd side)
+        if (any_side) reload<C>(k, own);
+        colours<C>(k, own, mask, idx, idy, om, om1);   // 3.
+        if (any_side) cta_sync();                      // 4. the sides' cells
+    }
+    if (any_side) reload<C>(k, own);
+    store_block<kVec>(k, pout, w, i0, j0);
+}
+
+// ---- one sweep of a large level -------------------------------------------- //
+// A persistent CTA walks over tiles and, while it sweeps one, has the next
+// one's operands on the way: a thread issues seven TMA tile loads (the window
+// of phi, rhs, the inverse diagonal and the four faces) into one staging buffer
+// that is free again as soon as the threads have taken their blocks into
+// registers, so the loads' latency is off the chain of colour passes and their
+// addresses off the instruction stream (with a cp.async a row and array instead,
+// 690 instructions a thread and tile and 57.7 us at 2048^2 in FP32).
+template <class C>
+struct Stage {
+    using T = typename C::T;
+    static constexpr int kAlign = 16 / (int)sizeof(T);                // a TMA load starts at a multiple of 16 bytes
+    static constexpr int PW = (C::WX + 1 + (kAlign - 2) + kAlign - 1) / kAlign * kAlign;   // the window and a face
+    static constexpr int PH = C::WY + 1;
+    static constexpr int kA = (PW * PH * (int)sizeof(T) + 127) / 128 * 128 / (int)sizeof(T);   // 128-byte aligned
+    static constexpr unsigned kBytes = PW * PH * sizeof(T);
+    enum { A_XX, A_XY, A_YX, A_YY, A_D, A_P, A_F, kArrays };
+    static constexpr size_t kSmem = (size_t)kArrays * kA * sizeof(T) + 128;
+};
+
+// A CTA gives up on its tile loads after kWaitLimit polls or kWaitNs, far
+// above any real wait (microseconds); a poll sleeps up to kSuspendNs.
+constexpr long kWaitLimit = 1L << 22;
+constexpr unsigned long long kWaitNs = 200000000ull;
+constexpr unsigned kSuspendNs = 20000;
+
 __device__ __forceinline__ void mbar_init(unsigned bar, unsigned count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(bar), "r"(count) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
@@ -176,8 +699,6 @@ __device__ __forceinline__ void mbar_init(unsigned bar, unsigned count) {
 __device__ __forceinline__ void mbar_expect_tx(unsigned bar, unsigned bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"(bytes) : "memory");
 }
-// Test phase `parity`; a thread whose phase is not complete sleeps in the
-// instruction until it completes or kSuspendNs pass.
 __device__ __forceinline__ bool mbar_try_wait(unsigned bar, unsigned parity) {
     unsigned ok;
     asm volatile(
@@ -192,29 +713,16 @@ __device__ __forceinline__ unsigned long long global_ns() {
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
     return t;
 }
-// Bounded wait for phase 0 of the barrier (kWaitLimit polls and kWaitNs at
-// most); false if it did not complete.  Between polls the warp sleeps, 32 ns
-// at first and at most 256 ns, so a CTA waiting for its tile takes few issue
-// slots from the CTAs computing beside it.
-__device__ __forceinline__ bool mbar_wait0(unsigned bar) {
+// Bounded wait for the barrier's phase of the given parity; false if it did not complete.
+__device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity) {
+    if (mbar_try_wait(bar, parity)) return true;
     const unsigned long long t0 = global_ns();
-    unsigned nap = 32;
     for (long k = 0; k < kWaitLimit; ++k) {
-        if (mbar_try_wait(bar, 0)) return true;
+        if (mbar_try_wait(bar, parity)) return true;
         if (global_ns() - t0 > kWaitNs) break;
-        __nanosleep(nap);
-        nap = nap < 256 ? 2 * nap : nap;
     }
     return false;
 }
-// Programmatic dependent launch: a grid launched with the programmatic
-// serialization attribute may start before the grid ahead of it in the stream
-// has finished; griddepcontrol.wait returns once that grid has completed and
-// its writes are visible (at once when there is none), and launch_dependents
-// lets the next such grid start as SM resources free up.
-__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void allow_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-
 // One 2-D tile (the map's box) of `map` at element coordinates (x, y); x is a
 // multiple of 16 bytes.
 __device__ __forceinline__ void tma_load_2d(unsigned dst, const CUtensorMap* map, int x, int y, unsigned bar) {
@@ -224,354 +732,241 @@ __device__ __forceinline__ void tma_load_2d(unsigned dst, const CUtensorMap* map
         : "memory");
 }
 
-// Interior colour c on the tile grown by (3 - c + E + G), G the extra grow of
-// an early sweep of a multi-sweep launch: first cell (ci0, cj0), cw cells
-// per row, n cells, and the magic number for k / cw (n <= 37 x 25 and cw <=
-// 37, well inside the exact range of the 24-bit multiply).  Lane
-// c of each group of four computes colour c; every lane then reads all four
-// by shuffle, so a warp spends one divide, not four per thread.
-__device__ __forceinline__ void colour_ranges(int X0, int X1, int Y0, int Y1, int E, int G, int mi0, int mi1,
-                                              int mj0, int mj1, int* ci0, int* cj0, int* ccw, int* cn, unsigned* cm) {
-    const int c = threadIdx.x & 3;
-    const int grow = 3 - c + E + G;
-    int i0 = max(X0 - grow, mi0), i1 = min(X1 + grow, mi1);
-    int j0 = max(Y0 - grow, mj0), j1 = min(Y1 + grow, mj1);
-    i0 += (i0 & 1) != colour_ci(c);
-    j0 += (j0 & 1) != colour_cj(c);
-    const int cw = (i1 - i0 + 1) / 2, ch = (j1 - j0 + 1) / 2;
-    const int n = (cw > 0 && ch > 0) ? cw * ch : 0;
-    const unsigned m = fastdiv24_magic(cw > 0 ? cw : 1);
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        ci0[k] = __shfl_sync(0xffffffffu, i0, k);
-        cj0[k] = __shfl_sync(0xffffffffu, j0, k);
-        ccw[k] = __shfl_sync(0xffffffffu, cw, k);
-        cn[k] = __shfl_sync(0xffffffffu, n, k);
-        cm[k] = __shfl_sync(0xffffffffu, m, k);
-    }
-}
-
-template <class T>
-struct Tile {
-    T* s;   // seven arrays of PW x PH, origin (pox, poy)
-    int pox, poy;
+// The next tile, as the thread that places it leaves it for the others.
+struct NextTile {
+    int t, job, inner;   // t < 0: none
+    Window w;
 };
 
-// One Gauss-Seidel update of (i,j) from shared memory (same operations as gs9).
-// f and d are rhs and the inverse diagonal at (i,j).
-template <class W, class T>
-__device__ __forceinline__ void gs9_tile(const Tile<T>& t, T idx, T idy, const BCd& b, int homog, int i, int j, int xr,
-                                         int yr, T om, T om1, T f, T d) {
-    T* c = t.s + (j - t.poy) * W::PW + (i - t.pox);
-    St9T<T> s;
-    gather9(SLoadT<T>{c, W::PW}, xr, yr, s);
-    FacesT<T> fc;
-    fc.xxw = c[W::oXX]; fc.xxe = c[W::oXX + 1];
-    fc.xyw = c[W::oXY]; fc.xye = c[W::oXY + 1];
-    fc.yys = c[W::oYY]; fc.yyn = c[W::oYY + W::PW];
-    fc.yxs = c[W::oYX]; fc.yxn = c[W::oYX + W::PW];
-    const T lphi = lap9f(s, fc, idx, idy, i, j, xr, yr, b, homog);
-    const T p = c[0];
-    const T newphi = p + (f - lphi) * d;
-    c[0] = om * newphi + om1 * p;
+// Tile t of a level's partition; true for a tile of the inner region, whose
+// whole window lies inside the domain, off its sides.
+__device__ __forceinline__ bool place_tile(const SweepTiles& S, int t, int nx, int ny, Window& w) {
+    int r = 0;
+    while (r + 1 < S.n && t >= S.r[r + 1].first) ++r;
+    const SweepTiles::Region& R = S.r[r];
+    const int q = t - R.first, by = q / R.gx, bx = q - by * R.gx;
+    const int X0 = R.x0 + 2 * (bx * R.px + min(bx, R.rx)), X1 = min(R.x1, X0 + 2 * (R.px + (bx < R.rx)));
+    const int Y0 = R.y0 + 2 * (by * R.py + min(by, R.ry)), Y1 = min(R.y1, Y0 + 2 * (R.py + (by < R.ry)));
+    if (R.inner) w.set(X0, X1, Y0, Y1, 4, 2, 4, 4, nx, ny);
+    else w.set(X0, X1, Y0, Y1, 6, 4, 6, 6, nx, ny);
+    return R.inner;
 }
 
-// Two interior updates at once in packed FP32 arithmetic (add / mul / fma on
-// a pair of floats, one instruction for both lanes): cells a and b of the
-// same colour, each lane the operations of gs9_tile on an interior cell in
-// the same order, except that the seven places where a product is added to
-// another term -- each flux's two terms, the operator's x and y parts, the
-// update p + (f - Lp) d and the relaxation om new + om1 p -- are fused
-// multiply-adds, rounded once.  (The code generator fuses packed multiplies
-// into adds on its own; writing the fused form makes the arithmetic defined
-// by the source.)  Differences are a + b * (-1): an exact product and one
-// rounding, the same as a - b.  Where the colour has an odd number of cells
-// the last thread's b is a itself and only a is written back.
-__device__ __forceinline__ float2 f2add(float2 a, float2 b) { return __fadd2_rn(a, b); }
-__device__ __forceinline__ float2 f2mul(float2 a, float2 b) { return __fmul2_rn(a, b); }
-__device__ __forceinline__ float2 f2fma(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
-__device__ __forceinline__ float2 f2sub(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.f, -1.f), a); }
+// A level as a large sweep's CTA sees it.
+template <class T>
+struct LevelRef {
+    const DFT<T>*pin, *pout;
+    const GeoT<T>* g;
+    const BCd* b;
+    int nx, ny;
+};
 
-// f and d hold rhs and the inverse diagonal at the two cells.
-template <class W>
-__device__ __forceinline__ void gs9_pair(float* a, float* b, bool write_b, float2 f, float2 d, float2 idx, float2 idy,
-                                         float2 om, float2 om1) {
-    constexpr int P = W::PW;
-    const auto L = [a, b](int o) { return make_float2(a[o], b[o]); };
-    const float2 p = L(0), pe = L(1), pw = L(-1), pn = L(P), ps = L(-P);
-    const float2 ene = L(1 + P), enw = L(-1 + P), ese = L(1 - P), esw = L(-1 - P);
-    const float2 q = make_float2(0.25f, 0.25f);
-    // interior cell: ee = pe, ew = pw, en = pn, es = ps (lap9f's four fluxes)
-    const float2 xfe = f2fma(f2mul(L(W::oXX + 1), f2sub(pe, p)), idx,
-                             f2mul(f2mul(f2mul(L(W::oXY + 1), q), f2sub(f2add(f2sub(ene, ese), pn), ps)), idy));
-    const float2 xfw = f2fma(f2mul(L(W::oXX), f2sub(p, pw)), idx,
-                             f2mul(f2mul(f2mul(L(W::oXY), q), f2sub(f2add(f2sub(pn, ps), enw), esw)), idy));
-    const float2 yfn = f2fma(f2mul(L(W::oYY + P), f2sub(pn, p)), idy,
-                             f2mul(f2mul(f2mul(L(W::oYX + P), q), f2sub(f2add(f2sub(ene, enw), pe), pw)), idx));
-    const float2 yfs = f2fma(f2mul(L(W::oYY), f2sub(p, ps)), idy,
-                             f2mul(f2mul(f2mul(L(W::oYX), q), f2sub(f2add(f2sub(pe, pw), ese), esw)), idx));
-    const float2 lphi = f2fma(f2sub(xfe, xfw), idx, f2mul(f2sub(yfn, yfs), idy));
-    const float2 newphi = f2fma(f2sub(f, lphi), d, p);
-    const float2 r = f2fma(om, newphi, f2mul(om1, p));
-    a[0] = r.x;
-    if (write_b) b[0] = r.y;
-}
-
-// The sweep of tile (bx, by) of a level, by one CTA (the body of k_sweep9
-// and of the lockstep batch's k_sweep9_jobs).  m and b may live in kernel
-// parameter space or in global memory.
-template <bool kTma, class T, int TX, int K>
-__device__ __forceinline__ void sweep_tile(const SweepMaps& m, const DFT<T>& pin, const DFT<T>& pout,
-                                           const DFT<T>& rhs, const DFT<T>& invd, const GeoT<T>& g, const BCd& b,
-                                           int homog, int nx, int ny, int4 part, double omega, int* status, int bx,
-                                           int by) {
-    using W = Win<T, TX, K>;
-    extern __shared__ __align__(1024) unsigned char smem_raw[];
-    T* smem = reinterpret_cast<T*>(smem_raw);
-    // tile bounds: part = (nx / gx, nx % gx, ny / gy, ny % gy); the first
-    // nx % gx columns of tiles are one cell wider
-    const int X0 = bx * part.x + min(bx, part.y), X1 = X0 + part.x + (bx < part.y ? 1 : 0);
-    const int Y0 = by * part.z + min(by, part.w), Y1 = Y0 + part.z + (by < part.w ? 1 : 0);
-    const Per pr = periodic_of(b);
-    const bool edge_tile = (!pr.xl && X0 == 0) || (!pr.xh && X1 >= nx) || (!pr.yl && Y0 == 0) || (!pr.yh && Y1 >= ny);
-    const int E = edge_tile ? 2 : 0;
-    const T idx = T(g.idx), idy = T(g.idy);
-    const T om = T(omega), om1 = T(1.0 - omega);
-    Tile<T> t;
-    t.s = smem;
-    t.pox = (X0 - W::kH) & ~(W::kAlign - 1);
-    t.poy = Y0 - W::kH;
-    // one scalar update, rhs and the inverse diagonal from the window or global memory
-    const auto gs = [&](int i, int j, int xr, int yr) {
-        T f, d;
-        if constexpr (W::kRI) {
-            const int o = (j - t.poy) * W::PW + (i - t.pox);
-            f = t.s[o + W::oF];
-            d = t.s[o + W::oD];
-        } else {
-            f = AT(rhs, i, j);
-            d = AT(invd, i, j);
-        }
-        gs9_tile<W>(t, idx, idy, b, homog, i, j, xr, yr, om, om1, f, d);
+// One sweep of the tiles blockIdx.x, blockIdx.x + gridDim.x, ... below total.
+// find(t, job, inner, window) places tile t (job: in, the level of the tile
+// before); level(job) gives its level, maps(job) its descriptors.
+template <class C, class T, class Find, class Level, class Maps>
+__device__ __forceinline__ void sweep_stream(int total, int homog, double omega, int* status, Find find, Level level,
+                                             Maps maps) {
+    using S = Stage<C>;
+    using V = typename Pair<T>::type;
+    __shared__ T s[4 * C::PS];
+    __shared__ T strips[4 * kStrip * kAlong];
+    __shared__ NextTile tiles[2];
+    __shared__ LevelRef<T> levels[2];
+    __shared__ int bad;
+    __shared__ __align__(8) unsigned long long barrier_word;
+    extern __shared__ unsigned char stage_raw[];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int kbx = lane % C::LB, kby = warp * C::RB + lane / C::LB;
+    T* stage = reinterpret_cast<T*>(stage_raw + ((128 - ((unsigned)__cvta_generic_to_shared(stage_raw) & 127)) & 127));
+    const unsigned sb = (unsigned)__cvta_generic_to_shared(stage), bar = (unsigned)__cvta_generic_to_shared(&barrier_word);
+    T* own = s + (kby + 1) * C::P + kbx + 1;
+    const bool issuer = tid == C::kThreads - 32;   // the last warp serves no side
+    const auto load_const = [&](const NextTile& n) {
+        const SweepMaps& m = *maps(n.job);
+        const int x = n.w.ox & ~(S::kAlign - 1);
+        mbar_expect_tx(bar, S::kArrays * S::kBytes);
+        tma_load_2d(sb + S::A_XX * S::kA * sizeof(T), &m.xx, x, n.w.oy, bar);
+        tma_load_2d(sb + S::A_XY * S::kA * sizeof(T), &m.xy, x, n.w.oy, bar);
+        tma_load_2d(sb + S::A_YX * S::kA * sizeof(T), &m.yx, x, n.w.oy, bar);
+        tma_load_2d(sb + S::A_YY * S::kA * sizeof(T), &m.yy, x, n.w.oy, bar);
+        tma_load_2d(sb + S::A_D * S::kA * sizeof(T), &m.invd, x, n.w.oy, bar);
     };
-
-    // interior colour ranges (i in [mi0, mi1), j in [mj0, mj1)) on shrinking
-    // regions, and their divide-free index maps, set up while the loads fly
-    const int mi0 = pr.xl ? 0 : 1, mi1 = pr.xh ? nx : nx - 1;
-    const int mj0 = pr.yl ? 0 : 1, mj1 = pr.yh ? ny : ny - 1;
-    int ci0[4], cj0[4], ccw[4], cn[4];
-    unsigned cm[4];
-
-    // 1. stage phi on tile + (4 + E) and the operands on tile + (3 + E)
-    // (the first of K sweeps works on the tile grown by G0 = (K - 1)(4 + E))
-    const int G0 = (K - 1) * (4 + E);
-    const int hp = G0 + 4 + E, hc = G0 + 3 + E;
-    const int pi0 = max(X0 - hp, -1), pi1 = min(X1 + hp, nx + 1), pj0 = max(Y0 - hp, -1), pj1 = min(Y1 + hp, ny + 1);
-    const int ci0s = max(X0 - hc, 0), ci1s = min(X1 + hc, nx), cj0s = max(Y0 - hc, 0), cj1s = min(Y1 + hc, ny);
-    if (kTma) {
-        // the whole window of every array; what lies outside a field reads as 0 and is never used
-        const unsigned sb = (unsigned)__cvta_generic_to_shared(smem), bar = sb + W::oBarBytes;
-        constexpr unsigned kS = sizeof(T);
-        if (sb & 127) {   // TMA destinations must be 128-byte aligned
-            if (threadIdx.x == 0) set_status(status, DST_MISALIGNED);
-            return;
-        }
-        if (threadIdx.x == 0) mbar_init(bar, 1);
-        __syncthreads();
-        // The descriptors exist only for a solver's own arrays, whose faces
-        // and inverse diagonal do not change during a solve: their tiles are
-        // requested before the wait for the previous grid (the solver
-        // launches these sweeps as programmatic dependents of the kernel
-        // before them), phi and rhs after it.
-        if (threadIdx.x == 0) {
-            mbar_expect_tx(bar, W::NA * W::kBoxBytes);
-            if constexpr (W::kRI) tma_load_2d(sb + W::oD * kS, &m.invd, t.pox, t.poy, bar);
-            tma_load_2d(sb + W::oXX * kS, &m.xx, t.pox, t.poy, bar);
-            tma_load_2d(sb + W::oXY * kS, &m.xy, t.pox, t.poy, bar);
-            tma_load_2d(sb + W::oYX * kS, &m.yx, t.pox, t.poy, bar);
-            tma_load_2d(sb + W::oYY * kS, &m.yy, t.pox, t.poy, bar);
-        }
-        grid_dependency_wait();
-        if (threadIdx.x == 0) {
-            tma_load_2d(sb, &m.pin, t.pox - m.pcb, t.poy - m.prb, bar);
-            if constexpr (W::kRI) tma_load_2d(sb + W::oF * kS, &m.rhs, t.pox, t.poy, bar);
-        }
-        colour_ranges(X0, X1, Y0, Y1, E, G0, mi0, mi1, mj0, mj1, ci0, cj0, ccw, cn, cm);
-        // one warp polls the barrier; the others sleep in the block barrier
-        // instead of taking issue slots from the CTAs that are computing
-        const bool landed = threadIdx.x >= 32 || mbar_wait0(bar);
-        if (!__syncthreads_and(landed)) {   // never seen; leave the tile unwritten and report
-            if (threadIdx.x == 0) {
-                set_status(status, DST_TIMEOUT);
-                mbar_wait0(bar);   // let copies still in flight land before the CTA exits
-            }
-            return;
-        }
-    } else {
-        grid_dependency_wait();
-        stage(smem, W::PW, t.pox, t.poy, pin, pi0, pi1, pj0, pj1);
-        if constexpr (W::kRI) {
-            stage(smem + W::oF, W::PW, t.pox, t.poy, rhs, ci0s, ci1s, cj0s, cj1s);
-            stage(smem + W::oD, W::PW, t.pox, t.poy, invd, ci0s, ci1s, cj0s, cj1s);
-        }
-        stage(smem + W::oXX, W::PW, t.pox, t.poy, g.xx, ci0s, ci1s + 1, cj0s, cj1s);
-        stage(smem + W::oXY, W::PW, t.pox, t.poy, g.xy, ci0s, ci1s + 1, cj0s, cj1s);
-        stage(smem + W::oYX, W::PW, t.pox, t.poy, g.yx, ci0s, ci1s, cj0s, cj1s + 1);
-        stage(smem + W::oYY, W::PW, t.pox, t.poy, g.yy, ci0s, ci1s, cj0s, cj1s + 1);
-        colour_ranges(X0, X1, Y0, Y1, E, G0, mi0, mi1, mj0, mj1, ci0, cj0, ccw, cn, cm);
-        cp_async_wait_all();
-        __syncthreads();
+    const auto load_fields = [&](const NextTile& n) {
+        const SweepMaps& m = *maps(n.job);
+        const int x = n.w.ox & ~(S::kAlign - 1);
+        tma_load_2d(sb + S::A_P * S::kA * sizeof(T), &m.phi, x, n.w.oy, bar);
+        tma_load_2d(sb + S::A_F * S::kA * sizeof(T), &m.rhs, x, n.w.oy, bar);
+    };
+    if (issuer) {
+        mbar_init(bar, 1);
+        bad = 0;
+        NextTile& n = tiles[0];
+        n.t = blockIdx.x;
+        n.job = 0;
+        find(n);
+        levels[0] = level(n.job);
+        load_const(n);   // constant during a solve: requested before the wait for the kernel ahead
     }
-    // 2.-4. once per sweep.  Sweep s of K works on the tile grown by
-    //    G = (K - 1 - s)(4 + E): what the next sweep reads of it (tile +
-    //    G) comes out exact, as the halo argument above gives for one sweep.
-    for (int sw = 0; sw < K; ++sw) {
-        const int G = (K - 1 - sw) * (4 + E);
-        if (sw > 0) colour_ranges(X0, X1, Y0, Y1, E, G, mi0, mi1, mj0, mj1, ci0, cj0, ccw, cn, cm);
-        // 2. sweep-start ghost fill on the staged ghost cells (the ghost rows and
-        //    columns of tiles on the domain boundary only), on the sweep's footprint
-        const int qi0 = max(X0 - (G + 4 + E), -1), qi1 = min(X1 + G + 4 + E, nx + 1);
-        const int qj0 = max(Y0 - (G + 4 + E), -1), qj1 = min(Y1 + G + 4 + E, ny + 1);
-        if (qi0 < 0 || qi1 > nx || qj0 < 0 || qj1 > ny) {
-            const PinLoad<T, W::PW> P{smem, t.pox, t.poy, pi0, pi1, pj0, pj1, pin};
-            const int lw = qi1 - qi0, lh = qj1 - qj0;
-            for (int k = threadIdx.x; k < 2 * (lw + lh); k += blockDim.x) {
-                int i, j;
-                if (k < lw) { i = qi0 + k; j = qj0; }
-                else if (k < 2 * lw) { i = qi0 + k - lw; j = qj1 - 1; }
-                else if (k < 2 * lw + lh) { i = qi0; j = qj0 + k - 2 * lw; }
-                else { i = qi1 - 1; j = qj0 + k - 2 * lw - lh; }
-                if (i >= 0 && i < nx && j >= 0 && j < ny) continue;
-                smem[(j - t.poy) * W::PW + (i - t.pox)] = sweep_ghost(P, b, homog, nx, ny, i, j);
+    grid_dependency_wait();
+    if (issuer) load_fields(tiles[0]);
+    cta_sync();
+    unsigned parity = 0;
+    // One tile; kInner: of the inner region, without sides.  (Two copies: the
+    // sides' code takes so many registers that the FP32 kernel spills, which the
+    // inner tiles then do not see.)  False after the last one.
+    const auto tile = [&](auto inner_tag, int it) -> bool {
+        constexpr bool kInner = decltype(inner_tag)::value;
+        const Window& w = tiles[it].w;
+        const LevelRef<T>& L0 = levels[it];
+        const T idx = T(L0.g->idx), idy = T(L0.g->idy), om = T(omega), om1 = T(1.0 - omega);
+        Block<T> k;
+        {
+            const T* q = stage + 2 * kby * S::PW + (w.ox & (S::kAlign - 1)) + 2 * kbx;
+#pragma unroll
+            for (int r = 0; r < 3; ++r) {
+                const auto get = [&](int a, T& v0, T& v1) {
+                    const V v = *reinterpret_cast<const V*>(q + a * S::kA + r * S::PW);
+                    v0 = v.x;
+                    v1 = v.y;
+                };
+                get(S::A_YX, k.yx[r][0], k.yx[r][1]);
+                get(S::A_YY, k.yy[r][0], k.yy[r][1]);
+                if (r < 2) {
+                    get(S::A_XX, k.xx[r][0], k.xx[r][1]);
+                    get(S::A_XY, k.xy[r][0], k.xy[r][1]);
+                    get(S::A_D, k.d[r][0], k.d[r][1]);
+                    get(S::A_P, k.p[r][0], k.p[r][1]);
+                    get(S::A_F, k.f[r][0], k.f[r][1]);
+                    k.xx[r][2] = q[S::A_XX * S::kA + r * S::PW + 2];
+                    k.xy[r][2] = q[S::A_XY * S::kA + r * S::PW + 2];
+                }
             }
         }
-        __syncthreads();
-
-        // 3. interior colour passes on shrinking regions.  Interior cells are
-        //    i in [mi0, mi1), j in [mj0, mj1) (a pass has at most 21 x 21 of them
-        //    on a 32 x 32 tile, 37 x 21 on a 64 x 32 one).  FP64: a thread per
-        //    cell.  FP32: a thread per two cells, k and k + ceil(n/2) of the
-        //    colour's list, so a warp's lanes still read consecutive cells of the
-        //    colour (two-way bank conflicts, as one cell per thread).
-        if constexpr (sizeof(T) == 4) {
-            const float2 idx2 = make_float2(idx, idx), idy2 = make_float2(idy, idy);
-            const float2 om2 = make_float2(om, om), om12 = make_float2(om1, om1);
-    #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                const int nh = (cn[c] + 1) >> 1;
-                for (int k = threadIdx.x; k < nh; k += blockDim.x) {
-                    const int kb = (k + nh < cn[c]) ? k + nh : k;
-                    const int ja = fastdiv24(k, cm[c]), jb = fastdiv24(kb, cm[c]);
-                    const int ia = ci0[c] + 2 * (k - ja * ccw[c]), ib = ci0[c] + 2 * (kb - jb * ccw[c]);
-                    T* ca = t.s + (cj0[c] + 2 * ja - t.poy) * W::PW + (ia - t.pox);
-                    T* cb = t.s + (cj0[c] + 2 * jb - t.poy) * W::PW + (ib - t.pox);
-                    float2 f2, d2;
-                    if constexpr (W::kRI) {
-                        f2 = make_float2(ca[W::oF], cb[W::oF]);
-                        d2 = make_float2(ca[W::oD], cb[W::oD]);
-                    } else {
-                        const long ra = cj0[c] + 2 * ja, rb = cj0[c] + 2 * jb;
-                        const long ga = ra * rhs.ld + ia, gb = rb * rhs.ld + ib;
-                        const long ha = ra * invd.ld + ia, hb = rb * invd.ld + ib;
-                        f2 = make_float2(__ldg(rhs.p + ga), __ldg(rhs.p + gb));
-                        d2 = make_float2(__ldg(invd.p + ha), __ldg(invd.p + hb));
-                    }
-                    gs9_pair<W>(ca, cb, kb != k, f2, d2, idx2, idy2, om2, om12);
-                }
-                __syncthreads();
-            }
-        } else {
-    #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                for (int k = threadIdx.x; k < cn[c]; k += blockDim.x) {
-                    const int kj = fastdiv24(k, cm[c]);
-                    const int i = ci0[c] + 2 * (k - kj * ccw[c]), j = cj0[c] + 2 * kj;
-                    gs(i, j, RMID, RMID);
-                }
-                __syncthreads();
+        const bool any_side = !kInner && w.any();
+        if (any_side) fixed_ghosts<C>(s, w, *L0.pin, *L0.b, L0.nx, L0.ny);
+        const unsigned mask =
+            settle<C, kInner>(k, s, strips, w, kbx, kby, idx, idy, om, *L0.b, L0.nx, L0.ny);
+        cta_sync();   // the planes are in place, the staging buffer is read and the next tile placed
+        const bool more = tiles[it ^ 1].t >= 0;
+        if (issuer && more && !bad) {
+            load_const(tiles[it ^ 1]);
+            load_fields(tiles[it ^ 1]);
+        }
+        if (any_side) {
+            with_side<C>(warp, [&](auto L) {
+                L.place(w, *L0.g, *L0.b, homog, L0.nx, L0.ny, om, om1);
+                L.fill(s, *L0.pin, w, *L0.b, homog, L0.nx, L0.ny, 0);
+            });
+            cta_sync();
+            reload<C>(k, own);
+        }
+        colours<C>(k, own, mask, idx, idy, om, om1);
+        if (any_side) {
+            with_side<C>(warp, [&](auto L) {
+                L.place(w, *L0.g, *L0.b, homog, L0.nx, L0.ny, om, om1);
+                L.take(strips, w, *L0.b, homog);
+                L.pass(s, strips, w, *L0.g, *L0.b, homog, L0.nx, L0.ny);
+            });
+            cta_sync();
+            reload<C>(k, own);
+            store_ghosts<C>(s, *L0.pout, w, warp, L0.nx, L0.ny);
+        }
+        store_block<true>(k, *L0.pout, w, w.ox + 2 * kbx, w.oy + 2 * kby);
+        return more;
+    };
+#pragma unroll 1
+    for (int it = 0;; it ^= 1) {
+        if (issuer) {   // the tile after this one, while this one's loads are in flight
+            NextTile& n = tiles[it ^ 1];
+            n.t = tiles[it].t + gridDim.x;
+            n.job = tiles[it].job;
+            if (n.t < total) {
+                find(n);
+                levels[it ^ 1] = level(n.job);
+            } else {
+                n.t = -1;
             }
         }
-
-        // 4. boundary pass (edge tiles only; uniform per CTA): per colour, the
-        //    edge cells of that colour along each non-periodic side within the
-        //    tile grown by G + 1, then the corners in turn
-        if (edge_tile) {
-            const int ei0 = max(X0 - 1 - G, mi0), ei1 = min(X1 + 1 + G, mi1);
-            const int ej0 = max(Y0 - 1 - G, mj0), ej1 = min(Y1 + 1 + G, mj1);
-            const bool sxl = !pr.xl && X0 == 0, sxh = !pr.xh && X1 >= nx;
-            const bool syl = !pr.yl && Y0 == 0, syh = !pr.yh && Y1 >= ny;
-            for (int c = 0; c < 4; ++c) {
-                const int ci = colour_ci(c), cj = colour_cj(c);
-                const int ia = ei0 + ((ei0 & 1) != ci), ja = ej0 + ((ej0 & 1) != cj);
-                const int ni = (ei1 > ia) ? (ei1 - ia + 1) / 2 : 0, nj = (ej1 > ja) ? (ej1 - ja + 1) / 2 : 0;
-                const int n0 = (syl && cj == 0) ? ni : 0;
-                const int n1 = n0 + ((syh && ((ny - 1) & 1) == cj) ? ni : 0);
-                const int n2 = n1 + ((sxl && ci == 0) ? nj : 0);
-                const int n3 = n2 + ((sxh && ((nx - 1) & 1) == ci) ? nj : 0);
-                if (n3 == 0) continue;   // no cell of this colour on the tile's sides (uniform per CTA): no barrier
-                for (int k = threadIdx.x; k < n3; k += blockDim.x) {
-                    if (k < n0) gs(ia + 2 * k, 0, RMID, RLO);
-                    else if (k < n1) gs(ia + 2 * (k - n0), ny - 1, RMID, RHI);
-                    else if (k < n2) gs(0, ja + 2 * (k - n1), RLO, RMID);
-                    else gs(nx - 1, ja + 2 * (k - n2), RHI, RMID);
-                }
-                __syncthreads();
-            }
-            // the corners inside the tile grown by G, in turn (uniform per CTA;
-            // most edge tiles hold none and skip the phase and its barrier)
-            unsigned corners = 0;
-            for (int c = 0; c < 4; ++c) {
-                const int i = (c & 1) ? nx - 1 : 0, j = (c & 2) ? ny - 1 : 0;
-                if (i < X0 - G || i >= X1 + G || j < Y0 - G || j >= Y1 + G) continue;
-                const int xr = region(i, nx, pr.xl, pr.xh), yr = region(j, ny, pr.yl, pr.yh);
-                if (xr != RMID && yr != RMID) corners |= 1u << c;
-            }
-            if (corners) {
-                if (threadIdx.x == 0) {
-                    for (int c = 0; c < 4; ++c) {
-                        if (!((corners >> c) & 1u)) continue;
-                        const int i = (c & 1) ? nx - 1 : 0, j = (c & 2) ? ny - 1 : 0;
-                        gs(i, j, region(i, nx, pr.xl, pr.xh), region(j, ny, pr.yl, pr.yh));
-                    }
-                }
-                __syncthreads();
-            }
+        if (!mbar_wait(bar, parity)) {   // never seen: report, finish the tile (its result is void) and stop
+            bad = 1;
+            if (lane == 0) set_status(status, DST_TIMEOUT);
         }
-    }   // sweeps
-
-    // 5. write the tile, and the ghost cells next to it (the state fill_ghosts
-    //    leaves: filled at the start of the sweep)
-    const int wi0 = (X0 == 0) ? -1 : X0, wi1 = (X1 >= nx) ? nx + 1 : X1;
-    const int wj0 = (Y0 == 0) ? -1 : Y0, wj1 = (Y1 >= ny) ? ny + 1 : Y1;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int j = wj0 + warp; j < wj1; j += (blockDim.x >> 5)) {
-        const T* srow = smem + (j - t.poy) * W::PW - t.pox;
-        T* grow = &AT(pout, 0, j);
-        for (int i = wi0 + lane; i < wi1; i += 32) grow[i] = srow[i];
+        parity ^= 1;
+        if (!(tiles[it].inner ? tile(std::true_type(), it) : tile(std::false_type(), it))) break;
+        cta_sync();   // the planes are read no more
+        if (bad) {
+            if (issuer) mbar_wait(bar, parity);   // let copies still in flight land before the CTA exits
+            break;
+        }
     }
 }
 
-template <bool kTma, class T, int TX, int K = 1>
-__global__ void __launch_bounds__((Win<T, TX, K>::kThreads), (Win<T, TX, K>::kMinBlocks))
-    k_sweep9(const __grid_constant__ SweepMaps m, DFT<T> pin, DFT<T> pout, DFT<T> rhs, DFT<T> invd, GeoT<T> g,
-             const __grid_constant__ BCd b, int homog, int nx, int ny, int4 part, double omega, int* status) {
+template <class C>
+__global__ void __launch_bounds__(C::kThreads, C::kMinBlocks)
+    k_sweep9_stream(const __grid_constant__ SweepMaps m, const __grid_constant__ DFT<typename C::T> pin,
+                    const __grid_constant__ DFT<typename C::T> pout, const __grid_constant__ GeoT<typename C::T> g,
+                    const __grid_constant__ BCd b, const __grid_constant__ SweepTiles tiles, int homog, int nx, int ny,
+                    double omega, int* status) {
+    using T = typename C::T;
     allow_dependents();
-    sweep_tile<kTma, T, TX, K>(m, pin, pout, rhs, invd, g, b, homog, nx, ny, part, omega, status, blockIdx.x,
-                               blockIdx.y);
+    const SweepMaps* const mp = &m;
+    sweep_stream<C, T>(
+        tiles.total, homog, omega, status, [&](NextTile& n) { n.inner = place_tile(tiles, n.t, nx, ny, n.w); },
+        [&](int) { return LevelRef<T>{&pin, &pout, &g, &b, nx, ny}; }, [mp](int) { return mp; });
+}
+
+// The same over the levels of many problems (lockstep batches).  Descriptors in
+// a job table may have been rewritten since the last launch that read them
+// (tables are rebuilt when the set of unconverged problems changes): the
+// tensor-map proxy is made to see the new ones before use.
+template <class C>
+__global__ void __launch_bounds__(C::kThreads, C::kMinBlocks)
+    k_sweep9_stream_jobs(const SweepJobT<typename C::T>* __restrict__ jobs, const int* __restrict__ pre, int njobs,
+                         int total, int flip, int* status) {
+    using T = typename C::T;
+    allow_dependents();
+    sweep_stream<C, T>(
+        total, 1, 1.0, status,
+        [&](NextTile& n) {
+            const bool first = n.t < (int)gridDim.x;
+            int job = n.job;
+            while (job + 1 < njobs && __ldg(pre + job + 1) <= n.t) ++job;   // a CTA's tiles come in order
+            if (first || job != n.job) {
+                const SweepMaps& m = jobs[job].m[flip];
+                for (const CUtensorMap* d : {&m.phi, &m.rhs, &m.invd, &m.xx, &m.xy, &m.yx, &m.yy})
+                    asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(d) : "memory");
+            }
+            n.job = job;
+            const SweepJobT<T>& J = jobs[job];
+            n.inner = place_tile(J.tiles, n.t - __ldg(pre + job), J.nx, J.ny, n.w);
+        },
+        [&](int job) {
+            const SweepJobT<T>& J = jobs[job];
+            return LevelRef<T>{&J.buf[flip], &J.buf[flip ^ 1], &J.g, &J.b, J.nx, J.ny};
+        },
+        [&](int job) { return &jobs[job].m[flip]; });
+}
+
+template <class C, bool kVec>
+__global__ void __launch_bounds__(C::kThreads, C::kMinBlocks)
+    k_sweep9(DFT<typename C::T> pin, DFT<typename C::T> pout, DFT<typename C::T> rhs, DFT<typename C::T> invd,
+             GeoT<typename C::T> g, const __grid_constant__ BCd b, int homog, int nx, int ny, double omega, int K) {
+    allow_dependents();
+    sweep_tile<C, kVec>(pin, pout, rhs, invd, g, b, homog, nx, ny, gridDim.x, gridDim.y, omega, K, blockIdx.x,
+                        blockIdx.y);
 }
 
 // Lockstep batches: one launch sweeps the same level of many problems.  Job
 // k owns blocks [pre[k], pre[k + 1]) of the grid, one per tile of its level
 // (row-major over its gx x gy tiles); a block finds its job by binary
-// search.  flip selects the buffer each job's phi is read from (the job's s0
-// xor flip), so one job table serves every sweep of a smoothing call.
-// Descriptors in a job table may have been rewritten since the last launch
-// that read them (tables are rebuilt when the set of unconverged problems
-// changes): the tensor-map proxy is made to see the new ones before use.
-template <class T, int TX, int K>
-__global__ void __launch_bounds__((Win<T, TX, K>::kThreads), (Win<T, TX, K>::kMinBlocks))
-    k_sweep9_jobs(const SweepJobT<T>* __restrict__ jobs, const int* __restrict__ pre, int njobs, int flip,
-                  double omega, int* status) {
+// search.  flip selects the buffer each job's phi is read from, so one job
+// table serves every sweep of a smoothing call; a job whose level is one tile
+// is swept in place.
+template <class C>
+__global__ void __launch_bounds__(C::kThreads, C::kMinBlocks)
+    k_sweep9_jobs(const SweepJobT<typename C::T>* __restrict__ jobs, const int* __restrict__ pre, int njobs, int K,
+                  int flip) {
     allow_dependents();
     const int blk = blockIdx.x;
     int lo = 0, hi = njobs - 1;
@@ -580,26 +975,140 @@ __global__ void __launch_bounds__((Win<T, TX, K>::kThreads), (Win<T, TX, K>::kMi
         if (__ldg(pre + mid) <= blk) lo = mid;
         else hi = mid - 1;
     }
-    const SweepJobT<T>& J = jobs[lo];
-    const int q = blk - __ldg(pre + lo), side = J.s0 ^ flip;
-    const SweepMaps& m = J.m[side];
-    if (threadIdx.x == 0) {
-        for (const CUtensorMap* d : {&m.pin, &m.rhs, &m.invd, &m.xx, &m.xy, &m.yx, &m.yy})
-            asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(d) : "memory");
+    const SweepJobT<typename C::T>& J = jobs[lo];
+    const int q = blk - __ldg(pre + lo), side = J.in_place ? 0 : flip;
+    sweep_tile<C, true>(J.buf[side], J.buf[J.in_place ? 0 : side ^ 1], J.rhs, J.invd, J.g, J.b, 1, J.nx, J.ny, J.gx,
+                        J.gy, 1.0, K, q % J.gx, q / J.gx);
+}
+
+int sm_count() {
+    static std::mutex mu;
+    static int n[64] = {};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
+    std::lock_guard<std::mutex> lock(mu);
+    if (!n[dev] && cudaDeviceGetAttribute(&n[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+        cudaGetLastError();
+        n[dev] = 148;
     }
-    __syncthreads();
-    sweep_tile<true, T, TX, K>(m, J.buf[side], J.buf[side ^ 1], J.rhs, J.invd, J.g, J.b, 1, J.nx, J.ny, J.part, omega,
-                               status, q % J.gx, q / J.gx);
+    return n[dev];
+}
+
+template <class T>
+bool pair_aligned(const DFT<T>& f) {
+    return (reinterpret_cast<uintptr_t>(f.p) & (2 * sizeof(T) - 1)) == 0 && (f.ld & 1) == 0;
+}
+
+// The shapes in use: several sweeps a launch of small levels, and one sweep a
+// launch of large ones.
+using Small32 = Shape<float, 28, 32, true, 1>;
+using Large32 = Shape<float, 16, 32, false, 2>;
+using Small64 = Shape<double, 12, 16, true, 1>;
+using Large64 = Shape<double, 16, 32, false, 1>;
+template <class T>
+struct Shapes;
+template <>
+struct Shapes<float> {
+    using Small = Small32;
+    using Large = Large32;
+};
+template <>
+struct Shapes<double> {
+    using Small = Small64;
+    using Large = Large64;
+};
+
+cudaLaunchConfig_t config(dim3 grid, int threads, size_t smem, int dependent, cudaLaunchAttribute* at,
+                          cudaStream_t st) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    at->id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at->val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = dependent ? 1 : 0;
+    return cfg;
+}
+
+template <class T>
+const SweepMaps* maps_for(const LevelMaps* m, const DFT<T>& pin, const DFT<T>& rhs, const DFT<T>& invd,
+                          const GeoT<T>& g) {
+    if (!m || !m->ok || (const void*)rhs.p != m->rhs || (const void*)invd.p != m->invd || (const void*)g.xx.p != m->xx)
+        return nullptr;
+    return (const void*)pin.p == m->pa ? &m->a : (const void*)pin.p == m->pb ? &m->b : nullptr;
+}
+
+template <bool kVec, class T>
+cudaError_t launch_any(const DFT<T>& pin, const DFT<T>& pout, const DFT<T>& rhs, const DFT<T>& invd,
+                       const GeoT<T>& g, const BCd& b, int homog, int nx, int ny, double omega, const SweepPlan& p,
+                       int dependent, const LevelMaps* maps, int* status, cudaStream_t st) {
+    using S = typename Shapes<T>::Small;
+    using L = typename Shapes<T>::Large;
+    cudaLaunchAttribute at;
+    if (p.small) {
+        const cudaLaunchConfig_t cfg = config(dim3(p.gx, p.gy), S::kThreads, 0, dependent, &at, st);
+        return cudaLaunchKernelEx(&cfg, k_sweep9<S, kVec>, pin, pout, rhs, invd, g, b, homog, nx, ny, omega, p.k);
+    }
+    const SweepMaps* m = maps_for(maps, pin, rhs, invd, g);
+    if (!m) return cudaErrorInvalidValue;
+    const SweepTiles tiles = sweep_large_tiles<T>(nx, ny);
+    const int ctas = std::min(tiles.total, L::kMinBlocks * sm_count());
+    const cudaLaunchConfig_t cfg = config(dim3(ctas), L::kThreads, Stage<L>::kSmem, dependent, &at, st);
+    return cudaLaunchKernelEx(&cfg, k_sweep9_stream<L>, *m, pin, pout, g, b, tiles, homog, nx, ny, omega, status);
+}
+
+template <class T>
+cudaError_t sweep_impl(const DFT<T>& pin, const DFT<T>& pout, const DFT<T>& rhs, const DFT<T>& invd,
+                       const GeoT<T>& g, const BCd& b, int homog, int nx, int ny, double omega, const SweepPlan& p,
+                       int dependent, const LevelMaps* maps, int* status, cudaStream_t st) {
+    const DFT<T> fields[] = {pin, pout, rhs, invd, g.xx, g.xy, g.yx, g.yy};
+    bool vec = true;
+    for (const DFT<T>& f : fields) vec = vec && pair_aligned(f);
+    cudaError_t e = sweep_kernels_init();
+    if (e != cudaSuccess) return e;
+    if (vec) e = launch_any<true>(pin, pout, rhs, invd, g, b, homog, nx, ny, omega, p, dependent, maps, status, st);
+    else if constexpr (sizeof(T) == 8) e = launch_any<false>(pin, pout, rhs, invd, g, b, homog, nx, ny, omega, p, dependent, maps, status, st);
+    else e = cudaErrorMisalignedAddress;   // FP32 fields are the solver's own, always aligned
+    count_launch();
+    return e;
+}
+
+template <class C>
+SweepPlan tiles_of(int nx, int ny, int k) {
+    SweepPlan p;
+    p.k = k;
+    p.small = true;
+    // a direction the window covers whole needs no halo
+    p.gx = nx <= C::WX ? 1 : ((nx + 1) / 2 + C::tx(k) / 2 - 1) / (C::tx(k) / 2);
+    p.gy = ny <= C::WY ? 1 : ((ny + 1) / 2 + C::ty(k) / 2 - 1) / (C::ty(k) / 2);
+    return p;
+}
+
+template <class F>
+cudaError_t allow_smem(F* k, size_t bytes) {
+    return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
 }  // namespace
 
-bool sweep_fusable(const BCd& b) {
-    for (int s = 0; s < 4; ++s) {
-        const int t = b.type[s];
-        if (t != T_DIRI && t != T_NEUM && t != T_PERIODIC) return false;
-    }
-    return true;
+// Per device: dynamic shared memory above 48 KB must be opted into (before any
+// stream capture).
+cudaError_t sweep_kernels_init() {
+    static std::mutex mu;
+    static unsigned long long done = 0;
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    std::lock_guard<std::mutex> lock(mu);
+    if (dev < 64 && (done >> dev) & 1ull) return cudaSuccess;
+    e = allow_smem(k_sweep9_stream<Large32>, Stage<Large32>::kSmem);
+    if (e == cudaSuccess) e = allow_smem(k_sweep9_stream_jobs<Large32>, Stage<Large32>::kSmem);
+    if (e == cudaSuccess) e = allow_smem(k_sweep9_stream<Large64>, Stage<Large64>::kSmem);
+    if (e == cudaSuccess) e = allow_smem(k_sweep9_stream_jobs<Large64>, Stage<Large64>::kSmem);
+    if (e == cudaSuccess && dev < 64) done |= 1ull << dev;
+    return e;
 }
 
 namespace {
@@ -619,277 +1128,152 @@ PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
     return fn;
 }
 
+// A 2-D map of the width x height elements of f, box the large shape's window.
 template <class T>
-constexpr CUtensorMapDataType map_type() {
-    return sizeof(T) == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
-}
-
-// A 2-D map of `width` x `height` elements at `base`, row pitch ld, box PW x PH.
-template <class W, class T>
-bool encode(CUtensorMap* m, const T* base, long width, long height, int ld) {
+bool encode(CUtensorMap* m, const DFT<T>& f, int width, int height) {
+    using S = Stage<typename Shapes<T>::Large>;
     const PFN_cuTensorMapEncodeTiled_v12000 fn = encode_fn();
-    if (!fn || ((uintptr_t)base & 15) || (((long)ld * (long)sizeof(T)) & 15) || width > ld || width <= 0 ||
-        height <= 0)
-        return false;
+    if (!fn || ((uintptr_t)f.p & 15) || (((long)f.ld * (long)sizeof(T)) & 15)) return false;
     const cuuint64_t dims[2] = {(cuuint64_t)width, (cuuint64_t)height};
-    const cuuint64_t strides[1] = {(cuuint64_t)ld * sizeof(T)};
-    const cuuint32_t box[2] = {(cuuint32_t)W::PW, (cuuint32_t)W::PH};
+    const cuuint64_t strides[1] = {(cuuint64_t)f.ld * sizeof(T)};
+    const cuuint32_t box[2] = {(cuuint32_t)S::PW, (cuuint32_t)S::PH};
     const cuuint32_t es[2] = {1, 1};
-    return fn(m, map_type<T>(), 2, const_cast<T*>(base), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
-              CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
-template <class W, class T>
-bool prepare_maps(SweepMaps* m, const DFT<T>& e, const DFT<T>& rhs, const DFT<T>& invd, const GeoT<T>& g, int nx,
-                  int ny) {
-    // phi from the 16-byte-aligned column kAlign left of column 0 (so the
-    // ghost column -1 is inside), and row -1; the ghost column nx must lie
-    // inside the pitch
-    m->pcb = -W::kAlign;
-    m->prb = -1;
-    if (e.ld < nx + 1 + W::kAlign) return false;
-    return encode<W>(&m->pin, &AT(e, m->pcb, -1), e.ld, ny + 2, e.ld) && encode<W>(&m->rhs, rhs.p, nx, ny, rhs.ld) &&
-           encode<W>(&m->invd, invd.p, nx, ny, invd.ld) && encode<W>(&m->xx, g.xx.p, nx + 1, ny, g.xx.ld) &&
-           encode<W>(&m->xy, g.xy.p, nx + 1, ny, g.xy.ld) && encode<W>(&m->yx, g.yx.p, nx, ny + 1, g.yx.ld) &&
-           encode<W>(&m->yy, g.yy.p, nx, ny + 1, g.yy.ld);
-}
-
-template <class T, int TX, int K>
-cudaError_t set_attr_jobs() {
-    return cudaFuncSetAttribute(k_sweep9_jobs<T, TX, K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)Win<T, TX, K>::kSmemBytes);
-}
-
-template <class T, int TX, int K = 1>
-cudaError_t set_attr() {
-    cudaError_t e = cudaFuncSetAttribute(k_sweep9<true, T, TX, K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)Win<T, TX, K>::kSmemBytes);
-    if constexpr (K == 1) {   // several sweeps per launch: the solver's own arrays (TMA) only
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(k_sweep9<false, T, TX, K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)Win<T, TX, K>::kSmemBytes);
-    }
-    return e;
-}
-
-int sm_count() {
-    static std::mutex mu;
-    static int n[64] = {};
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
-    std::lock_guard<std::mutex> lock(mu);
-    if (!n[dev] && cudaDeviceGetAttribute(&n[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
-        cudaGetLastError();
-        n[dev] = 148;
-    }
-    return n[dev];
-}
-
-// Tile width for a level: FP32 levels take 64-wide tiles when those alone
-// fill every SM with as many CTAs as fit; smaller levels, whose sweep lasts
-// about one CTA's latency, keep the narrower tiles and their larger grid.
-template <class T>
-int tile_width(int nx, int ny) {
-    if (sizeof(T) == 8) return 32;
-    const long wide = (long)((nx + 63) / 64) * ((ny + kTY - 1) / kTY);
-    return wide >= (long)Win<float, 64>::kMinBlocks * sm_count() ? 64 : 32;
+    return fn(m, sizeof(T) == 8 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, f.p, dims,
+              strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 template <class T>
-void tma_prepare(SweepTma* t, const DFT<T>& ea, const DFT<T>& eb, const DFT<T>& rhs, const DFT<T>& invd,
-                 const GeoT<T>& g, int nx, int ny) {
-    t->tx = tile_width<T>(nx, ny);
-    bool wide = false;
-    if constexpr (sizeof(T) == 4) {
-        wide = t->tx == 64;
-        if (wide)
-            t->ok = prepare_maps<Win<T, 64>>(&t->ma, ea, rhs, invd, g, nx, ny) &&
-                    prepare_maps<Win<T, 64>>(&t->mb, eb, rhs, invd, g, nx, ny);
-    }
-    if (!wide)
-        t->ok = prepare_maps<Win<T, 32>>(&t->ma, ea, rhs, invd, g, nx, ny) &&
-                prepare_maps<Win<T, 32>>(&t->mb, eb, rhs, invd, g, nx, ny);
-    // two sweeps per launch: levels of 32-wide tiles that one wave of the
-    // two-sweep CTAs covers (their sweeps last about one CTA's latency)
-    const long tiles = (long)((nx + 31) / 32) * ((ny + kTY - 1) / kTY);
-    t->ok2 = t->ok && !wide && tiles <= (long)Win<T, 32, 2>::kMinBlocks * sm_count() &&
-             prepare_maps<Win<T, 32, 2>>(&t->ma2, ea, rhs, invd, g, nx, ny) &&
-             prepare_maps<Win<T, 32, 2>>(&t->mb2, eb, rhs, invd, g, nx, ny);
-    t->pa = ea.p;
-    t->pb = eb.p;
-    t->rhs = rhs.p;
-    t->invd = invd.p;
-    t->xx = g.xx.p;
-}
-
-template <class T, int TX, int K = 1>
-cudaError_t launch_tiles(const SweepMaps* m, const DFT<T>& pin, const DFT<T>& pout, const DFT<T>& rhs,
-                         const DFT<T>& invd, const GeoT<T>& g, const BCd& b, int homog, int nx, int ny, double omega,
-                         int* status, cudaStream_t st) {
-    using W = Win<T, TX, K>;
-    dim3 grd((nx + TX - 1) / TX, (ny + kTY - 1) / kTY);
-    const int4 part = make_int4(nx / (int)grd.x, nx % (int)grd.x, ny / (int)grd.y, ny % (int)grd.y);
-    if (m) {
-        // a solver's sweep: a programmatic dependent of the kernel before it
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = grd;
-        cfg.blockDim = dim3(W::kThreads);
-        cfg.dynamicSmemBytes = W::kSmemBytes;
-        cfg.stream = st;
-        cudaLaunchAttribute at[1];
-        at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        at[0].val.programmaticStreamSerializationAllowed = 1;
-        cfg.attrs = at;
-        cfg.numAttrs = 1;
-        return cudaLaunchKernelEx(&cfg, k_sweep9<true, T, TX, K>, *m, pin, pout, rhs, invd, g, b, homog, nx, ny,
-                                  part, omega, status);
-    }
-    if constexpr (K == 1) {
-        static const SweepMaps none{};
-        k_sweep9<false, T, TX><<<grd, W::kThreads, W::kSmemBytes, st>>>(none, pin, pout, rhs, invd, g, b, homog, nx,
-                                                                        ny, part, omega, status);
-        return cudaGetLastError();
-    }
-    return cudaErrorNotSupported;
-}
-
-template <class T>
-cudaError_t sweep_impl(const DFT<T>& pin, const DFT<T>& pout, const DFT<T>& rhs, const DFT<T>& invd,
-                       const GeoT<T>& g, const BCd& b, int homog, int nx, int ny, double omega, const SweepTma* tma,
-                       int* status, cudaStream_t st) {
-    cudaError_t e = sweep_kernels_init();
-    if (e != cudaSuccess) return e;
-    const SweepMaps* m = nullptr;
-    if (tma && tma->ok && (const void*)rhs.p == tma->rhs && (const void*)invd.p == tma->invd &&
-        (const void*)g.xx.p == tma->xx)
-        m = ((const void*)pin.p == tma->pa) ? &tma->ma : ((const void*)pin.p == tma->pb) ? &tma->mb : nullptr;
-    const int tx = m ? tma->tx : tile_width<T>(nx, ny);
-    bool wide = false;
-    if constexpr (sizeof(T) == 4) {
-        wide = tx == 64;
-        if (wide) e = launch_tiles<T, 64>(m, pin, pout, rhs, invd, g, b, homog, nx, ny, omega, status, st);
-    }
-    if (!wide) e = launch_tiles<T, 32>(m, pin, pout, rhs, invd, g, b, homog, nx, ny, omega, status, st);
-    count_launch();
-    return e;
+void prepare(LevelMaps* m, const DFT<T>& ea, const DFT<T>& eb, const DFT<T>& rhs, const DFT<T>& invd,
+             const GeoT<T>& g, int nx, int ny) {
+    m->ok = encode(&m->a.phi, ea, nx, ny) && encode(&m->b.phi, eb, nx, ny) && encode(&m->a.rhs, rhs, nx, ny) &&
+            encode(&m->a.invd, invd, nx, ny) && encode(&m->a.xx, g.xx, nx + 1, ny) &&
+            encode(&m->a.xy, g.xy, nx + 1, ny) && encode(&m->a.yx, g.yx, nx, ny + 1) &&
+            encode(&m->a.yy, g.yy, nx, ny + 1);
+    const CUtensorMap phi = m->b.phi;
+    m->b = m->a;
+    m->b.phi = phi;
+    m->pa = ea.p;
+    m->pb = eb.p;
+    m->rhs = rhs.p;
+    m->invd = invd.p;
+    m->xx = g.xx.p;
 }
 
 }  // namespace
 
-// Per device: dynamic shared memory above 48 KB must be opted into.
-cudaError_t sweep_kernels_init() {
-    static std::mutex mu;
-    static unsigned long long done = 0;
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return e;
-    std::lock_guard<std::mutex> lock(mu);
-    if (dev < 64 && (done >> dev) & 1ull) return cudaSuccess;
-    e = set_attr<double, 32>();
-    if (e == cudaSuccess) e = set_attr<float, 32>();
-    if (e == cudaSuccess) e = set_attr<float, 64>();
-    if (e == cudaSuccess) e = set_attr<float, 32, 2>();
-    if (e == cudaSuccess) e = set_attr<double, 32, 2>();
-    if (e == cudaSuccess) e = set_attr_jobs<double, 32, 1>();
-    if (e == cudaSuccess) e = set_attr_jobs<double, 32, 2>();
-    if (e == cudaSuccess) e = set_attr_jobs<float, 32, 1>();
-    if (e == cudaSuccess) e = set_attr_jobs<float, 64, 1>();
-    if (e == cudaSuccess) e = set_attr_jobs<float, 32, 2>();
-    if (e == cudaSuccess && dev < 64) done |= 1ull << dev;
-    return e;
+void sweep_maps_prepare(LevelMaps* m, const DF& ea, const DF& eb, const DF& rhs, const DF& invd, const Geo& g, int nx,
+                        int ny) {
+    prepare(m, ea, eb, rhs, invd, g, nx, ny);
+}
+void sweep_maps_prepare(LevelMaps* m, const DF32& ea, const DF32& eb, const DF32& rhs, const DF32& invd,
+                        const Geo32& g, int nx, int ny) {
+    prepare(m, ea, eb, rhs, invd, g, nx, ny);
 }
 
-void sweep_tma_prepare(SweepTma* t, const DF& ea, const DF& eb, const DF& rhs, const DF& invd, const Geo& g, int nx,
-                       int ny) {
-    tma_prepare(t, ea, eb, rhs, invd, g, nx, ny);
-}
-void sweep_tma_prepare(SweepTma* t, const DF32& ea, const DF32& eb, const DF32& rhs, const DF32& invd,
-                       const Geo32& g, int nx, int ny) {
-    tma_prepare(t, ea, eb, rhs, invd, g, nx, ny);
-}
-
-cudaError_t launch_sweep9(const DF& pin, const DF& pout, const DF& rhs, const DF& invd, const Geo& g, const BCd& b,
-                          int homog, int nx, int ny, double omega, const SweepTma* tma, int* status,
-                          cudaStream_t st) {
-    return sweep_impl(pin, pout, rhs, invd, g, b, homog, nx, ny, omega, tma, status, st);
-}
-cudaError_t launch_sweep9(const DF32& pin, const DF32& pout, const DF32& rhs, const DF32& invd, const Geo32& g,
-                          const BCd& b, int homog, int nx, int ny, double omega, const SweepTma* tma, int* status,
-                          cudaStream_t st) {
-    return sweep_impl(pin, pout, rhs, invd, g, b, homog, nx, ny, omega, tma, status, st);
-}
-
-bool sweep_pair_ok(const SweepTma* tma, const BCd& b) {
-    if (!tma || !tma->ok2 || !sweep_fusable(b)) return false;
-    for (int s = 0; s < 4; ++s)   // a periodic ghost would be read from global memory, one sweep stale
-        if (b.type[s] == T_PERIODIC) return false;
+bool sweep_fusable(const BCd& b) {
+    for (int s = 0; s < 4; ++s) {
+        const int t = b.type[s];
+        if (t != T_DIRI && t != T_NEUM && t != T_PERIODIC) return false;
+    }
     return true;
 }
 
+// The tiles of one sweep of a large level.  Away from the sides a tile needs 4
+// columns left, 2 right and 4 rows either side of it (a column is reached
+// through fewer colours than a row); beside a side, where the boundary pass
+// reads two cells further, 6, 4, 6 and 6.  So the grid is cut into an inner
+// rectangle of larger tiles and a frame of bands along the sides.
 template <class T>
-cudaError_t sweep_pair_impl(const DFT<T>& pin, const DFT<T>& pout, const DFT<T>& rhs, const DFT<T>& invd,
-                            const GeoT<T>& g, const BCd& b, int homog, int nx, int ny, double omega,
-                            const SweepTma* tma, int* status, cudaStream_t st) {
-    if (!sweep_pair_ok(tma, b) || (const void*)rhs.p != tma->rhs || (const void*)invd.p != tma->invd ||
-        (const void*)g.xx.p != tma->xx)
-        return cudaErrorNotSupported;
-    const SweepMaps* m =
-        ((const void*)pin.p == tma->pa) ? &tma->ma2 : ((const void*)pin.p == tma->pb) ? &tma->mb2 : nullptr;
-    if (!m) return cudaErrorNotSupported;
-    cudaError_t e = sweep_kernels_init();
-    if (e == cudaSuccess) e = launch_tiles<T, 32, 2>(m, pin, pout, rhs, invd, g, b, homog, nx, ny, omega, status, st);
-    count_launch();
-    return e;
+SweepTiles sweep_large_tiles(int nx, int ny) {
+    using L = typename Shapes<T>::Large;
+    constexpr int bx0 = L::WX - 4, bx1 = L::WX - 6, by = L::WY - 6;   // bands: left, right, bottom and top
+    SweepTiles S = {};
+    const auto add = [&](int x0, int x1, int y0, int y1, int tx, int ty, int inner) {
+        SweepTiles::Region& R = S.r[S.n++];
+        const int hx = (x1 - x0 + 1) / 2, hy = (y1 - y0 + 1) / 2;
+        R.x0 = x0, R.x1 = x1, R.y0 = y0, R.y1 = y1, R.inner = inner;
+        R.gx = (hx + tx / 2 - 1) / (tx / 2);
+        R.gy = (hy + ty / 2 - 1) / (ty / 2);
+        R.px = hx / R.gx, R.rx = hx % R.gx, R.py = hy / R.gy, R.ry = hy % R.gy;
+        R.first = S.total;
+        S.total += R.gx * R.gy;
+    };
+    if (nx < bx0 + bx1 + L::WX || ny < 2 * by + L::WY) {   // too narrow for a frame
+        add(0, nx, 0, ny, nx <= L::WX ? L::WX : L::tx(1), ny <= L::WY ? L::WY : L::ty(1), 0);
+        return S;
+    }
+    const int xr = (nx - bx1 + 1) & ~1, yt = (ny - by + 1) & ~1;   // even
+    add(0, nx, 0, by, L::tx(1), by, 0);
+    add(0, nx, yt, ny, L::tx(1), by, 0);
+    add(0, bx0, by, yt, bx0, L::ty(1), 0);
+    add(xr, nx, by, yt, bx1, L::ty(1), 0);
+    add(bx0, xr, by, yt, L::WX - 6, L::WY - 8, 1);
+    return S;
 }
+template SweepTiles sweep_large_tiles<float>(int, int);
+template SweepTiles sweep_large_tiles<double>(int, int);
 
-cudaError_t launch_sweep9_pair(const DF32& pin, const DF32& pout, const DF32& rhs, const DF32& invd, const Geo32& g,
-                               const BCd& b, int homog, int nx, int ny, double omega, const SweepTma* tma,
-                               int* status, cudaStream_t st) {
-    return sweep_pair_impl(pin, pout, rhs, invd, g, b, homog, nx, ny, omega, tma, status, st);
+// Sweeps of the next launch, of `left` still to do.  A level inside one window
+// takes all of them; a level whose tiles for 4 (2, 1) sweeps do not outnumber
+// the SMs takes that many in the small shape, since its launch lasts one CTA's
+// latency whatever it recomputes in the halo (256^2 in FP32: 2.9 us a sweep at
+// 4, 3.5 at 2, 5.0 at 1; 512^2, where 4 and 2 need a second round: 7.6, 6.1 and
+// 5.7).  A larger one takes one in the large shape (1024^2: 13.5 us against
+// 14.1 for two a launch, 2048^2: 38 against 49).  A caller's arrays, without
+// descriptors, stay with the small shape.  A periodic side's ghosts come from
+// global memory as they stand at the start of the launch, so it takes one.
+template <class T>
+SweepPlan sweep_plan(int nx, int ny, const BCd& b, int left, const LevelMaps* maps) {
+    using S = typename Shapes<T>::Small;
+    bool periodic = false;
+    for (int s = 0; s < 4; ++s) periodic = periodic || b.type[s] == T_PERIODIC;
+    if (nx <= S::WX && ny <= S::WY) return tiles_of<S>(nx, ny, periodic ? 1 : left);
+    for (int k = periodic ? 1 : 4; k >= 1; k /= 2) {
+        if (left < k || S::tx(k) < 12 || S::ty(k) < 12) continue;
+        const SweepPlan p = tiles_of<S>(nx, ny, k);
+        if ((long)p.gx * p.gy <= sm_count()) return p;
+    }
+    if (maps && maps->ok) return SweepPlan{1, 0, 0, false};
+    return tiles_of<S>(nx, ny, periodic || left < 2 || S::ty(2) < 12 ? 1 : 2);
 }
-cudaError_t launch_sweep9_pair(const DF& pin, const DF& pout, const DF& rhs, const DF& invd, const Geo& g,
-                               const BCd& b, int homog, int nx, int ny, double omega, const SweepTma* tma,
-                               int* status, cudaStream_t st) {
-    return sweep_pair_impl(pin, pout, rhs, invd, g, b, homog, nx, ny, omega, tma, status, st);
-}
+template SweepPlan sweep_plan<float>(int, int, const BCd&, int, const LevelMaps*);
+template SweepPlan sweep_plan<double>(int, int, const BCd&, int, const LevelMaps*);
 
-namespace {
-template <class T, int TX, int K>
-cudaError_t jobs_launch(const SweepJobT<T>* jobs, const int* pre, int njobs, int nblocks, int flip, int* status,
-                        cudaStream_t st) {
-    using W = Win<T, TX, K>;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(nblocks);
-    cfg.blockDim = dim3(W::kThreads);
-    cfg.dynamicSmemBytes = W::kSmemBytes;
-    cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k_sweep9_jobs<T, TX, K>, jobs, pre, njobs, flip, 1.0, status);
+cudaError_t launch_sweep9(const DF& pin, const DF& pout, const DF& rhs, const DF& invd, const Geo& g, const BCd& b,
+                          int homog, int nx, int ny, double omega, const SweepPlan& p, int dependent,
+                          const LevelMaps* maps, int* status, cudaStream_t st) {
+    return sweep_impl(pin, pout, rhs, invd, g, b, homog, nx, ny, omega, p, dependent, maps, status, st);
 }
-}  // namespace
+cudaError_t launch_sweep9(const DF32& pin, const DF32& pout, const DF32& rhs, const DF32& invd, const Geo32& g,
+                          const BCd& b, int homog, int nx, int ny, double omega, const SweepPlan& p, int dependent,
+                          const LevelMaps* maps, int* status, cudaStream_t st) {
+    return sweep_impl(pin, pout, rhs, invd, g, b, homog, nx, ny, omega, p, dependent, maps, status, st);
+}
 
 template <class T>
-cudaError_t launch_sweep9_jobs(const SweepJobT<T>* jobs, const int* pre, int njobs, int nblocks, int tx, int k,
+cudaError_t launch_sweep9_jobs(const SweepJobT<T>* jobs, const int* pre, int njobs, int nblocks, int k, int small,
                                int flip, int* status, cudaStream_t st) {
     if (njobs < 1 || nblocks < 1) return cudaSuccess;
+    using S = typename Shapes<T>::Small;
+    using L = typename Shapes<T>::Large;
     cudaError_t e = sweep_kernels_init();
     if (e != cudaSuccess) return e;
-    if (tx == 32 && k == 1) e = jobs_launch<T, 32, 1>(jobs, pre, njobs, nblocks, flip, status, st);
-    else if (tx == 32 && k == 2) e = jobs_launch<T, 32, 2>(jobs, pre, njobs, nblocks, flip, status, st);
-    else if (sizeof(T) == 4 && tx == 64 && k == 1) e = jobs_launch<float, 64, 1>(
-        reinterpret_cast<const SweepJobT<float>*>(jobs), pre, njobs, nblocks, flip, status, st);
-    else return cudaErrorInvalidValue;
+    cudaLaunchAttribute at;
+    if (small) {
+        const cudaLaunchConfig_t cfg = config(dim3(nblocks), S::kThreads, 0, 1, &at, st);
+        e = cudaLaunchKernelEx(&cfg, k_sweep9_jobs<S>, jobs, pre, njobs, k, flip);
+    } else {
+        const int ctas = std::min(nblocks, L::kMinBlocks * sm_count());
+        const cudaLaunchConfig_t cfg = config(dim3(ctas), L::kThreads, Stage<L>::kSmem, 1, &at, st);
+        e = cudaLaunchKernelEx(&cfg, k_sweep9_stream_jobs<L>, jobs, pre, njobs, nblocks, flip, status);
+    }
     count_launch();
     return e;
 }
-template cudaError_t launch_sweep9_jobs<double>(const SweepJobT<double>*, const int*, int, int, int, int, int, int*,
-                                                cudaStream_t);
-template cudaError_t launch_sweep9_jobs<float>(const SweepJobT<float>*, const int*, int, int, int, int, int, int*,
-                                               cudaStream_t);
+template cudaError_t launch_sweep9_jobs<double>(const SweepJobT<double>*, const int*, int, int, int, int, int,
+                                                int*, cudaStream_t);
+template cudaError_t launch_sweep9_jobs<float>(const SweepJobT<float>*, const int*, int, int, int, int, int,
+                                               int*, cudaStream_t);
 
 }  // namespace mgp
