@@ -393,6 +393,8 @@ struct mgp_solver {
     std::vector<Lv> lv;
     Lv* d_lv = nullptr;
     Lv* d_shadow = nullptr; // coarse levels' shared-memory layout (offsets), or nullptr
+    TinyLv* d_tiny = nullptr;       // the tiny coarse levels' dense forms, or nullptr
+    double* d_tinymat = nullptr;
     int shadow_bytes = 0;
     // MGP_FLAG_DIRECT_COARSE: level db (>= dc) is the V-cycle's bottom, solved
     // with d_ainv, its operator's inverse (transposed); db = -1 without.
@@ -462,7 +464,7 @@ void solver_free(mgp_solver* s) {
     // pool (its stream may already be gone: a server worker's, say), as
     // cudaFree would have waited for the device
     cudaDeviceSynchronize();
-    for (void* p : {(void*)s->d_lv, (void*)s->d_shadow, (void*)s->d_ainv, (void*)s->gm_base, (void*)s->gm_red,
+    for (void* p : {(void*)s->d_lv, (void*)s->d_shadow, (void*)s->d_tiny, (void*)s->d_tinymat, (void*)s->d_ainv, (void*)s->gm_base, (void*)s->gm_red,
                     (void*)s->gctl.bar, (void*)s->gctl.part, (void*)s->d_ref, (void*)s->d_status,
                     (void*)s->d_bcbuf, (void*)s->d_red})
         dfree(p, nullptr);
@@ -617,6 +619,80 @@ int build_direct_coarse(mgp_solver* s, cudaStream_t st) {
     }
     s->d_ainv = A;
     s->db = db;
+    return MGP_OK;
+}
+
+// The dense forms of the coarse levels of at most kTinyCells cells, for the
+// staged coarse cycle: *off (doubles of its shared memory taken so far) grows by
+// the matrices that fit, those read most often first; the others are read from
+// global memory.
+int build_tiny(mgp_solver* s, size_t* off, cudaStream_t st) {
+    const int md = s->maxdepth, dd = s->kind == MGP_KIND_DD;
+    bool any = false;
+    for (int k = 0; k < 4; ++k)
+        if (s->types[k] != MGP_BCTYPE_DIRI && s->types[k] != MGP_BCTYPE_NEUM && s->types[k] != MGP_BCTYPE_PERIODIC)
+            return MGP_OK;
+    std::vector<TinyLv> tiny(md + 1);
+    size_t total = 0, scratch_n = 0;
+    std::vector<size_t> at((size_t)(md + 1) * kTinyMats, 0);
+    for (int d = 0; d <= md; ++d) {
+        TinyLv& T = tiny[d];
+        std::memset(&T, 0, sizeof T);
+        for (int q = 0; q < kTinyMats; ++q) T.off[q] = -1;
+        const Lv& L = s->lv[d];
+        if (d < s->dc || (long)L.nx * L.ny > kTinyCells || L.nx < 4 || L.ny < 4) continue;
+        if (s->d_ainv && !s->direct_large && d >= s->db) continue;   // the exact bottom and what lies below it
+        any = true;
+        T.n = L.nx * L.ny;
+        if (!dd)   // stored Neumann ghosts two cells in from a corner whose other side is not Neumann
+            for (int c = 0; c < 4; ++c) {
+                const int tx = s->types[c & 1], ty = s->types[2 + (c >> 1)];
+                if ((tx == MGP_BCTYPE_NEUM) == (ty == MGP_BCTYPE_NEUM)) continue;
+                const int ci = (c & 1) ? L.nx : -1, cj = (c >> 1) ? L.ny : -1;
+                const int ii = (c & 1) ? L.nx - 3 : 2, jj = (c >> 1) ? L.ny - 3 : 2;
+                T.gi[T.ng] = ty == MGP_BCTYPE_NEUM ? ii : ci;
+                T.gj[T.ng] = ty == MGP_BCTYPE_NEUM ? cj : jj;
+                ++T.ng;
+            }
+        for (int q = 0; q < kTinyMats; ++q) {
+            if ((q == TM_C && !dd) || ((q == TM_A || q == TM_M || q == TM_AM) && d != md)) continue;
+            at[(size_t)d * kTinyMats + q] = total + 1;   // 0: no such matrix
+            total += (size_t)T.n * (T.n + ((q == TM_U || q == TM_A) ? T.ng : 0));
+        }
+        scratch_n = std::max(scratch_n, tiny_scratch_doubles(L));
+    }
+    if (!any) return MGP_OK;
+    double* scratch = nullptr;
+    if (dmalloc(&s->d_tinymat, total * sizeof(double), st) != cudaSuccess ||
+        dmalloc(&s->d_tiny, sizeof(TinyLv) * (md + 1), st) != cudaSuccess ||
+        dmalloc(&scratch, scratch_n * sizeof(double), st) != cudaSuccess) {
+        cudaGetLastError();
+        return set_err(MGP_ENOMEM, "device allocation failed");
+    }
+    cudaError_t e = cudaSuccess;
+    for (int d = 0; d <= md && e == cudaSuccess; ++d) {
+        TinyLv& T = tiny[d];
+        if (!T.n) continue;
+        for (int q = 0; q < kTinyMats; ++q) {
+            const size_t a = at[(size_t)d * kTinyMats + q];
+            T.m[q] = a ? s->d_tinymat + (a - 1) : nullptr;
+        }
+        e = launch_tiny_columns(s->lv[d], T, dd, scratch, st);
+    }
+    for (int q : {TM_M, TM_AM, TM_U, TM_S, TM_A, TM_C})
+        for (int d = md; d >= s->dc; --d) {
+            TinyLv& T = tiny[d];
+            if (!T.n || !T.m[q]) continue;
+            const size_t len = (size_t)T.n * (T.n + ((q == TM_U || q == TM_A) ? T.ng : 0));
+            if ((*off + len) * sizeof(double) > (size_t)kCoarseSmemMax) continue;
+            T.off[q] = (int)*off;
+            *off += len;
+        }
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(s->d_tiny, tiny.data(), sizeof(TinyLv) * (md + 1), cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);   // tiny leaves scope
+    dfree(scratch, st);
+    if (e != cudaSuccess) return set_err(MGP_ECUDA, "tiny levels: %s", cudaGetErrorString(e));
     return MGP_OK;
 }
 
@@ -841,6 +917,8 @@ int solver_build(mgp_solver* s, const mgp_box* valid, const mgp_geo* geo, const 
                 place(L.vv, L.nx, L.ny, 0);
             }
         }
+        if (md - s->dc + 1 <= kMaxCoarseLevels && off * sizeof(double) <= (size_t)kCoarseSmemMax)
+            RC(build_tiny(s, &off, st));
         const size_t bytes = off * sizeof(double);
         if (md - s->dc + 1 <= kMaxCoarseLevels && bytes <= (size_t)kCoarseSmemMax) {
             if (dmalloc(&s->d_shadow, sizeof(Lv) * (md + 1), st) != cudaSuccess) {
@@ -1005,6 +1083,7 @@ int coarse_cycle(mgp_solver* s, int d, int numcycles, int nd, int nu, int nb) {
     a.refy = s->d_ref + s->maxdepth + 1;
     a.status = s->d_status;
     a.shadow = s->d_shadow;
+    a.tiny = s->d_tiny;
     a.smem_bytes = s->shadow_bytes;
     a.grid_ctas = s->grid_ctas;
     a.cluster = s->coarse_cluster;
@@ -1882,6 +1961,7 @@ CoarseArgs coarse_args_of(mgp_solver* s, int d, int nd, int nu, int nb) {
     a.refy = s->d_ref + s->maxdepth + 1;
     a.status = s->d_status;
     a.shadow = s->d_shadow;
+    a.tiny = s->d_tiny;
     a.smem_bytes = s->shadow_bytes;
     a.grid_ctas = 0;
     a.cluster = 0;

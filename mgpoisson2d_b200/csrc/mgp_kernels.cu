@@ -1502,25 +1502,28 @@ __device__ void b_relax9(const Lv& L, const DF& phi, const DF& rhs, int homog, d
     }
 }
 
-// 5-point red-black sweeps of the deferred-correction smoother (DD:153-334).
-// modrhs is computed once per call, into L.w.
+// One 5-point red-black sweep of the deferred-correction smoother for a modified rhs.
+template <class S>
+__device__ void b_sweep_dd(const Lv& L, const DF& phi, const DF& modrhs, int homog, double omega) {
+    const int nx = L.nx, ny = L.ny, hx = (nx + 1) / 2;
+    b_fill<S>(phi, L.g, L.bc, homog, 1, nx, ny);   // DD:259, neum_ghosts = .true.
+    for (int colour = 0; colour < 2; ++colour) {
+        SLOOP(k, hx * ny) {
+            const int j = k / hx, i = 2 * (k % hx) + ((colour + j) & 1);
+            if (i < nx) dd_gs(phi, modrhs, L.invd, L.g, i, j, omega);
+        }
+        S::sync();
+    }
+}
+
+// The deferred-correction smoother (DD:153-334).  modrhs is computed once per call, into L.w.
 template <class S>
 __device__ void b_relax_dd(const Lv& L, const DF& phi, const DF& rhs, int homog, double omega, int sweeps) {
     const int nx = L.nx, ny = L.ny;
     if (sweeps == 0) return;
     SLOOP(k, nx * ny) AT(L.w, k % nx, k / nx) = dd_modrhs(phi, rhs, L.g, nx, ny, k % nx, k / nx);
     S::sync();
-    const int hx = (nx + 1) / 2;
-    for (int it = 0; it < sweeps; ++it) {
-        b_fill<S>(phi, L.g, L.bc, homog, 1, nx, ny);   // DD:259, neum_ghosts = .true.
-        for (int colour = 0; colour < 2; ++colour) {
-            SLOOP(k, hx * ny) {
-                const int j = k / hx, i = 2 * (k % hx) + ((colour + j) & 1);
-                if (i < nx) dd_gs(phi, L.w, L.invd, L.g, i, j, omega);
-            }
-            S::sync();
-        }
-    }
+    for (int it = 0; it < sweeps; ++it) b_sweep_dd<S>(L, phi, L.w, homog, omega);
 }
 
 // out = rhs - L[phi] (mode 1) or L[phi] (mode 0); fills phi's ghosts first as the Fortran routines do.
@@ -1646,6 +1649,217 @@ __device__ int b_bicgstab(const Lv& L, const DF& phi, const DF& rhs, int homog, 
 }
 
 // ---------------------------------------------------------------------------
+// Tiny levels as dense operators (TinyLv).  On 64 cells a sweep of the block
+// routines is ten barrier-separated phases, each a chain of some hundred
+// instructions of one or two warps: 4 to 5 us, and solve_bicgstab2 on the 4 x 4
+// bottom made 400 of them, 245 of the 457 us of a 32^2 coarse cycle (48 sweeps
+// of the levels above it most of the rest).  A sweep is a linear map of e, the
+// rhs and a few stored ghosts, so here it is one matrix-vector product of at
+// most 64 x 68, four threads a row and two barriers (0.15 us), and a BiCGStab
+// iteration four of them and five dot products that every warp forms on its own
+// (0.7 us).  FP64 throughout; the products sum in another order than the sweeps,
+// so results agree to rounding, and are the same wherever the level is solved.
+// ---------------------------------------------------------------------------
+struct TinyWork {
+    double x[kTinyCells + 4], c[kTinyCells], part[2][4 * kTinyCells];
+    double r[kTinyCells], rt[kTinyCells], p[kTinyCells], v[kTinyCells], t[kTinyCells], e[kTinyCells], y[kTinyCells];
+};
+static_assert(4 * kTinyCells <= kCoarseThreads, "four threads per row of a tiny level");
+
+// out_q = mat_q x for q < Q (n rows, nin inputs), then f(k, out...) by the thread of row k.
+template <int Q, class F>
+__device__ __forceinline__ void tiny_apply(const double* m0, const double* m1, const double* x, int n, int nin,
+                                           TinyWork& W, F f) {
+    const int q = threadIdx.x / n, k = threadIdx.x - q * n;
+    if (q < 4) {
+        const int b = q * nin / 4, e = (q + 1) * nin / 4;
+        double a0 = 0.0, a1 = 0.0, c0 = 0.0, c1 = 0.0;
+        int m = b;
+#pragma unroll 4
+        for (; m + 1 < e; m += 2) {
+            a0 = a0 + m0[m * n + k] * x[m];
+            a1 = a1 + m0[(m + 1) * n + k] * x[m + 1];
+            if (Q > 1) {
+                c0 = c0 + m1[m * n + k] * x[m];
+                c1 = c1 + m1[(m + 1) * n + k] * x[m + 1];
+            }
+        }
+        if (m < e) {
+            a0 = a0 + m0[m * n + k] * x[m];
+            if (Q > 1) c0 = c0 + m1[m * n + k] * x[m];
+        }
+        W.part[0][threadIdx.x] = a0 + a1;
+        if (Q > 1) W.part[1][threadIdx.x] = c0 + c1;
+    }
+    __syncthreads();
+    if (threadIdx.x < n) {
+        const double* p = W.part[0] + threadIdx.x;
+        const double a = (p[0] + p[n]) + (p[2 * n] + p[3 * n]);
+        double c = 0.0;
+        if (Q > 1) {
+            const double* u = W.part[1] + threadIdx.x;
+            c = (u[0] + u[n]) + (u[2 * n] + u[3 * n]);
+        }
+        f(threadIdx.x, a, c);
+    }
+    __syncthreads();
+}
+
+// a . b, or max |a| with kMax, by every warp on its own (the same bits in all).
+template <bool kMax>
+__device__ __forceinline__ double tiny_dot(const double* a, const double* b, int n) {
+    const int l = threadIdx.x & 31;
+    double u = 0.0, w = 0.0;
+    if (l < n) u = kMax ? fabs(a[l]) : a[l] * b[l];
+    if (l + 32 < n) w = kMax ? fabs(a[l + 32]) : a[l + 32] * b[l + 32];
+    u = kMax ? fmax(u, w) : u + w;
+    for (int o = 16; o > 0; o >>= 1) {
+        const double z = __shfl_xor_sync(0xffffffffu, u, o);
+        u = kMax ? fmax(u, z) : u + z;
+    }
+    return u;
+}
+
+// x = the level's cells and the stored ghosts that enter.
+__device__ __forceinline__ void tiny_load(const TinyLv& T, const DF& e, int nx, TinyWork& W) {
+    const int t = threadIdx.x;
+    if (t < T.n) W.x[t] = AT(e, t % nx, t / nx);
+    else if (t < T.n + T.ng) W.x[t] = AT(e, T.gi[t - T.n], T.gj[t - T.n]);
+    __syncthreads();
+}
+
+// b_relax on a tiny level.  The ghosts the sweeps would leave are made only where
+// someone reads them (ghosts): a DD cycle's finest level, whose correction is
+// added to phi with its ghosts.
+__device__ __forceinline__ void tiny_relax(const TinyLv& T, const Lv& L, int sweeps, int dd, bool ghosts, TinyWork& W) {
+    if (sweeps <= 0) return;
+    const int n = T.n, nin = n + T.ng, nx = L.nx;
+    tiny_load(T, L.e, nx, W);
+    const double r = threadIdx.x < n ? AT(L.r, threadIdx.x % nx, threadIdx.x / nx) : 0.0;
+    if (dd) {
+        tiny_apply<1>(T.m[TM_C], nullptr, W.x, n, n, W, [&](int k, double a, double) { W.y[k] = r + a; });
+    } else {
+        if (threadIdx.x < n) W.y[threadIdx.x] = r;
+        __syncthreads();
+    }
+    tiny_apply<1>(T.m[TM_S], nullptr, W.y, n, n, W, [&](int k, double a, double) { W.c[k] = a; });
+    for (int it = 0; it < sweeps; ++it) {
+        if (ghosts && it == sweeps - 1) {
+            if (threadIdx.x < n) AT(L.e, threadIdx.x % nx, threadIdx.x / nx) = W.x[threadIdx.x];
+            __syncthreads();
+            b_fill<BlockScope>(L.e, L.g, L.bc, 1, 1, nx, L.ny);   // DD:259
+        }
+        tiny_apply<1>(T.m[TM_U], nullptr, W.x, n, nin, W, [&](int k, double a, double) { W.x[k] = a + W.c[k]; });
+    }
+    if (threadIdx.x < n) AT(L.e, threadIdx.x % nx, threadIdx.x / nx) = W.x[threadIdx.x];
+    __syncthreads();
+}
+
+// b_bicgstab(L, L.e, L.r, 1, 1e-6, 80, 5, 0) on a tiny level, statement for
+// statement, with the two preconditioner sweeps and the operator as one pair of
+// matrices.  Of L.e's ghosts, MG's Dirichlet and periodic ones are refilled before
+// they are read and its Neumann ones gain nothing from the correction; DD's are
+// those of the final e, since every term of it carries its own.
+__device__ __forceinline__ int tiny_bicgstab(const TinyLv& T, const Lv& L, int dd, TinyWork& W) {
+    const double tol = 1.0e-6, reps = 1.0e-12, hang = 1.0e-7, small = 1.0e-30;
+    const int max_iters = 80, max_restarts = 5;
+    const int n = T.n, nin = n + T.ng, nx = L.nx, t = threadIdx.x;
+    const double vol = L.g.dx * L.g.dy;
+    const double rhs = t < n ? AT(L.r, t % nx, t / nx) : 0.0;
+    double rho[4] = {0, 0, 0, 0}, norm[2], alpha[2] = {0, 0}, beta[2] = {0, 0}, omg[2] = {0, 0};
+    int recount = 0, i = 0, restarts = 0, init = 1;
+    auto pnorm = [&]() { return dd ? tiny_dot<true>(W.r, W.r, n) : sqrt(vol * tiny_dot<false>(W.r, W.r, n)); };
+    auto residual = [&]() {   // r = rhs - L[phi], rt = r, e = 0
+        tiny_load(T, L.e, nx, W);
+        tiny_apply<1>(T.m[TM_A], nullptr, W.x, n, nin, W, [&](int k, double a, double) {
+            W.r[k] = rhs - a;
+            W.rt[k] = rhs - a;
+            W.e[k] = 0.0;
+        });
+    };
+    auto add = [&]() {   // phi += e
+        if (t < n) AT(L.e, t % nx, t / nx) = AT(L.e, t % nx, t / nx) + W.e[t];
+        __syncthreads();
+    };
+    residual();
+    norm[0] = pnorm();
+    const double initial_norm = norm[0], initial_rnorm = norm[0];
+    norm[1] = norm[0];
+    while (((i < max_iters) && (norm[0] > tol * norm[1])) && (norm[1] > 0.0)) {
+        i = i + 1;
+        norm[1] = norm[0];
+        alpha[1] = alpha[0];
+        beta[1] = beta[0];
+        omg[1] = omg[0];
+        rho[3] = rho[2];
+        rho[2] = rho[1];
+        rho[1] = vol * tiny_dot<false>(W.rt, W.r, n);
+        if (rho[1] == 0.0) {
+            add();
+            if (dd) b_fill<BlockScope>(L.e, L.g, L.bc, 1, 1, nx, L.ny);
+            return 0;
+        }
+        if (!init) beta[1] = (rho[1] / rho[2]) * (alpha[1] / omg[1]);
+        if (t < n) W.p[t] = init ? W.r[t] : beta[1] * (W.p[t] - omg[1] * W.v[t]) + W.r[t];
+        init = 0;
+        __syncthreads();
+        tiny_apply<2>(T.m[TM_M], T.m[TM_AM], W.p, n, n, W, [&](int k, double a, double c) {
+            W.y[k] = a;
+            W.v[k] = c;
+        });
+        const double m = vol * tiny_dot<false>(W.rt, W.v, n);
+        alpha[0] = rho[1] / m;
+        const bool sound = fabs(m) > small * fabs(rho[1]);
+        __syncthreads();
+        if (t < n) {
+            if (sound) {
+                W.r[t] = W.r[t] + -alpha[0] * W.v[t];
+                W.e[t] = W.e[t] + alpha[0] * W.y[t];
+            } else {
+                W.r[t] = 0.0;
+            }
+        }
+        __syncthreads();
+        norm[0] = sound ? pnorm() : 0.0;
+        if ((norm[0] > tol * initial_norm) && (norm[0] > reps * initial_rnorm)) {
+            tiny_apply<2>(T.m[TM_M], T.m[TM_AM], W.r, n, n, W, [&](int k, double a, double c) {
+                W.y[k] = a;
+                W.t[k] = c;
+            });
+            const double tr = vol * tiny_dot<false>(W.t, W.r, n), tt = vol * tiny_dot<false>(W.t, W.t, n);
+            omg[0] = tr / tt;
+            __syncthreads();
+            if (t < n) {
+                W.e[t] = W.e[t] + omg[0] * W.y[t];
+                W.r[t] = W.r[t] + -omg[0] * W.t[t];
+            }
+            __syncthreads();
+            norm[0] = pnorm();
+        }
+        if ((norm[0] <= tol * initial_norm) || (norm[0] <= reps * initial_rnorm)) break;
+        if ((omg[0] == 0.0) || (norm[0] > (1.0 - hang) * norm[1])) {
+            if (recount == 0) {
+                recount = 1;
+            } else {
+                recount = 0;
+                add();
+                if (restarts == max_restarts) break;   // then e is added again below (P2:2466)
+                residual();
+                norm[0] = pnorm();
+                rho[1] = rho[2] = rho[3] = 0.0;
+                alpha[0] = beta[0] = omg[0] = 0.0;
+                restarts = restarts + 1;
+                init = 1;
+            }
+        }
+    }
+    __syncthreads();
+    add();
+    if (dd) b_fill<BlockScope>(L.e, L.g, L.bc, 1, 1, nx, L.ny);
+    return isfinite(norm[0]) ? DST_OK : DST_NONFINITE;
+}
+
+// ---------------------------------------------------------------------------
 // The coarse sub-cycle: vcycle_noinit(d0) run to the bottom in one CTA.
 // ---------------------------------------------------------------------------
 template <class S>
@@ -1709,12 +1923,24 @@ __device__ void b_direct(const Lv& L, const double* ainv) {
 // vcycle_noinit(d0) down to the bottom and back, on the levels lv[d0..maxdepth]
 // (every thread of the block runs it).  Returns a nonzero status on a
 // non-finite bottom residual.
+// tiny (BlockScope only, nullable): the levels' dense forms, W their work space.
 template <class S>
-__device__ int coarse_body(const Lv* lv, const CoarseArgs& a, double* sh) {
+__device__ int coarse_body(const Lv* lv, const CoarseArgs& a, double* sh, const TinyLv* tiny = nullptr,
+                           TinyWork* W = nullptr) {
     int cnt[32];
     const double relax_omega = a.dd ? 4.0 / 5.0 : 1.0;
     int d = a.d0;
     int st = 0;
+    const auto is_tiny = [&](int l) { return !S::kGrid && tiny && tiny[l].n > 0; };
+    const auto relax = [&](int l, int sweeps) {
+        if constexpr (!S::kGrid) {
+            if (is_tiny(l)) {
+                tiny_relax(tiny[l], lv[l], sweeps, a.dd, a.dd && l == a.d0, *W);
+                return;
+            }
+        }
+        b_relax<S>(lv[l], lv[l].e, lv[l].r, 1, relax_omega, sweeps, a.dd);
+    };
 visit:
     {
         const Lv& L = lv[d];
@@ -1724,12 +1950,15 @@ visit:
                 b_direct<S>(L, a.ainv);
                 goto up;
             }
-            b_relax<S>(L, L.e, L.r, 1, relax_omega, a.nb, a.dd);
-            const int s = b_bicgstab<S>(L, L.e, L.r, 1, 1.0e-6, 80, 5, 0, a.dd, sh);
+            relax(d, a.nb);
+            int s;
+            if constexpr (S::kGrid) s = b_bicgstab<S>(L, L.e, L.r, 1, 1.0e-6, 80, 5, 0, a.dd, sh);
+            else s = is_tiny(d) ? tiny_bicgstab(tiny[d], L, a.dd, *W)
+                                : b_bicgstab<S>(L, L.e, L.r, 1, 1.0e-6, 80, 5, 0, a.dd, sh);
             if (s) st = s;
             goto up;
         }
-        b_relax<S>(L, L.e, L.r, 1, relax_omega, a.nd, a.dd);
+        relax(d, a.nd);
         b_apply<S>(L, L.w, L.e, L.r, 1, 1, a.dd);
         const Lv& Cl = lv[d + 1];
         const int rx = a.refx[d], ry = a.refy[d];
@@ -1754,7 +1983,7 @@ finish:
     {
         const Lv& L = lv[d];
         b_prolong<S>(L, lv[d + 1], a.refx[d], a.refy[d], 1, sh);
-        b_relax<S>(L, L.e, L.r, 1, relax_omega, a.nu, a.dd);
+        relax(d, a.nu);
     }
     goto up;
 }
@@ -1785,6 +2014,8 @@ __device__ __forceinline__ void coarse_cycle_smem(const CoarseArgs& a) {
     extern __shared__ double smem[];
     __shared__ double sh[kCoarseThreads];
     __shared__ Lv sl[kMaxCoarseLevels];
+    __shared__ TinyLv st_[kMaxCoarseLevels];
+    __shared__ TinyWork W;
     const int nl = a.maxdepth - a.d0 + 1;
     if (threadIdx.x < nl) {
         Lv L = a.shadow[a.d0 + threadIdx.x];
@@ -1809,9 +2040,24 @@ __device__ __forceinline__ void coarse_cycle_smem(const CoarseArgs& a) {
         b_copy_in(S.g.yy, G.g.yy, 0, nx, 0, ny + 1);
         if (k == 0) b_copy_in(S.r, G.r, 0, nx, 0, ny);
     }
+    if (a.tiny) {   // the dense forms that have a place in shared memory
+        for (int k = 0; k < nl; ++k) {
+            const TinyLv& G = a.tiny[a.d0 + k];
+            if (threadIdx.x == 0) st_[k] = G;
+            if (!G.n) continue;
+            for (int q = 0; q < kTinyMats; ++q) {
+                if (G.off[q] < 0) continue;
+                double* dst = smem + G.off[q];
+                const double* src = G.m[q];
+                const int len = G.n * (q == TM_U || q == TM_A ? G.n + G.ng : G.n);
+                BLOOP(m, len) cp_async8(dst + m, src + m);
+                if (threadIdx.x == 0) st_[k].m[q] = dst;
+            }
+        }
+    }
     cp_async_wait_all();
     __syncthreads();
-    const int s = coarse_body<BlockScope>(sl - a.d0, a, sh);
+    const int s = coarse_body<BlockScope>(sl - a.d0, a, sh, a.tiny ? st_ - a.d0 : nullptr, &W);
     for (int k = 0; k < nl; ++k) {
         const Lv &S = sl[k], &G = a.lv[a.d0 + k];
         b_copy(G.e, S.e, -1, S.nx + 1, -1, S.ny + 1);
@@ -1850,6 +2096,74 @@ cudaError_t launch_coarse_jobs(const CoarseJob* jobs, int njobs, int smem_bytes,
         }
     }
     k_coarse_jobs<<<njobs, kCoarseThreads, smem_bytes, st>>>(jobs);
+    count_launch();
+    return cudaGetLastError();
+}
+
+// Columns of a tiny level's matrices: block b computes one column of one of them
+// by running the block routines on a unit vector.  Scratch per block: two fields
+// with a ghost ring and two without.
+__global__ void __launch_bounds__(kCoarseThreads) k_tiny_columns(Lv L, TinyLv T, int dd, double* scratch) {
+    const int nx = L.nx, ny = L.ny, n = T.n, nin = n + T.ng, ld = nx + 2;
+    const size_t sz = (size_t)ld * (ny + 2);
+    double* base = scratch + (2 * sz + 2 * n) * blockIdx.x;
+    const DF phi{base + ld + 1, ld}, out{base + sz + ld + 1, ld}, rhs{base + 2 * sz, nx}, w{base + 2 * sz + n, nx};
+    const double om = dd ? 4.0 / 5.0 : 1.0, omb = dd ? 4.0 / 5.0 : 1.0 - 1.0 / 3.0;
+    b_setval<BlockScope>(phi, 0.0, nx, ny, 1);
+    b_setval<BlockScope>(rhs, 0.0, nx, ny, 0);
+    b_setval<BlockScope>(w, 0.0, nx, ny, 0);
+    L.w = w;
+    int b = blockIdx.x, q = TM_U;   // which matrix, which column
+    for (; q < kTinyMats; ++q) {
+        if (!T.m[q] || q == TM_AM) continue;   // M's columns give AM's too
+        const int cols = q == TM_U || q == TM_A ? nin : n;
+        if (b < cols) break;
+        b -= cols;
+    }
+    if (q == kTinyMats) return;
+    if (threadIdx.x == 0) {
+        if (q == TM_S || q == TM_M) AT(rhs, b % nx, b / nx) = 1.0;
+        else if (b < n) AT(phi, b % nx, b / nx) = 1.0;
+        else AT(phi, T.gi[b - n], T.gj[b - n]) = 1.0;
+        if (q == TM_M) AT(phi, b % nx, b / nx) = AT(L.invd, b % nx, b / nx);
+    }
+    __syncthreads();
+    const auto put = [&](int to, const DF& f) {
+        double* m = const_cast<double*>(T.m[to]) + (size_t)b * n;
+        BLOOP(k, n) m[k] = AT(f, k % nx, k / nx);
+    };
+    if (q == TM_U || q == TM_S) {
+        if (dd) b_sweep_dd<BlockScope>(L, phi, rhs, 1, om);
+        else b_relax9<BlockScope>(L, phi, rhs, 1, om, 1);
+        put(q, phi);
+    } else if (q == TM_A) {
+        b_apply<BlockScope>(L, out, phi, rhs, 1, 0, dd);
+        put(q, out);
+    } else if (q == TM_M) {
+        b_relax<BlockScope>(L, phi, rhs, 1, omb, 2, dd);
+        put(TM_M, phi);
+        __syncthreads();
+        b_apply<BlockScope>(L, out, phi, rhs, 1, 0, dd);
+        put(TM_AM, out);
+    } else {   // TM_C: the modified rhs of e with a zero rhs
+        BLOOP(k, n) AT(w, k % nx, k / nx) = dd_modrhs(phi, rhs, L.g, nx, ny, k % nx, k / nx);
+        __syncthreads();
+        put(q, w);
+    }
+}
+
+static int tiny_columns(const TinyLv& T) {
+    int c = 0;
+    for (int q = 0; q < kTinyMats; ++q)
+        if (T.m[q] && q != TM_AM) c += (q == TM_U || q == TM_A) ? T.n + T.ng : T.n;
+    return c;
+}
+size_t tiny_scratch_doubles(const Lv& L) {
+    const size_t n = (size_t)L.nx * L.ny, sz = (size_t)(L.nx + 2) * (L.ny + 2);
+    return (2 * sz + 2 * n) * (kTinyMats * (n + 4));
+}
+cudaError_t launch_tiny_columns(const Lv& L, const TinyLv& T, int dd, double* scratch, cudaStream_t st) {
+    k_tiny_columns<<<tiny_columns(T), kCoarseThreads, 0, st>>>(L, T, dd, scratch);
     count_launch();
     return cudaGetLastError();
 }

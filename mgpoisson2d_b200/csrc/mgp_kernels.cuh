@@ -42,6 +42,25 @@ struct GridCtl {
     unsigned long long wait_ns;   // a CTA's longest wait at one barrier
 };
 
+// Levels of at most this many cells run as dense operators in the staged coarse
+// cycle (TinyLv), where every side is Dirichlet, Neumann or periodic.
+constexpr int kTinyCells = 64;
+// A level's smoothing sweep, operator and bottom preconditioner as dense
+// matrices over its n cells (i fastest), stored by input: entry (k, m) at
+// [m * n + k].  A sweep and the operator read up to four stored Neumann ghosts
+// (where a Dirichlet or periodic x side meets a Neumann y side, or the other way
+// round, the corner cell's closure does): inputs n .. n + ng - 1.
+enum { TM_U, TM_S, TM_A, TM_M, TM_AM, TM_C, kTinyMats };
+struct TinyLv {
+    int n;               // cells, 0: not a tiny level
+    int ng;              // stored ghosts that enter U and A
+    int gi[4], gj[4];    // where
+    // U, S: one sweep, e' = U [e, ghosts] + S r (DD: S acts on the modified rhs, r + C e at the call's start)
+    // A: L[e] = A [e, ghosts]
+    // M, AM (bottom level): two sweeps of solve_bicgstab2's preconditioner from p * invdiags, and L of that
+    const double* m[kTinyMats];
+    int off[kTinyMats];  // place in the staged coarse cycle's shared memory (doubles), -1: read from global memory
+};
 struct CoarseArgs {
     const Lv* lv;        // device array of levels
     int d0;              // level the cycle starts at (vcycle_noinit(d0) semantics)
@@ -53,6 +72,7 @@ struct CoarseArgs {
     const int* refy;
     int* status;         // device int: 0 ok, nonzero = error code
     const Lv* shadow;    // device array: the levels' layout in shared memory (offsets), or nullptr
+    const TinyLv* tiny;  // device array: the levels' dense forms, or nullptr
     int smem_bytes;      // dynamic shared memory the staged levels need
     const double* ainv;  // MGP_FLAG_DIRECT_COARSE: inverse of level maxdepth's operator, transposed, or nullptr
     int grid_ctas;       // > 1: run as a cooperative grid of this many CTAs (gctl set)
@@ -74,6 +94,11 @@ constexpr int kGjPanel = 16;
 constexpr int kMaxCoarseLevels = 16;
 // Largest staged coarse hierarchy (bytes of dynamic shared memory).
 constexpr int kCoarseSmemMax = 200 * 1024;
+
+// Columns of a tiny level's matrices into T.m (device memory), a CTA a column.
+// scratch: tiny_scratch_doubles(L) doubles.
+size_t tiny_scratch_doubles(const Lv& L);
+cudaError_t launch_tiny_columns(const Lv& L, const TinyLv& T, int dd, double* scratch, cudaStream_t st);
 
 // Parameters of the single-CTA BiCGStab (solve_bicgstab2).
 struct BicgArgs {
