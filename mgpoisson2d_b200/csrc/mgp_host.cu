@@ -1009,7 +1009,16 @@ int smooth_body(mgp_solver* s, int d, int nu) {
     if (nu <= 0) return MGP_OK;
     if (s->kind == MGP_KIND_DD) {
         CK(launch_dd_modrhs(L.w, L.e, L.r, L.g, L.nx, L.ny, st));   // DD:226-250
-        for (int k = 0; k < nu; ++k) {
+        const bool fused = L.e2.p && dd_sweep_fusable(L.bc);
+        for (int k = 0, done = 0; k < nu; k += done) {
+            done = 0;
+            if (fused)
+                CK(launch_dd_sweeps(L.e, L.e2, L.w, L.invd, L.g, L.bc, L.nx, L.ny, 4.0 / 5.0, nu - k, &done, st));
+            if (done) {
+                std::swap(L.e, L.e2);
+                continue;
+            }
+            done = 1;
             CK(launch_fill(L.e, L.g, L.bc, 1, 1, L.nx, L.ny, st));   // DD:259
             CK(launch_dd_colour(L.e, L.w, L.invd, L.g, L.nx, L.ny, 4.0 / 5.0, 0, st));
             CK(launch_dd_colour(L.e, L.w, L.invd, L.g, L.nx, L.ny, 4.0 / 5.0, 1, st));
@@ -1138,7 +1147,18 @@ int vcycle32(mgp_solver* s, int d, int numcycles, int nd, int nu, int nb) {
             if (dd) {
                 if (nu_ <= 0) return MGP_OK;
                 CK(launch_dd_modrhs(L.w, L.e, L.r, L.g, L.nx, L.ny, st));   // DD:226-250
-                for (int k = 0; k < nu_; ++k) {
+                const bool fused = dd_sweep_fusable(F.bc);
+                for (int k = 0, done = 0; k < nu_; k += done) {
+                    done = 0;
+                    if (fused)   // the BF16 study rounds after each sweep
+                        CK(launch_dd_sweeps(L.e, L.e2, L.w, L.invd, L.g, F.bc, L.nx, L.ny, 4.0 / 5.0,
+                                            b16 && d >= 1 ? 1 : nu_ - k, &done, st));
+                    if (done) {
+                        std::swap(L.e, L.e2);
+                        CK(round16(L.e, d, L.nx, L.ny, 1));
+                        continue;
+                    }
+                    done = 1;
                     CK(launch_fill(L.e, L.g, F.bc, 1, 1, L.nx, L.ny, st));   // DD:259
                     CK(launch_dd_colour(L.e, L.w, L.invd, L.g, L.nx, L.ny, 4.0 / 5.0, 0, st));
                     CK(launch_dd_colour(L.e, L.w, L.invd, L.g, L.nx, L.ny, 4.0 / 5.0, 1, st));

@@ -360,6 +360,16 @@ cudaError_t launch_dd_modrhs(const DF& out, const DF& phi, const DF& rhs, const 
                              cudaStream_t st);
 cudaError_t launch_dd_colour(const DF& phi, const DF& modrhs, const DF& invd, const Geo& g, int nx, int ny,
                              double omega, int colour, cudaStream_t st);
+// Several red-black sweeps (ghost fill included) in one launch, pin to pout (two
+// buffers) for the modified rhs m; *done of the `left` sweeps were launched.  A
+// programmatic dependent: the faces and invd must not be written by the kernel
+// ahead.  Sides must be Dirichlet or Neumann with LAH ghosts (dd_sweep_fusable);
+// the solver's own arrays (rows aligned to pairs).
+bool dd_sweep_fusable(const BCd& b);
+cudaError_t launch_dd_sweeps(const DF& pin, const DF& pout, const DF& m, const DF& invd, const Geo& g, const BCd& b,
+                             int nx, int ny, double omega, int left, int* done, cudaStream_t st);
+cudaError_t launch_dd_sweeps(const DF32& pin, const DF32& pout, const DF32& m, const DF32& invd, const Geo32& g,
+                             const BCd& b, int nx, int ny, double omega, int left, int* done, cudaStream_t st);
 // The same three on FP32 fields (the grid levels of a mixed-precision DD V-cycle).
 cudaError_t launch_dd_apply(const DF32& out, const DF32& phi, const DF32& rhs, const Geo32& g, const BCd& b, int nx,
                             int ny, int mode, cudaStream_t st);
