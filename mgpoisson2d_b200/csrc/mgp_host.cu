@@ -8,6 +8,7 @@
 // step; the levels small enough for one CTA run their whole sub-cycle in
 // k_coarse_cycle.
 #include <cuda_runtime.h>
+#include <cudaTypedefs.h>
 
 #include <algorithm>
 #include <cmath>
@@ -286,7 +287,16 @@ int stage_out(const DF& d, const mgp_array* u, int nxv, int nyv, int gmax, cudaS
     return MGP_OK;
 }
 
+// One value from host or device memory.  Pageable host memory, where a boundary
+// value nearly always lies, is read directly: through cudaMemcpy each of a call's
+// four cost several microseconds of driver time.
 int read_scalar(const double* p, double* out) {
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, p) == cudaSuccess && at.type == cudaMemoryTypeUnregistered) {
+        *out = *p;
+        return MGP_OK;
+    }
+    cudaGetLastError();
     CK(cudaMemcpy(out, p, sizeof(double), cudaMemcpyDefault));
     return MGP_OK;
 }
@@ -1700,41 +1710,117 @@ int oneshot(int which, const mgp_box* valid, mgp_array* phi, mgp_array* rhs, con
 }
 
 // ---------------------------------------------------------------------------
-// Operator-level calls: a short-lived context that stages the arguments.
+// Operator-level calls: a short-lived context for the arguments.  An array in
+// this device's memory is worked on where it lies; host memory (and whatever the
+// driver does not vouch for) is staged through device buffers from the solvers'
+// pool.  With every array staged and every buffer from cudaMalloc, a 2048^2
+// residual took 6.2 ms for a kernel of 78 us: 5.4 ms of allocation, 0.39 ms of
+// copies and fills.
 // ---------------------------------------------------------------------------
+PFN_cuPointerGetAttributes_v7000 pointer_attributes_fn() {
+    static PFN_cuPointerGetAttributes_v7000 fn = nullptr;
+    static std::once_flag once;
+    std::call_once(once, [] {
+        void* p = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuPointerGetAttributes", &p, cudaEnableDefault, &q) == cudaSuccess &&
+            q == cudaDriverEntryPointSuccess)
+            fn = reinterpret_cast<PFN_cuPointerGetAttributes_v7000>(p);
+        else
+            cudaGetLastError();
+    });
+    return fn;
+}
+
+// Whether [p, p + bytes) is plain device memory of the current device.
+bool device_range(const void* p, size_t bytes) {
+    const PFN_cuPointerGetAttributes_v7000 fn = pointer_attributes_fn();
+    int dev = 0;
+    if (!fn || cudaGetDevice(&dev) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    unsigned type = 0, managed = 0;
+    int ordinal = -1;
+    CUdeviceptr start = 0;
+    size_t size = 0;
+    CUpointer_attribute at[] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_IS_MANAGED,
+                                CU_POINTER_ATTRIBUTE_DEVICE_ORDINAL, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR,
+                                CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+    void* out[] = {&type, &managed, &ordinal, &start, &size};
+    if (fn(5, at, out, (CUdeviceptr)p) != CUDA_SUCCESS) return false;
+    return type == CU_MEMORYTYPE_DEVICE && !managed && ordinal == dev && (CUdeviceptr)p >= start &&
+           (CUdeviceptr)p + bytes <= start + size;
+}
+
 struct OpCtx {
     std::vector<void*> bufs;
     cudaStream_t st = nullptr;
+    // The memory every array of the call spans: an array that is written is
+    // worked on in place only where no other array of the call shares memory
+    // with it (a staged one is read whole before anything is written, and
+    // written back at the end).
+    struct Span {
+        const void* data;
+        uintptr_t lo, hi;
+    };
+    std::vector<Span> spans;
     ~OpCtx() {
-        for (void* p : bufs) cudaFree(p);
+        for (void* p : bufs) dfree(p, st);   // ordered after the call's work
     }
+    void span(const mgp_array* a, int nxv, int nyv) {
+        if (!a || !a->data || a->ngx < 0 || a->ngy < 0 || nxv < 1 || nyv < 1) return;
+        const uintptr_t lo = (uintptr_t)a->data;
+        const size_t n = (size_t)(nyv + 2 * a->ngy - 1) * array_ld(a, nxv) + nxv + 2 * a->ngx;
+        spans.push_back(Span{a, lo, lo + n * sizeof(double)});
+    }
+    void span(const mgp_geo* g, const mgp_box* v) {
+        if (!g) return;
+        span(&g->J, v->nx, v->ny);
+        span(&g->Jgup_xx, v->nx + 1, v->ny);
+        span(&g->Jgup_xy, v->nx + 1, v->ny);
+        span(&g->Jgup_yx, v->nx, v->ny + 1);
+        span(&g->Jgup_yy, v->nx, v->ny + 1);
+    }
+    // Whether the array can be used where it lies, with g ghost layers; alone:
+    // only if no other array of the call overlaps it.
+    bool view(const mgp_array* a, int nxv, int nyv, int g, bool alone, DF* f) {
+        if (a->ngx < g || a->ngy < g || ((uintptr_t)a->data & 7)) return false;
+        const int ld = array_ld(a, nxv);
+        const size_t n = (size_t)(nyv + 2 * a->ngy - 1) * ld + nxv + 2 * a->ngx;
+        const uintptr_t lo = (uintptr_t)a->data, hi = lo + n * sizeof(double);
+        if (!device_range(a->data, n * sizeof(double))) return false;
+        if (alone)
+            for (const Span& s : spans)
+                if (s.data != a && s.lo < hi && lo < s.hi) return false;
+        f->ld = ld;
+        f->p = a->data + a->ngx + (size_t)a->ngy * ld;
+        return true;
+    }
+    // A device buffer with g ghost layers, all zero.
     int field(DF* f, int nxv, int nyv, int g) {
         const int ld = ((nxv + 2 * g + 31) / 32) * 32;
         const size_t pad = g ? 32 : 0;
         const size_t n = (size_t)(nyv + 2 * g) * ld + 2 * pad;
         double* p = nullptr;
-        if (cudaMalloc(&p, n * 8) != cudaSuccess) {
-            cudaGetLastError();
-            return set_err(MGP_ENOMEM, "cudaMalloc failed");
-        }
-        bufs.push_back(p);
+        RC(dbuf(&p, n));
         CK(cudaMemsetAsync(p, 0, n * 8, st));
         f->ld = ld;
         f->p = p + pad + (size_t)g * ld;
         return MGP_OK;
     }
     int dbuf(double** p, size_t n) {
-        if (cudaMalloc(p, n * 8) != cudaSuccess) {
+        if (dmalloc(p, n * 8, st) != cudaSuccess) {
             cudaGetLastError();
-            return set_err(MGP_ENOMEM, "cudaMalloc failed");
+            return set_err(MGP_ENOMEM, "device allocation failed");
         }
         bufs.push_back(*p);
         return MGP_OK;
     }
     int ibuf(int** p) {
-        if (cudaMalloc(p, sizeof(int)) != cudaSuccess) {
+        if (dmalloc(p, sizeof(int), st) != cudaSuccess) {
             cudaGetLastError();
-            return set_err(MGP_ENOMEM, "cudaMalloc failed");
+            return set_err(MGP_ENOMEM, "device allocation failed");
         }
         bufs.push_back(*p);
         CK(cudaMemsetAsync(*p, 0, sizeof(int), st));
@@ -1744,32 +1830,42 @@ struct OpCtx {
     int geo(const mgp_geo* g, const mgp_box* v, Geo* out) {
         if (!g) return set_err(MGP_EINVAL, "null geometry");
         DF J, xx, xy, yx, yy;
-        RC(check_array(&g->J, v->nx, "J"));
-        RC(check_array(&g->Jgup_xx, v->nx + 1, "Jgup_xx"));
-        RC(check_array(&g->Jgup_xy, v->nx + 1, "Jgup_xy"));
-        RC(check_array(&g->Jgup_yx, v->nx, "Jgup_yx"));
-        RC(check_array(&g->Jgup_yy, v->nx, "Jgup_yy"));
-        RC(field(&J, v->nx, v->ny, 0));
-        RC(field(&xx, v->nx + 1, v->ny, 0));
-        RC(field(&xy, v->nx + 1, v->ny, 0));
-        RC(field(&yx, v->nx, v->ny + 1, 0));
-        RC(field(&yy, v->nx, v->ny + 1, 0));
-        RC(stage_in(&g->J, v->nx, v->ny, J, 0, st));
-        RC(stage_in(&g->Jgup_xx, v->nx + 1, v->ny, xx, 0, st));
-        RC(stage_in(&g->Jgup_xy, v->nx + 1, v->ny, xy, 0, st));
-        RC(stage_in(&g->Jgup_yx, v->nx, v->ny + 1, yx, 0, st));
-        RC(stage_in(&g->Jgup_yy, v->nx, v->ny + 1, yy, 0, st));
+        RC(in(&g->J, v->nx, v->ny, 0, &J, "J"));
+        RC(in(&g->Jgup_xx, v->nx + 1, v->ny, 0, &xx, "Jgup_xx"));
+        RC(in(&g->Jgup_xy, v->nx + 1, v->ny, 0, &xy, "Jgup_xy"));
+        RC(in(&g->Jgup_yx, v->nx, v->ny + 1, 0, &yx, "Jgup_yx"));
+        RC(in(&g->Jgup_yy, v->nx, v->ny + 1, 0, &yy, "Jgup_yy"));
         *out = make_geo(J, xx, xy, yx, yy, g->dx, g->dy);
         return MGP_OK;
     }
+    // An array the call only reads.
     int in(const mgp_array* a, int nxv, int nyv, int g, DF* f, const char* what) {
         RC(check_array(a, nxv, what));
+        if (view(a, nxv, nyv, g, false, f)) return MGP_OK;
         RC(field(f, nxv, nyv, g));
         return stage_in(a, nxv, nyv, *f, g, st);
     }
+    // An array the call reads and writes, or (out) writes whole; back() returns it.
+    int inout(const mgp_array* a, int nxv, int nyv, int g, DF* f, const char* what) {
+        RC(check_array(a, nxv, what));
+        if (view(a, nxv, nyv, g, true, f)) return MGP_OK;
+        RC(field(f, nxv, nyv, g));
+        return stage_in(a, nxv, nyv, *f, g, st);
+    }
+    int out(const mgp_array* a, int nxv, int nyv, DF* f, const char* what) {
+        RC(check_array(a, nxv, what));
+        if (view(a, nxv, nyv, 0, true, f)) return MGP_OK;
+        return field(f, nxv, nyv, 0);
+    }
+    int back(const DF& f, const mgp_array* a, int nxv, int nyv, int gmax) {
+        if (f.p == a->data + a->ngx + (size_t)a->ngy * array_ld(a, nxv)) return MGP_OK;   // it lies there
+        return stage_out(f, a, nxv, nyv, gmax, st);
+    }
     int bc(const mgp_bdry* b, const mgp_box* v, int homog, BCd* out) {
         double* d = nullptr;
-        RC(dbuf(&d, 2 * (size_t)(v->nx + v->ny + 2)));
+        bool values = false;
+        for (int s = 0; b && s < 4; ++s) values = values || b->mode[s] == MGP_BCMODE_NONUNIFORM;
+        if (values) RC(dbuf(&d, 2 * (size_t)(v->nx + v->ny + 2)));
         return make_bc(b, v, homog, d, out, st);
     }
     int finish() {
@@ -2482,14 +2578,16 @@ int mgp_fill_ghosts(const mgp_box* valid, mgp_array* phi, const mgp_bdry* bc, co
     RC(check_array(phi, valid->nx, "phi"));
     RC(ghost_cap(phi));
     OpCtx c;
+    c.span(phi, valid->nx, valid->ny);
+    c.span(geo, valid);
     DF p;
     Geo g;
     BCd b;
-    RC(c.in(phi, valid->nx, valid->ny, 1, &p, "phi"));
+    RC(c.inout(phi, valid->nx, valid->ny, 1, &p, "phi"));
     RC(c.geo(geo, valid, &g));
     RC(c.bc(bc, valid, homog, &b));
     CK(launch_fill(p, g, b, homog, do_neum, valid->nx, valid->ny, c.st));
-    RC(stage_out(p, phi, valid->nx, valid->ny, 1, c.st));
+    RC(c.back(p, phi, valid->nx, valid->ny, 1));
     return c.finish();
 }
 
@@ -2499,10 +2597,11 @@ int mgp_extrapolate_ghosts(const mgp_box* valid, mgp_array* phi, int order) {
     RC(ghost_cap(phi));
     if (order < 0 || order > 3) return set_err(MGP_EINVAL, "extrapolate_ghosts: order is not supported");
     OpCtx c;
+    c.span(phi, valid->nx, valid->ny);
     DF p;
-    RC(c.in(phi, valid->nx, valid->ny, 1, &p, "phi"));
+    RC(c.inout(phi, valid->nx, valid->ny, 1, &p, "phi"));
     CK(launch_extrapolate(p, valid->nx, valid->ny, phi->ngx, phi->ngy, order, c.st));
-    RC(stage_out(p, phi, valid->nx, valid->ny, 1, c.st));
+    RC(c.back(p, phi, valid->nx, valid->ny, 1));
     return c.finish();
 }
 
@@ -2512,14 +2611,16 @@ int mgp_compute_invdiags(const mgp_box* valid, mgp_array* invdiags, const mgp_ge
     RC(no_lah(bc));
     RC(check_array(invdiags, valid->nx, "invdiags"));
     OpCtx c;
+    c.span(invdiags, valid->nx, valid->ny);
+    c.span(geo, valid);
     DF d;
     Geo g;
     BCd b;
-    RC(c.field(&d, valid->nx, valid->ny, 0));
+    RC(c.out(invdiags, valid->nx, valid->ny, &d, "invdiags"));
     RC(c.geo(geo, valid, &g));
     RC(c.bc(bc, valid, homog, &b));
     CK(launch_invdiag(d, g, b, homog, valid->nx, valid->ny, (g_flags & MGP_FLAG_DIRICHLET_COUPLED_DIAG) ? 1 : 0, c.st));
-    RC(stage_out(d, invdiags, valid->nx, valid->ny, 0, c.st));
+    RC(c.back(d, invdiags, valid->nx, valid->ny, 0));
     return c.finish();
 }
 
@@ -2531,17 +2632,20 @@ int mgp_compute_laplacian(const mgp_box* valid, mgp_array* lap, mgp_array* phi, 
     RC(check_array(phi, valid->nx, "phi"));
     RC(ghost_cap(phi));
     OpCtx c;
+    c.span(lap, valid->nx, valid->ny);
+    c.span(phi, valid->nx, valid->ny);
+    c.span(geo, valid);
     DF l, p;
     Geo g;
     BCd b;
-    RC(c.field(&l, valid->nx, valid->ny, 0));
-    RC(c.in(phi, valid->nx, valid->ny, 1, &p, "phi"));
+    RC(c.out(lap, valid->nx, valid->ny, &l, "lap"));
+    RC(c.inout(phi, valid->nx, valid->ny, 1, &p, "phi"));
     RC(c.geo(geo, valid, &g));
     RC(c.bc(bc, valid, homog, &b));
     CK(launch_fill(p, g, b, homog, 0, valid->nx, valid->ny, c.st));
     CK(launch_apply(l, p, l, g, b, homog, valid->nx, valid->ny, 0, jscale, c.st));
-    RC(stage_out(l, lap, valid->nx, valid->ny, 0, c.st));
-    RC(stage_out(p, phi, valid->nx, valid->ny, 1, c.st));
+    RC(c.back(l, lap, valid->nx, valid->ny, 0));
+    RC(c.back(p, phi, valid->nx, valid->ny, 1));
     return c.finish();
 }
 
@@ -2556,11 +2660,13 @@ int mgp_compute_pd(const mgp_box* valid, mgp_array* pd, const mgp_array* phi, in
     if (dir == nodedir && ((dir == 1 && phi->ngx < 1) || (dir == 2 && phi->ngy < 1)))
         return set_err(MGP_EINVAL, "compute_pd: the nodal derivative needs a ghost layer");
     OpCtx c;
+    c.span(pd, fx, fy);
+    c.span(phi, nx, ny);
     DF d, p;
-    RC(c.field(&d, fx, fy, 0));
+    RC(c.out(pd, fx, fy, &d, "pd"));
     RC(c.in(phi, nx, ny, 1, &p, "phi"));
     CK(launch_pd(d, p, nx, ny, valid->dx, valid->dy, dir, nodedir, c.st));
-    RC(stage_out(d, pd, fx, fy, 0, c.st));
+    RC(c.back(d, pd, fx, fy, 0));
     return c.finish();
 }
 
@@ -2574,19 +2680,23 @@ int mgp_compute_grad(const mgp_box* valid, mgp_array* xflux, mgp_array* yflux, m
     RC(ghost_cap(phi));
     if (phi->ngx < 1 || phi->ngy < 1) return set_err(MGP_EINVAL, "compute_grad: phi needs a ghost layer");
     OpCtx c;
+    c.span(xflux, nx + 1, ny);
+    c.span(yflux, nx, ny + 1);
+    c.span(phi, nx, ny);
+    c.span(geo, valid);
     DF x, y, p;
     Geo g;
     BCd b;
-    RC(c.field(&x, nx + 1, ny, 0));
-    RC(c.field(&y, nx, ny + 1, 0));
-    RC(c.in(phi, nx, ny, 1, &p, "phi"));
+    RC(c.out(xflux, nx + 1, ny, &x, "xflux"));
+    RC(c.out(yflux, nx, ny + 1, &y, "yflux"));
+    RC(c.inout(phi, nx, ny, 1, &p, "phi"));
     RC(c.geo(geo, valid, &g));
     RC(c.bc(bc, valid, homog, &b));
     CK(launch_fill(p, g, b, homog, 0, nx, ny, c.st));   // P2:828
     CK(launch_grad(x, y, p, g, b, homog, nx, ny, c.st));
-    RC(stage_out(x, xflux, nx + 1, ny, 0, c.st));
-    RC(stage_out(y, yflux, nx, ny + 1, 0, c.st));
-    RC(stage_out(p, phi, nx, ny, 1, c.st));
+    RC(c.back(x, xflux, nx + 1, ny, 0));
+    RC(c.back(y, yflux, nx, ny + 1, 0));
+    RC(c.back(p, phi, nx, ny, 1));
     return c.finish();
 }
 
@@ -2595,14 +2705,16 @@ int mgp_fill_boundary_fluxes(const mgp_box* valid, mgp_array* xflux, mgp_array* 
     RC(check_box(valid));
     const int nx = valid->nx, ny = valid->ny;
     OpCtx c;
+    c.span(xflux, nx + 1, ny);
+    c.span(yflux, nx, ny + 1);
     DF x, y;
     BCd b;
-    RC(c.in(xflux, nx + 1, ny, 0, &x, "xflux"));
-    RC(c.in(yflux, nx, ny + 1, 0, &y, "yflux"));
+    RC(c.inout(xflux, nx + 1, ny, 0, &x, "xflux"));
+    RC(c.inout(yflux, nx, ny + 1, 0, &y, "yflux"));
     RC(c.bc(bc, valid, homog, &b));
     CK(launch_boundary_fluxes(x, y, b, homog, nx, ny, c.st));
-    RC(stage_out(x, xflux, nx + 1, ny, 0, c.st));
-    RC(stage_out(y, yflux, nx, ny + 1, 0, c.st));
+    RC(c.back(x, xflux, nx + 1, ny, 0));
+    RC(c.back(y, yflux, nx, ny + 1, 0));
     return c.finish();
 }
 
@@ -2611,12 +2723,15 @@ int mgp_compute_div(const mgp_box* valid, mgp_array* div, const mgp_array* xflux
     const int nx = valid->nx, ny = valid->ny;
     RC(check_array(div, nx, "div"));
     OpCtx c;
+    c.span(div, nx, ny);
+    c.span(xflux, nx + 1, ny);
+    c.span(yflux, nx, ny + 1);
     DF d, x, y;
-    RC(c.field(&d, nx, ny, 0));
+    RC(c.out(div, nx, ny, &d, "div"));
     RC(c.in(xflux, nx + 1, ny, 0, &x, "xflux"));
     RC(c.in(yflux, nx, ny + 1, 0, &y, "yflux"));
     CK(launch_div(d, x, y, nx, ny, valid->dx, valid->dy, c.st));
-    RC(stage_out(d, div, nx, ny, 0, c.st));
+    RC(c.back(d, div, nx, ny, 0));
     return c.finish();
 }
 
@@ -2628,18 +2743,22 @@ int mgp_compute_residual(const mgp_box* valid, mgp_array* res, const mgp_array* 
     RC(check_array(phi, valid->nx, "phi"));
     RC(ghost_cap(phi));
     OpCtx c;
+    c.span(res, valid->nx, valid->ny);
+    c.span(rhs, valid->nx, valid->ny);
+    c.span(phi, valid->nx, valid->ny);
+    c.span(geo, valid);
     DF r, f, p;
     Geo g;
     BCd b;
-    RC(c.field(&r, valid->nx, valid->ny, 0));
+    RC(c.out(res, valid->nx, valid->ny, &r, "res"));
     RC(c.in(rhs, valid->nx, valid->ny, 0, &f, "rhs"));
-    RC(c.in(phi, valid->nx, valid->ny, 1, &p, "phi"));
+    RC(c.inout(phi, valid->nx, valid->ny, 1, &p, "phi"));
     RC(c.geo(geo, valid, &g));
     RC(c.bc(bc, valid, homog, &b));
     CK(launch_fill(p, g, b, homog, 0, valid->nx, valid->ny, c.st));
     CK(launch_apply(r, p, f, g, b, homog, valid->nx, valid->ny, 1, jscale, c.st));
-    RC(stage_out(r, res, valid->nx, valid->ny, 0, c.st));
-    RC(stage_out(p, phi, valid->nx, valid->ny, 1, c.st));
+    RC(c.back(r, res, valid->nx, valid->ny, 0));
+    RC(c.back(p, phi, valid->nx, valid->ny, 1));
     return c.finish();
 }
 
@@ -2653,11 +2772,15 @@ int mgp_relax_jacobi(const mgp_box* valid, mgp_array* phi, const mgp_array* rhs,
     if (maxiters == 0) return MGP_OK;
     const int nx = valid->nx, ny = valid->ny;
     OpCtx c;
+    c.span(phi, nx, ny);
+    c.span(rhs, nx, ny);
+    c.span(invdiags, nx, ny);
+    c.span(geo, valid);
     DF p, f, d, r;
     Geo g;
     BCd b;
     double* red = nullptr;
-    RC(c.in(phi, nx, ny, 1, &p, "phi"));
+    RC(c.inout(phi, nx, ny, 1, &p, "phi"));
     RC(c.in(rhs, nx, ny, 0, &f, "rhs"));
     RC(c.in(invdiags, nx, ny, 0, &d, "invdiags"));
     RC(c.field(&r, nx, ny, 0));
@@ -2692,7 +2815,7 @@ int mgp_relax_jacobi(const mgp_box* valid, mgp_array* phi, const mgp_array* rhs,
             if (h / rscale <= tol) break;
         }
     }
-    RC(stage_out(p, phi, nx, ny, 1, c.st));
+    RC(c.back(p, phi, nx, ny, 1));
     return c.finish();
 }
 
@@ -2708,16 +2831,21 @@ int mgp_relax_gs(const mgp_box* valid, mgp_array* phi, const mgp_array* rhs, con
         return set_err(MGP_EINVAL, "relax_gs: the device sweep needs at least 4 cells per direction");
     const int nx = valid->nx, ny = valid->ny;
     OpCtx c;
+    c.span(phi, nx, ny);
+    c.span(rhs, nx, ny);
+    c.span(invdiags, nx, ny);
+    c.span(geo, valid);
     DF p, p2, f, d, r;
     Geo g;
     BCd b;
     double* red = nullptr;
-    RC(c.field(&p2, nx, ny, 1));
-    RC(c.in(phi, nx, ny, 1, &p, "phi"));
+    RC(c.inout(phi, nx, ny, 1, &p, "phi"));
     RC(c.in(rhs, nx, ny, 0, &f, "rhs"));
     RC(c.in(invdiags, nx, ny, 0, &d, "invdiags"));
-    RC(c.field(&r, nx, ny, 0));
-    RC(c.dbuf(&red, kRedSlots));
+    if (tol > 0.0) {   // the residual norm between sweeps
+        RC(c.field(&r, nx, ny, 0));
+        RC(c.dbuf(&red, kRedSlots));
+    }
     RC(c.geo(geo, valid, &g));
     RC(c.bc(bc, valid, homog, &b));
     if (zerophi) CK(launch_fillval(p, 0.0, nx, ny, 1, 1, c.st));
@@ -2736,6 +2864,7 @@ int mgp_relax_gs(const mgp_box* valid, mgp_array* phi, const mgp_array* rhs, con
         if (rscale == 0.0) rscale = 1.0;
     }
     const bool fused = sweep_fusable(b);
+    if (fused) RC(c.field(&p2, nx, ny, 1));
     for (int it = 0; it < maxiters;) {
         if (fused) {   // several sweeps a launch where no norm is wanted between them
             const SweepPlan sp = sweep_plan<double>(nx, ny, b, tol > 0.0 ? 1 : maxiters - it, nullptr);
@@ -2752,7 +2881,7 @@ int mgp_relax_gs(const mgp_box* valid, mgp_array* phi, const mgp_array* rhs, con
             if (h / rscale <= tol) break;
         }
     }
-    RC(stage_out(p, phi, nx, ny, 1, c.st));
+    RC(c.back(p, phi, nx, ny, 1));
     return c.finish();
 }
 
@@ -2768,12 +2897,16 @@ int mgp_solve_bicgstab2(const mgp_box* valid, mgp_array* phi, const mgp_array* r
         return set_err(MGP_EINVAL, "solve_bicgstab2: the device sweep needs at least 4 cells per direction");
     const int nx = valid->nx, ny = valid->ny;
     OpCtx c;
+    c.span(phi, nx, ny);
+    c.span(rhs, nx, ny);
+    c.span(invdiags, nx, ny);
+    c.span(geo, valid);
     BicgArgs a;
     std::memset(&a, 0, sizeof a);
     Lv& L = a.L;
     L.nx = nx;
     L.ny = ny;
-    RC(c.in(phi, nx, ny, 1, &a.phi, "phi"));
+    RC(c.inout(phi, nx, ny, 1, &a.phi, "phi"));
     RC(c.in(rhs, nx, ny, 0, &a.rhs, "rhs"));
     RC(c.in(invdiags, nx, ny, 0, &L.invd, "invdiags"));
     RC(c.geo(geo, valid, &L.g));
@@ -2795,7 +2928,7 @@ int mgp_solve_bicgstab2(const mgp_box* valid, mgp_array* phi, const mgp_array* r
     a.zerophi = zerophi;
     a.dd = 0;
     CK(launch_bicgstab(a, c.st));
-    RC(stage_out(a.phi, phi, nx, ny, 1, c.st));
+    RC(c.back(a.phi, phi, nx, ny, 1));
     int dstat = 0;
     CK(cudaMemcpyAsync(&dstat, a.status, sizeof(int), cudaMemcpyDeviceToHost, c.st));
     RC(c.finish());
@@ -2815,13 +2948,16 @@ int mgp_restrict(const mgp_box* fine_valid, const mgp_array* fine, const mgp_box
     const int fx = fine_valid->nx + (offi == 0), fy = fine_valid->ny + (offj == 0);
     const int cx = crse_valid->nx + (offi == 0), cy = crse_valid->ny + (offj == 0);
     OpCtx c;
+    c.span(fine, fx, fy);
+    c.span(crse, cx, cy);
     DF f, cr;
     RC(c.in(fine, fx, fy, 0, &f, "fine"));
     RC(check_array(crse, cx, "crse"));
     const int cg = (crse->ngx > 0 || crse->ngy > 0) ? 1 : 0;
-    RC(c.field(&cr, cx, cy, cg));   // crse%data = zero (ghosts included)
+    if (!c.view(crse, cx, cy, 0, true, &cr)) RC(c.field(&cr, cx, cy, cg));   // crse%data = zero (ghosts included)
+    else if (cg) CK(launch_fillval(cr, 0.0, cx, cy, std::min(crse->ngx, 1), std::min(crse->ngy, 1), c.st));
     CK(launch_restrict(f, cr, crse_valid->nx, crse_valid->ny, rx, ry, kind, c.st));
-    RC(stage_out(cr, crse, cx, cy, cg, c.st));
+    RC(c.back(cr, crse, cx, cy, cg));
     return c.finish();
 }
 
@@ -2838,11 +2974,15 @@ int mgp_prolong(const mgp_box* fine_valid, mgp_array* fine, const mgp_box* crse_
         return set_err(MGP_ENOTSUP, "prolong: Needs updatin'");
     RC(ghost_cap(crse));
     OpCtx c;
+    c.span(fine, fine_valid->nx, fine_valid->ny);
+    c.span(crse, crse_valid->nx, crse_valid->ny);
+    c.span(fine_geo, fine_valid);
+    c.span(crse_geo, crse_valid);
     DF f, cr;
     Geo fg, cg;
     BCd b;
-    RC(c.in(fine, fine_valid->nx, fine_valid->ny, 1, &f, "fine"));
-    RC(c.in(crse, crse_valid->nx, crse_valid->ny, 1, &cr, "crse"));
+    RC(c.inout(fine, fine_valid->nx, fine_valid->ny, 1, &f, "fine"));
+    RC(c.inout(crse, crse_valid->nx, crse_valid->ny, 1, &cr, "crse"));
     RC(c.geo(fine_geo, fine_valid, &fg));
     RC(c.geo(crse_geo, crse_valid, &cg));
     RC(c.bc(crse_bc, crse_valid, 1, &b));
@@ -2862,8 +3002,8 @@ int mgp_prolong(const mgp_box* fine_valid, mgp_array* fine, const mgp_box* crse_
                          red + 2 * kRedBlocksMax, c.st));
         CK(launch_sub_mean(f, red + 2 * kRedBlocksMax, fine_valid->nx, fine_valid->ny, gx, gy, c.st));
     }
-    RC(stage_out(f, fine, fine_valid->nx, fine_valid->ny, 1, c.st));
-    RC(stage_out(cr, crse, crse_valid->nx, crse_valid->ny, 1, c.st));
+    RC(c.back(f, fine, fine_valid->nx, fine_valid->ny, 1));
+    RC(c.back(cr, crse, crse_valid->nx, crse_valid->ny, 1));
     return c.finish();
 }
 
