@@ -1761,7 +1761,6 @@ struct OpCtx {
     // with it (a staged one is read whole before anything is written, and
     // written back at the end).
     struct Span {
-        const void* data;
         uintptr_t lo, hi;
     };
     std::vector<Span> spans;
@@ -1772,7 +1771,7 @@ struct OpCtx {
         if (!a || !a->data || a->ngx < 0 || a->ngy < 0 || nxv < 1 || nyv < 1) return;
         const uintptr_t lo = (uintptr_t)a->data;
         const size_t n = (size_t)(nyv + 2 * a->ngy - 1) * array_ld(a, nxv) + nxv + 2 * a->ngx;
-        spans.push_back(Span{a, lo, lo + n * sizeof(double)});
+        spans.push_back(Span{lo, lo + n * sizeof(double)});
     }
     void span(const mgp_geo* g, const mgp_box* v) {
         if (!g) return;
@@ -1783,16 +1782,19 @@ struct OpCtx {
         span(&g->Jgup_yy, v->nx, v->ny + 1);
     }
     // Whether the array can be used where it lies, with g ghost layers; alone:
-    // only if no other array of the call overlaps it.
+    // only if no other array of the call overlaps it (its own span is the one
+    // that may; the same array passed twice has two).
     bool view(const mgp_array* a, int nxv, int nyv, int g, bool alone, DF* f) {
         if (a->ngx < g || a->ngy < g || ((uintptr_t)a->data & 7)) return false;
         const int ld = array_ld(a, nxv);
         const size_t n = (size_t)(nyv + 2 * a->ngy - 1) * ld + nxv + 2 * a->ngx;
         const uintptr_t lo = (uintptr_t)a->data, hi = lo + n * sizeof(double);
         if (!device_range(a->data, n * sizeof(double))) return false;
-        if (alone)
-            for (const Span& s : spans)
-                if (s.data != a && s.lo < hi && lo < s.hi) return false;
+        if (alone) {
+            int n_over = 0;
+            for (const Span& s : spans) n_over += s.lo < hi && lo < s.hi;
+            if (n_over > 1) return false;
+        }
         f->ld = ld;
         f->p = a->data + a->ngx + (size_t)a->ngy * ld;
         return true;

@@ -65,7 +65,31 @@ def _interior(phi):
     return Inner
 
 
+def _same(a):
+    """The array behind one descriptor, so that passing it twice passes one pointer twice."""
+    class Same:
+        valid, ngx, ngy, offi, offj = a.valid, a.ngx, a.ngy, a.offi, a.offj
+        one = a.c()
+
+        @staticmethod
+        def c():
+            return Same.one
+    return Same
+
+
+def _laplacian_onto_itself(M, w):
+    p = _same(w.phi)
+    M.compute_laplacian(p, p, w.geo, w.bc, False)
+
+
+def _residual_onto_itself(M, w):
+    p = _same(w.phi)
+    M.compute_residual(p, w.rhs, p, w.geo, w.bc, False)
+
+
 CALLS = {
+    "laplacian_onto_itself": _laplacian_onto_itself,
+    "residual_onto_itself": _residual_onto_itself,
     "residual": lambda M, w: M.compute_residual(w.out, w.rhs, w.phi, w.geo, w.bc, False),
     "residual_into_rhs": lambda M, w: M.compute_residual(w.rhs, w.rhs, w.phi, w.geo, w.bc, False),
     "residual_over_phi": lambda M, w: M.compute_residual(_interior(w.phi), w.rhs, w.phi, w.geo, w.bc, False),
