@@ -412,6 +412,7 @@ struct mgp_solver {
     int db = -1;
     double* d_ainv = nullptr;
     bool direct_large = false;
+    BlockBottom bb = {};   // the exact bottom of a dc of more than kDirectLargeCells cells (bb.mem), or empty
     // coarse cycle as a cooperative grid of grid_ctas CTAs (0: one CTA)
     int grid_ctas = 0;
     int coarse_cluster = 0;   // the grid_ctas CTAs form one thread-block cluster (2: one-CTA reduction order)
@@ -474,7 +475,7 @@ void solver_free(mgp_solver* s) {
     // pool (its stream may already be gone: a server worker's, say), as
     // cudaFree would have waited for the device
     cudaDeviceSynchronize();
-    for (void* p : {(void*)s->d_lv, (void*)s->d_shadow, (void*)s->d_tiny, (void*)s->d_tinymat, (void*)s->d_ainv, (void*)s->gm_base, (void*)s->gm_red,
+    for (void* p : {(void*)s->d_lv, (void*)s->d_shadow, (void*)s->d_tiny, (void*)s->d_tinymat, (void*)s->d_ainv, (void*)s->bb.mem, (void*)s->bb.items, (void*)s->gm_base, (void*)s->gm_red,
                     (void*)s->gctl.bar, (void*)s->gctl.part, (void*)s->d_ref, (void*)s->d_status,
                     (void*)s->d_bcbuf, (void*)s->d_red})
         dfree(p, nullptr);
@@ -577,6 +578,30 @@ int build_direct_large(mgp_solver* s, cudaStream_t st) {
     return MGP_OK;
 }
 
+// MGP_FLAG_DIRECT_LARGE on a level dc of more cells, which is then the
+// coarsest: its exact bottom by block cyclic reduction (mgp_bottom.cu), where
+// that has its memory and solves; else the reference bottom stays.  The line lies
+// at kDirectLargeCells because one launch of the dense inverse (8 MB, 5 us) beats
+// the reduction there (21 us on 33 x 35) and its inversion grows with the cube.
+int build_block_bottom(mgp_solver* s, cudaStream_t st) {
+    const Lv& L = s->lv[s->dc];
+    if (s->dc != s->maxdepth || !block_bottom_shape(L.nx, L.ny, L.bc, &s->bb)) {
+        s->bb = BlockBottom{};
+        return MGP_OK;
+    }
+    const BlockAlloc mem{[](void* ctx, size_t bytes) -> void* {
+                             void* p = nullptr;
+                             if (dmalloc(&p, bytes, (cudaStream_t)ctx) == cudaSuccess) return p;
+                             cudaGetLastError();
+                             return nullptr;
+                         },
+                         [](void* ctx, void* p) { dfree(p, (cudaStream_t)ctx); }, st};
+    bool ok = false;
+    const cudaError_t e = block_bottom_build(&s->bb, L.g, L.bc, L.nx, L.ny, mem, st, &ok);
+    if (e != cudaSuccess) return set_err(MGP_ECUDA, "direct coarse operator: %s", cudaGetErrorString(e));
+    return MGP_OK;
+}
+
 // MGP_FLAG_DIRECT_COARSE: the first level from dc down with at most
 // kDirectCells cells becomes the bottom, solved with its operator's inverse.
 // The operator (homogeneous BCs) is assembled on the device column by column,
@@ -589,6 +614,8 @@ int build_direct_coarse(mgp_solver* s, cudaStream_t st) {
     if ((s->flags & MGP_FLAG_DIRECT_LARGE) && (long)s->lv[s->dc].nx * s->lv[s->dc].ny <= kDirectLargeCells &&
         (long)s->lv[s->dc].nx * s->lv[s->dc].ny > kDirectCells)
         return build_direct_large(s, st);
+    if ((s->flags & MGP_FLAG_DIRECT_LARGE) && (long)s->lv[s->dc].nx * s->lv[s->dc].ny > kDirectLargeCells)
+        return build_block_bottom(s, st);
     int db = -1;
     for (int d = s->dc; d <= s->maxdepth; ++d)
         if ((long)s->lv[d].nx * s->lv[d].ny <= kDirectCells) {
@@ -1085,6 +1112,11 @@ int coarse_cycle(mgp_solver* s, int d, int numcycles, int nd, int nu, int nb) {
     if (s->direct_large && d == s->db) {   // the exact bottom at dc
         const Lv& L = s->lv[d];
         CK(launch_direct_apply(L.e, L.r, s->d_ainv, L.nx, L.ny, s->stream));
+        return MGP_OK;
+    }
+    if (s->bb.mem && d == s->dc) {
+        const Lv& L = s->lv[d];
+        CK(launch_block_bottom(s->bb, L.e, L.r, s->stream));
         return MGP_OK;
     }
     CoarseArgs a;
@@ -1910,6 +1942,7 @@ size_t solver_device_bytes(const mgp_solver* s) {
         const size_t n = (size_t)s->lv[s->db].nx * s->lv[s->db].ny;
         bytes += n * n * sizeof(double);
     }
+    bytes += s->bb.bytes;
     return bytes;
 }
 // Memory the solvers' pool on the current device holds but no solver uses
@@ -2050,6 +2083,7 @@ struct Plan {
     std::vector<Table<ProlongJob<float, double>>> pro3264;
     Table<CoarseJob> coarse;
     int coarse_smem = 0;
+    std::vector<mgp_solver*> block;   // problems whose bottom is solved by block cyclic reduction, in turn
     Table<DirectJob> direct;   // problems whose bottom is the coarse-cycle level, solved by its inverse
     Table<CellJob<float, double>> r_to32;   // mixed: level-0 rhs rounded to FP32
     Table<CellJob<float, float>> guess32;   // e = r invd on FP32 level 0
@@ -2141,6 +2175,8 @@ void build_plan(Plan& P, const std::vector<mgp_solver*>& ss, const std::vector<i
         if (s->direct_large && s->db == s->dc) {
             const Lv& B = s->lv[s->dc];
             P.direct.push(DirectJob{B.e, B.r, s->d_ainv, B.nx, B.ny}, direct_apply_blocks(B.nx, B.ny));
+        } else if (s->bb.mem) {
+            P.block.push_back(s);
         } else {
             CoarseJob cj;
             cj.a = coarse_args_of(s, s->dc, nd, nu, nb);
@@ -2249,6 +2285,7 @@ int lockstep_iteration(Plan& P, Lockstep* ls, int nd, int nu, cudaStream_t st) {
     }
     CK(launch_coarse_jobs(P.coarse.dj, P.coarse.n(), P.coarse_smem, st));
     CK(launch_direct_jobs(P.direct.dj, P.direct.dp, P.direct.n(), P.direct.blocks(), st));
+    for (mgp_solver* s : P.block) CK(launch_block_bottom(s->bb, s->lv[s->dc].e, s->lv[s->dc].r, st));
     for (int d = P.D - 1; d >= 0; --d) {   // up: fill the coarse correction, prolong, smooth (MG:818-845)
         CK(launch_fill_jobs(P.fpost64[d].dj, P.fpost64[d].dp, P.fpost64[d].n(), P.fpost64[d].blocks(), P.fpost_ph[d],
                             st));

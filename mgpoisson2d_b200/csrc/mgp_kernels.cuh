@@ -408,4 +408,30 @@ cudaError_t launch_bicgstab(const BicgArgs& a, cudaStream_t st);
 cudaError_t launch_relax_block(const Lv& L, const DF& phi, const DF& rhs, int homog, double omega, int sweeps,
                                int dd, int* status, cudaStream_t st);
 
+// The exact bottom of a level of more than kDirectLargeCells cells (mgp_bottom.cu):
+// block cyclic reduction over its lines of m cells.
+constexpr int kBlockLineMax = 160;                  // an inverted block fits one CTA's shared memory
+constexpr int kBlockStepsMax = 16;
+constexpr size_t kBlockBytesMax = 256ull << 20;     // of factors
+struct BlockBottom {
+    int m, lines, along_y, steps;                   // lines are rows (along_y) or columns of the level
+    int ndown[kBlockStepsMax + 1], odown[kBlockStepsMax + 1], nup[kBlockStepsMax + 1], oup[kBlockStepsMax + 1];
+    double *mem, *dinv, *p, *q, *fg, *r;            // one block of memory, nullptr without a factorisation
+    int4* items;
+    size_t bytes;
+};
+struct BlockAlloc {
+    void* (*get)(void* ctx, size_t bytes);          // nullptr when there is no memory
+    void (*put)(void* ctx, void* p);
+    void* ctx;
+};
+// Whether a level of these sides and types has such a bottom; sets its shape.
+bool block_bottom_shape(int nx, int ny, const BCd& bc, BlockBottom* b);
+// Factorises the level's operator (homogeneous sides) and tries it; synchronises st.
+// *ok: it solves.  Without memory or a sound factorisation *b is empty.
+cudaError_t block_bottom_build(BlockBottom* b, const Geo& g, const BCd& bc, int nx, int ny, const BlockAlloc& mem,
+                               cudaStream_t st, bool* ok);
+// e = A^-1 r on the level's cells (ghosts untouched).
+cudaError_t launch_block_bottom(const BlockBottom& b, const DF& e, const DF& r, cudaStream_t st);
+
 }  // namespace mgp
