@@ -17,7 +17,9 @@
 
 #include <cuda_bf16.h>
 
+#include "mgp_ddsweep.cuh"
 #include "mgp_kernels.cuh"
+#include "mgp_sweep.cuh"
 
 namespace mgp {
 
@@ -484,8 +486,8 @@ struct BlockScope {
     __device__ static int size() { return blockDim.x; }
     __device__ static void sync() { __syncthreads(); }
     __device__ static int rrank() { return threadIdx.x; }
-    __device__ static int rsize() { return blockDim.x; }
-    __device__ static bool ractive() { return true; }
+    __device__ static int rsize() { return kReduceThreads; }
+    __device__ static bool ractive() { return threadIdx.x < kReduceThreads; }
 };
 struct GridScope {
     __device__ static int cta() { return blockIdx.x; }
@@ -512,7 +514,7 @@ __device__ __forceinline__ void cluster_barrier() {
 }
 // kOrdered: its reductions are accumulated by the first CTA alone, thread t
 // summing cells t, t + blockDim, ... as BlockScope's thread t does, and
-// combined by the same block tree (the CTAs have BlockScope's kCoarseThreads
+// combined by the same block tree (the CTAs have its kReduceThreads
 // threads), so every result -- the sweeps, whose colour passes do not depend
 // on which thread updates a cell, and the reductions -- has the bits of the
 // one-CTA kernel; the result reaches the other CTAs through global memory.
@@ -1519,10 +1521,49 @@ __device__ __forceinline__ bool fusable_sides(const BCd& b) {
     return true;
 }
 
+// Sweeps of a level that fits one of the windows of mgp_sweep.cuh and
+// mgp_ddsweep.cuh, by the one-CTA kernels: the operator in registers through the
+// call and phi in planes, where b_sweep9 and b_sweep_dd read both from the level's
+// arrays in every phase: 32^2 cells, nine points, 5.5 -> 2.2 us a sweep; the cycle
+// below 32^2 (nine-point, eight sweeps a visit) 261 -> 146 us.  Bound by the
+// barriers and the latency of the chains between them.  The same operations in the
+// same order, so the same bits.
+using DdFlat64 = DdShape<double, 32>;   // 64 x 32
+using DdTall64 = DdShape<double, 16>;   // 32 x 64
+union HeldWork {
+    struct {
+        double planes[4 * (Small64::PS > Flat64::PS ? Small64::PS : Flat64::PS)];
+        double strips[4 * kStrip * kAlong];
+    };
+    double dd[4 * (DdFlat64::PS > DdTall64::PS ? DdFlat64::PS : DdTall64::PS)];
+};
+static_assert(Small64::kThreads == kCoarseThreads && Flat64::kThreads == kCoarseThreads &&
+                  32 * DdFlat64::NW == kCoarseThreads && 32 * DdTall64::NW == kCoarseThreads,
+              "a window takes the CTA");
+template <class C>
+__device__ __noinline__ void held_sweeps(HeldWork& H, const DF& phi, const DF& rhs, const DF& invd, const Geo& g,
+                                         const BCd& b, int homog, int nx, int ny, double omega, int sweeps) {
+    sweep_window<C, false, true>(H.planes, H.strips, phi, phi, rhs, invd, g, b, homog, nx, ny, 1, 1, omega, sweeps, 0, 0);
+    __syncthreads();
+}
+
 template <class S>
-__device__ void b_relax9(const Lv& L, const DF& phi, const DF& rhs, int homog, double omega, int sweeps) {
+__device__ void b_relax9(const Lv& L, const DF& phi, const DF& rhs, int homog, double omega, int sweeps,
+                         HeldWork* H = nullptr) {
     const int nx = L.nx, ny = L.ny;
     if (fusable_sides(L.bc)) {
+        if constexpr (!S::kGrid) {
+            if (H && sweeps > 0 && nx >= 4 && ny >= 4) {
+                if (nx <= Small64::WX && ny <= Small64::WY) {
+                    held_sweeps<Small64>(*H, phi, rhs, L.invd, L.g, L.bc, homog, nx, ny, omega, sweeps);
+                    return;
+                }
+                if (nx <= Flat64::WX && ny <= Flat64::WY) {
+                    held_sweeps<Flat64>(*H, phi, rhs, L.invd, L.g, L.bc, homog, nx, ny, omega, sweeps);
+                    return;
+                }
+            }
+        }
         for (int it = 0; it < sweeps; ++it) b_sweep9<S>(phi, rhs, L.invd, L.g, L.bc, homog, nx, ny, omega);
         return;
     }
@@ -1558,12 +1599,35 @@ __device__ void b_sweep_dd(const Lv& L, const DF& phi, const DF& modrhs, int hom
 }
 
 // The deferred-correction smoother (DD:153-334).  modrhs is computed once per call, into L.w.
+template <class B>
+__device__ __noinline__ void held_dd_sweeps(HeldWork& H, const DF& phi, const Lv& L, double omega, int sweeps) {
+    dd_window<B, false, true>(H.dd, phi, phi, L.w, L.invd, L.g.xx, L.g.yy, mirror_of<double>(L.bc), L.g.idx, L.g.idy, L.nx,
+                              L.ny, 1, 1, omega, sweeps, 0, 0);
+    __syncthreads();
+}
+
 template <class S>
-__device__ void b_relax_dd(const Lv& L, const DF& phi, const DF& rhs, int homog, double omega, int sweeps) {
+__device__ void b_relax_dd(const Lv& L, const DF& phi, const DF& rhs, int homog, double omega, int sweeps,
+                           HeldWork* H = nullptr) {
     const int nx = L.nx, ny = L.ny;
     if (sweeps == 0) return;
     SLOOP(k, nx * ny) AT(L.w, k % nx, k / nx) = dd_modrhs(phi, rhs, L.g, nx, ny, k % nx, k / nx);
     S::sync();
+    if constexpr (!S::kGrid) {
+        bool lah = true;   // the ghosts dd_window knows
+        for (int s = 0; s < 4; ++s)
+            lah = lah && (L.bc.type[s] == T_DIRI || L.bc.type[s] == T_NEUM) && L.bc.mode[s] == M_LAH;
+        if (H && lah && sweeps > 0) {
+            if (nx <= DdTall64::WX && ny <= DdTall64::WY) {
+                held_dd_sweeps<DdTall64>(*H, phi, L, omega, sweeps);
+                return;
+            }
+            if (nx <= DdFlat64::WX && ny <= DdFlat64::WY) {
+                held_dd_sweeps<DdFlat64>(*H, phi, L, omega, sweeps);
+                return;
+            }
+        }
+    }
     for (int it = 0; it < sweeps; ++it) b_sweep_dd<S>(L, phi, L.w, homog, omega);
 }
 
@@ -1591,15 +1655,16 @@ __device__ void b_apply(const Lv& L, const DF& out, const DF& phi, const DF& rhs
 }
 
 template <class S>
-__device__ void b_relax(const Lv& L, const DF& phi, const DF& rhs, int homog, double omega, int sweeps, int dd) {
-    if (dd) b_relax_dd<S>(L, phi, rhs, homog, omega, sweeps);
-    else b_relax9<S>(L, phi, rhs, homog, omega, sweeps);
+__device__ void b_relax(const Lv& L, const DF& phi, const DF& rhs, int homog, double omega, int sweeps, int dd,
+                        HeldWork* H = nullptr) {
+    if (dd) b_relax_dd<S>(L, phi, rhs, homog, omega, sweeps, H);
+    else b_relax9<S>(L, phi, rhs, homog, omega, sweeps, H);
 }
 
 // solve_bicgstab2 (P2:2253-2477; DD:339-566 with dd = 1).  Status: DST_OK or DST_NONFINITE.
 template <class S>
 __device__ int b_bicgstab(const Lv& L, const DF& phi, const DF& rhs, int homog, double tol, int max_iters,
-                          int max_restarts, int zerophi, int dd, double* sh) {
+                          int max_restarts, int zerophi, int dd, double* sh, HeldWork* H = nullptr) {
     const double reps = 1.0e-12, hang = 1.0e-7, small = 1.0e-30;
     const int norm_type = dd ? 0 : 2;
     const double relax_omega = dd ? 4.0 / 5.0 : 1.0 - 1.0 / 3.0;
@@ -1643,7 +1708,7 @@ __device__ int b_bicgstab(const Lv& L, const DF& phi, const DF& rhs, int homog, 
             S::sync();
         }
         b_mul<S>(pt, p, L.invd, nx, ny);
-        b_relax<S>(L, pt, p, 1, relax_omega, 2, dd);
+        b_relax<S>(L, pt, p, 1, relax_omega, 2, dd, H);
         b_apply<S>(L, v, pt, p, 1, 0, dd);
         const double m = b_dot<S>(rt, v, nx, ny, vol, sh);
         alpha[0] = rho[1] / m;
@@ -1657,7 +1722,7 @@ __device__ int b_bicgstab(const Lv& L, const DF& phi, const DF& rhs, int homog, 
         }
         if ((norm[0] > tol * initial_norm) && (norm[0] > reps * initial_rnorm)) {
             b_mul<S>(st, r, L.invd, nx, ny);
-            b_relax<S>(L, st, r, 1, relax_omega, 2, dd);
+            b_relax<S>(L, st, r, 1, relax_omega, 2, dd, H);
             b_apply<S>(L, t, st, r, 1, 0, dd);
             const double tr = b_dot<S>(t, r, nx, ny, vol, sh);
             const double tt = b_dot<S>(t, t, nx, ny, vol, sh);
@@ -1967,7 +2032,7 @@ __device__ void b_direct(const Lv& L, const double* ainv) {
 // tiny (BlockScope only, nullable): the levels' dense forms, W their work space.
 template <class S>
 __device__ int coarse_body(const Lv* lv, const CoarseArgs& a, double* sh, const TinyLv* tiny = nullptr,
-                           TinyWork* W = nullptr) {
+                           TinyWork* W = nullptr, HeldWork* H = nullptr) {
     int cnt[32];
     const double relax_omega = a.dd ? 4.0 / 5.0 : 1.0;
     int d = a.d0;
@@ -1980,7 +2045,7 @@ __device__ int coarse_body(const Lv* lv, const CoarseArgs& a, double* sh, const 
                 return;
             }
         }
-        b_relax<S>(lv[l], lv[l].e, lv[l].r, 1, relax_omega, sweeps, a.dd);
+        b_relax<S>(lv[l], lv[l].e, lv[l].r, 1, relax_omega, sweeps, a.dd, H);
     };
 visit:
     {
@@ -1995,7 +2060,7 @@ visit:
             int s;
             if constexpr (S::kGrid) s = b_bicgstab<S>(L, L.e, L.r, 1, 1.0e-6, 80, 5, 0, a.dd, sh);
             else s = is_tiny(d) ? tiny_bicgstab(tiny[d], L, a.dd, *W)
-                                : b_bicgstab<S>(L, L.e, L.r, 1, 1.0e-6, 80, 5, 0, a.dd, sh);
+                                : b_bicgstab<S>(L, L.e, L.r, 1, 1.0e-6, 80, 5, 0, a.dd, sh, H);
             if (s) st = s;
             goto up;
         }
@@ -2030,8 +2095,9 @@ finish:
 }
 
 __global__ void __launch_bounds__(kCoarseThreads, 1) k_coarse_cycle(CoarseArgs a) {
-    __shared__ double sh[kCoarseThreads];
-    const int s = coarse_body<BlockScope>(a.lv, a, sh);
+    __shared__ double sh[64];
+    __shared__ HeldWork H;
+    const int s = coarse_body<BlockScope>(a.lv, a, sh, nullptr, nullptr, &H);
     if (threadIdx.x == 0) set_status(a.status, s);
 }
 
@@ -2051,12 +2117,14 @@ __device__ __forceinline__ void rebase(DF& f, double* base) { f.p = base + (size
 // The same cycle with every coarse level held in shared memory: the levels'
 // arrays are copied in (the corrections with their ghosts, the operands, the
 // finest level's right-hand side), the cycle runs, the corrections go back.
-__device__ __forceinline__ void coarse_cycle_smem(const CoarseArgs& a) {
+union CoarseWork {   // no routine uses both
+    TinyWork tiny;
+    HeldWork held;
+};
+__device__ __forceinline__ void coarse_cycle_smem(const CoarseArgs& a, double* sh, CoarseWork& work) {
     extern __shared__ double smem[];
-    __shared__ double sh[kCoarseThreads];
     __shared__ Lv sl[kMaxCoarseLevels];
     __shared__ TinyLv st_[kMaxCoarseLevels];
-    __shared__ TinyWork W;
     const int nl = a.maxdepth - a.d0 + 1;
     if (threadIdx.x < nl) {
         Lv L = a.shadow[a.d0 + threadIdx.x];
@@ -2098,7 +2166,8 @@ __device__ __forceinline__ void coarse_cycle_smem(const CoarseArgs& a) {
     }
     cp_async_wait_all();
     __syncthreads();
-    const int s = coarse_body<BlockScope>(sl - a.d0, a, sh, a.tiny ? st_ - a.d0 : nullptr, &W);
+    const int s = coarse_body<BlockScope>(sl - a.d0, a, sh, a.tiny ? st_ - a.d0 : nullptr, &work.tiny,
+                                          &work.held);
     for (int k = 0; k < nl; ++k) {
         const Lv &S = sl[k], &G = a.lv[a.d0 + k];
         b_copy(G.e, S.e, -1, S.nx + 1, -1, S.ny + 1);
@@ -2106,17 +2175,22 @@ __device__ __forceinline__ void coarse_cycle_smem(const CoarseArgs& a) {
     if (threadIdx.x == 0) set_status(a.status, s);
 }
 
-__global__ void __launch_bounds__(kCoarseThreads, 1) k_coarse_cycle_smem(CoarseArgs a) { coarse_cycle_smem(a); }
+__global__ void __launch_bounds__(kCoarseThreads, 1) k_coarse_cycle_smem(CoarseArgs a) {
+    __shared__ double sh[64];
+    __shared__ CoarseWork work;
+    coarse_cycle_smem(a, sh, work);
+}
 
 // The coarse cycles of a lockstep batch: a CTA per problem, each with its own
 // arguments (staged in shared memory when its levels fit, else in place).
 __global__ void __launch_bounds__(kCoarseThreads, 1) k_coarse_jobs(const CoarseJob* __restrict__ jobs) {
+    __shared__ double sh[64];
+    __shared__ CoarseWork work;
     const CoarseArgs& a = jobs[blockIdx.x].a;
     if (a.shadow && a.smem_bytes > 0) {
-        coarse_cycle_smem(a);
+        coarse_cycle_smem(a, sh, work);
     } else {
-        __shared__ double sh[kCoarseThreads];
-        const int s = coarse_body<BlockScope>(a.lv, a, sh);
+        const int s = coarse_body<BlockScope>(a.lv, a, sh, nullptr, nullptr, &work.held);
         if (threadIdx.x == 0) set_status(a.status, s);
     }
 }
@@ -2533,8 +2607,8 @@ cudaError_t coarse_kernels_init() {
 // The coarse sub-cycle over a cooperative grid of a.grid_ctas CTAs (all
 // resident: one per SM at most), for hierarchies whose coarsest level is too
 // large for one CTA (the schedule stops coarsening at an odd side).
-__global__ void __launch_bounds__(kCoarseThreads, 1) k_coarse_cycle_grid(CoarseArgs a) {
-    __shared__ double sh[kCoarseThreads];
+__global__ void __launch_bounds__(kGridThreads, 1) k_coarse_cycle_grid(CoarseArgs a) {
+    __shared__ double sh[64];
     if (threadIdx.x == 0) {
         s_gctl = a.gctl;
         s_gred = 0;
@@ -2549,7 +2623,7 @@ __global__ void __launch_bounds__(kCoarseThreads, 1) k_coarse_cycle_grid(CoarseA
 // cluster barriers, for coarsest levels that one CTA cannot stage in shared
 // memory, where the grid version's time is its barriers.  kOrdered
 // (a.cluster == 2): the one-CTA kernel's reduction order and bits.
-static_assert(kClusterThreads == kCoarseThreads, "the cluster CTAs reduce in the one-CTA kernel's order");
+static_assert(kClusterThreads == kReduceThreads, "the cluster CTAs reduce in the one-CTA kernel's order");
 // Two CTAs an SM (128 registers, some spilled): a cluster CTA fits beside a
 // sweep CTA of another stream, so under a server's concurrent solves a
 // cluster does not wait for sixteen idle SMs in one GPC (served p99 at 10
@@ -2621,7 +2695,7 @@ int coarse_grid_ctas_max() {
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_coarse_cycle_grid, kCoarseThreads, 0) !=
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_coarse_cycle_grid, kGridThreads, 0) !=
             cudaSuccess) {
         cudaGetLastError();
         return 0;
@@ -2687,7 +2761,7 @@ cudaError_t launch_coarse_cycle(const CoarseArgs& a, cudaStream_t st) {
     if (a.grid_ctas > 1) {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(a.grid_ctas);
-        cfg.blockDim = dim3(kCoarseThreads);
+        cfg.blockDim = dim3(kGridThreads);
         cfg.stream = st;
         cudaLaunchAttribute at[1];
         at[0].id = cudaLaunchAttributeCooperative;
@@ -2710,9 +2784,10 @@ cudaError_t launch_coarse_cycle(const CoarseArgs& a, cudaStream_t st) {
 }
 
 __global__ void __launch_bounds__(kCoarseThreads, 1) k_bicgstab(BicgArgs a) {
-    __shared__ double sh[kCoarseThreads];
+    __shared__ double sh[64];
+    __shared__ HeldWork H;
     const int s = b_bicgstab<BlockScope>(a.L, a.phi, a.rhs, a.homog, a.tol, a.max_iters, a.max_restarts, a.zerophi,
-                                         a.dd, sh);
+                                         a.dd, sh, &H);
     if (threadIdx.x == 0) set_status(a.status, s);
 }
 

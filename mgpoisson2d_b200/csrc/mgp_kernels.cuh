@@ -92,8 +92,9 @@ constexpr int kDirectLargeCells = 1024;
 constexpr int kGjPanel = 16;
 
 constexpr int kMaxCoarseLevels = 16;
-// Largest staged coarse hierarchy (bytes of dynamic shared memory).
-constexpr int kCoarseSmemMax = 200 * 1024;
+// Largest staged coarse hierarchy (bytes of dynamic shared memory; the kernels'
+// own take 44 KB beside it).
+constexpr int kCoarseSmemMax = 180 * 1024;
 
 // Columns of a tiny level's matrices into T.m (device memory), a CTA a column.
 // scratch: tiny_scratch_doubles(L) doubles.
@@ -111,7 +112,9 @@ struct BicgArgs {
     int* status;
 };
 
-constexpr int kCoarseThreads = 256;
+constexpr int kCoarseThreads = 512;   // of the one-CTA coarse cycle: the shape of mgp_sweep.cuh's windows
+constexpr int kReduceThreads = 256;   // of them that accumulate its reductions
+constexpr int kGridThreads = 256;     // threads per CTA of the cooperative-grid coarse cycle
 constexpr int kClusterThreads = 256;   // threads per CTA of the cluster coarse cycle
 
 long long launch_count();
