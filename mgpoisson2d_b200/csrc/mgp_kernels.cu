@@ -1598,7 +1598,6 @@ __device__ void b_sweep_dd(const Lv& L, const DF& phi, const DF& modrhs, int hom
     }
 }
 
-// The deferred-correction smoother (DD:153-334).  modrhs is computed once per call, into L.w.
 template <class B>
 __device__ __noinline__ void held_dd_sweeps(HeldWork& H, const DF& phi, const Lv& L, double omega, int sweeps) {
     dd_window<B, false, true>(H.dd, phi, phi, L.w, L.invd, L.g.xx, L.g.yy, mirror_of<double>(L.bc), L.g.idx, L.g.idy, L.nx,
@@ -1606,13 +1605,10 @@ __device__ __noinline__ void held_dd_sweeps(HeldWork& H, const DF& phi, const Lv
     __syncthreads();
 }
 
+// Its sweeps for the modified rhs in L.w.
 template <class S>
-__device__ void b_relax_dd(const Lv& L, const DF& phi, const DF& rhs, int homog, double omega, int sweeps,
-                           HeldWork* H = nullptr) {
+__device__ void b_dd_sweeps(const Lv& L, const DF& phi, int homog, double omega, int sweeps, HeldWork* H) {
     const int nx = L.nx, ny = L.ny;
-    if (sweeps == 0) return;
-    SLOOP(k, nx * ny) AT(L.w, k % nx, k / nx) = dd_modrhs(phi, rhs, L.g, nx, ny, k % nx, k / nx);
-    S::sync();
     if constexpr (!S::kGrid) {
         bool lah = true;   // the ghosts dd_window knows
         for (int s = 0; s < 4; ++s)
@@ -1629,6 +1625,16 @@ __device__ void b_relax_dd(const Lv& L, const DF& phi, const DF& rhs, int homog,
         }
     }
     for (int it = 0; it < sweeps; ++it) b_sweep_dd<S>(L, phi, L.w, homog, omega);
+}
+// The deferred-correction smoother (DD:153-334).  modrhs is computed once per call, into L.w.
+template <class S>
+__device__ void b_relax_dd(const Lv& L, const DF& phi, const DF& rhs, int homog, double omega, int sweeps,
+                           HeldWork* H = nullptr) {
+    const int nx = L.nx, ny = L.ny;
+    if (sweeps == 0) return;
+    SLOOP(k, nx * ny) AT(L.w, k % nx, k / nx) = dd_modrhs(phi, rhs, L.g, nx, ny, k % nx, k / nx);
+    S::sync();
+    b_dd_sweeps<S>(L, phi, homog, omega, sweeps, H);
 }
 
 // out = rhs - L[phi] (mode 1) or L[phi] (mode 0); fills phi's ghosts first as the Fortran routines do.
@@ -1752,6 +1758,219 @@ __device__ int b_bicgstab(const Lv& L, const DF& phi, const DF& rhs, int homog, 
     }
     b_axpby<S>(phi, e, 1.0, 1.0, nx, ny, 1);
     return isfinite(norm[0]) ? DST_OK : DST_NONFINITE;
+}
+
+// ---------------------------------------------------------------------------
+// b_bicgstab(L, L.e, L.r, 1, 1e-6, 80, 5, 0) on a level the one-CTA kernel holds in
+// shared memory, statement for statement, with the vectors in registers: a thread
+// owns the cells k = t, t + 512, ... (kCells of them at most).  The general
+// routine's iteration is some seventy barrier-separated phases with an integer
+// division a cell, on 18 x 11 cells 300 clocks each; here the two preconditioner
+// calls (the sweep windows), an operator pass each and four reductions, of one
+// barrier and up to two values each, remain: deferred correction's cycle above an
+// 18 x 11 bottom 339 -> 257 us, the 9-point bottom of 41 x 22 cells 1.12 -> 0.82 ms
+// (66 k clocks an iteration, four sweeps of 7 k the most of it).  The reductions sum in another order
+// than b_reduce, so results agree to rounding; a level's size alone decides that
+// it is solved here, so they are the same alone and in a batch.
+// ---------------------------------------------------------------------------
+// a = sum of a, b = sum (max with kMax) of b over the CTA, the same bits in every
+// thread; sh: 64 doubles, flip alternates its halves.
+template <bool kMax>
+__device__ __forceinline__ void cell_reduce(double& a, double& b, double* sh, int& flip) {
+    const auto op = [](double x, double y) { return kMax ? fmax(x, y) : x + y; };
+    double* buf = sh + 32 * flip;
+    flip ^= 1;
+    for (int o = 16; o > 0; o >>= 1) {
+        const double u = __shfl_xor_sync(0xffffffffu, a, o), w = __shfl_xor_sync(0xffffffffu, b, o);
+        a = a + u;
+        b = op(b, w);
+    }
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (lane == 0) {
+        buf[warp] = a;
+        buf[16 + warp] = b;
+    }
+    __syncthreads();
+    a = buf[lane & 15];
+    b = buf[16 + (lane & 15)];
+    for (int o = 8; o > 0; o >>= 1) {
+        const double u = __shfl_xor_sync(0xffffffffu, a, o), w = __shfl_xor_sync(0xffffffffu, b, o);
+        a = a + u;
+        b = op(b, w);
+    }
+}
+static_assert(kCoarseThreads == 16 * 32, "cell_reduce combines sixteen warps");
+
+// Two preconditioner sweeps on z for the right-hand side f, and the ghosts the operator reads.
+__device__ __noinline__ void cell_precondition(const Lv& L, const DF& z, const DF& f, int dd, HeldWork& H) {
+    if (dd) {
+        b_dd_sweeps<BlockScope>(L, z, 1, 4.0 / 5.0, 2, &H);
+    } else {
+        b_relax9<BlockScope>(L, z, f, 1, 1.0 - 1.0 / 3.0, 2, &H);
+        b_fill<BlockScope>(z, L.g, L.bc, 1, 0, L.nx, L.ny);   // P2:935
+    }
+}
+
+template <bool kDd, int kCells>
+__device__ __noinline__ int cell_bicgstab(const Lv& L_, double* sh, HeldWork& H) {
+    const double tol = 1.0e-6, reps = 1.0e-12, hang = 1.0e-7, small = 1.0e-30;
+    const int max_iters = 80, max_restarts = 5;
+    const Lv& L = L_;
+    const DF phi = L.e, pt = L.pt, st = L.st, pp = L.pp, rr = L.rr;
+    const int nx = L.nx, ny = L.ny, n = nx * ny;
+    const double vol = L.g.dx * L.g.dy;
+    int ci[kCells], cj[kCells];
+    bool on[kCells];
+    double r[kCells], rt[kCells], p[kCells], v[kCells], e[kCells], d[kCells];
+#pragma unroll
+    for (int q = 0; q < kCells; ++q) {
+        const int k = (int)threadIdx.x + q * kCoarseThreads;
+        on[q] = k < n;
+        cj[q] = on[q] ? k / nx : 0;
+        ci[q] = on[q] ? k - cj[q] * nx : 0;
+        d[q] = on[q] ? AT(L.invd, ci[q], cj[q]) : 0.0;
+        r[q] = rt[q] = p[q] = v[q] = e[q] = 0.0;
+    }
+    for (int k = threadIdx.x; k < (nx + 2) * (ny + 2); k += kCoarseThreads) {
+        const int j = k / (nx + 2) - 1, i = k - (j + 1) * (nx + 2) - 1;
+        AT(pt, i, j) = 0.0;
+        AT(st, i, j) = 0.0;
+    }
+    int flip = 0;
+    const auto each = [&](auto f) {
+#pragma unroll
+        for (int q = 0; q < kCells; ++q)
+            if (on[q]) f(q, ci[q], cj[q]);
+    };
+    const auto lap = [&](const DF& z, int i, int j) {
+        return kDd ? dd_apply(z, L.g, L.bc, nx, ny, i, j) : apply9(z, L.g, L.bc, 1, nx, ny, i, j);
+    };
+    double rho_next = 0.0;   // rt . r, with the norm of r
+    const auto norm_rho = [&]() {
+        double a = 0.0, b = 0.0;
+        each([&](int q, int, int) {
+            a = a + rt[q] * r[q];
+            b = kDd ? fmax(b, fabs(r[q])) : b + r[q] * r[q];
+        });
+        cell_reduce<kDd>(a, b, sh, flip);
+        rho_next = vol * a;
+        return kDd ? b : sqrt(vol * b);
+    };
+    const auto residual = [&]() {   // r = rhs - L[phi], rt = r, e = 0
+        if (!kDd) b_fill<BlockScope>(phi, L.g, L.bc, 1, 0, nx, ny);
+        else __syncthreads();
+        each([&](int q, int i, int j) {
+            r[q] = AT(L.r, i, j) - lap(phi, i, j);
+            rt[q] = r[q];
+            e[q] = 0.0;
+        });
+        return norm_rho();
+    };
+    const auto add = [&]() {   // phi += e; DD: with the ghosts every term of e carries
+        __syncthreads();
+        each([&](int q, int i, int j) { AT(phi, i, j) = AT(phi, i, j) + e[q]; });
+        __syncthreads();
+        if (kDd) b_fill<BlockScope>(phi, L.g, L.bc, 1, 1, nx, ny);
+    };
+    // z = two sweeps for the right-hand side x (in f), w = L[z]
+    const auto precondition = [&](const DF& z, const DF& f, const double* x, double* w, double* zv) {
+        each([&](int q, int i, int j) {
+            AT(z, i, j) = x[q] * d[q];
+            AT(f, i, j) = x[q];
+        });
+        __syncthreads();
+        if (kDd) {
+            each([&](int, int i, int j) { AT(L.w, i, j) = dd_modrhs(z, f, L.g, nx, ny, i, j); });
+            __syncthreads();
+        }
+        cell_precondition(L, z, f, kDd, H);
+        each([&](int q, int i, int j) {
+            w[q] = lap(z, i, j);
+            zv[q] = AT(z, i, j);
+        });
+    };
+    double rho[4] = {0, 0, 0, 0}, norm[2], alpha[2] = {0, 0}, beta[2] = {0, 0}, omg[2] = {0, 0};
+    int recount = 0, i = 0, restarts = 0, init = 1;
+    norm[0] = residual();
+    const double initial_norm = norm[0], initial_rnorm = norm[0];
+    norm[1] = norm[0];
+    while (((i < max_iters) && (norm[0] > tol * norm[1])) && (norm[1] > 0.0)) {
+        i = i + 1;
+        norm[1] = norm[0];
+        alpha[1] = alpha[0];
+        beta[1] = beta[0];
+        omg[1] = omg[0];
+        rho[3] = rho[2];
+        rho[2] = rho[1];
+        rho[1] = rho_next;
+        if (rho[1] == 0.0) {
+            add();
+            return 0;
+        }
+        if (!init) beta[1] = (rho[1] / rho[2]) * (alpha[1] / omg[1]);
+        each([&](int q, int, int) { p[q] = init ? r[q] : beta[1] * (p[q] - omg[1] * v[q]) + r[q]; });
+        init = 0;
+        double z[kCells];
+        precondition(pt, pp, p, v, z);
+        double m = 0.0, unused = 0.0;
+        each([&](int q, int, int) { m = m + rt[q] * v[q]; });
+        cell_reduce<false>(m, unused, sh, flip);
+        m = vol * m;
+        alpha[0] = rho[1] / m;
+        if (fabs(m) > small * fabs(rho[1])) {
+            each([&](int q, int, int) {
+                r[q] = r[q] + -alpha[0] * v[q];
+                e[q] = e[q] + alpha[0] * z[q];
+            });
+            norm[0] = norm_rho();
+        } else {
+            each([&](int q, int, int) { r[q] = 0.0; });
+            norm[0] = 0.0;
+            rho_next = 0.0;
+        }
+        if ((norm[0] > tol * initial_norm) && (norm[0] > reps * initial_rnorm)) {
+            double t[kCells];
+            precondition(st, rr, r, t, z);
+            double tr = 0.0, tt = 0.0;
+            each([&](int q, int, int) {
+                tr = tr + t[q] * r[q];
+                tt = tt + t[q] * t[q];
+            });
+            cell_reduce<false>(tr, tt, sh, flip);
+            omg[0] = (vol * tr) / (vol * tt);
+            each([&](int q, int, int) {
+                e[q] = e[q] + omg[0] * z[q];
+                r[q] = r[q] + -omg[0] * t[q];
+            });
+            norm[0] = norm_rho();
+        }
+        if ((norm[0] <= tol * initial_norm) || (norm[0] <= reps * initial_rnorm)) break;
+        if ((omg[0] == 0.0) || (norm[0] > (1.0 - hang) * norm[1])) {
+            if (recount == 0) {
+                recount = 1;
+            } else {
+                recount = 0;
+                add();
+                if (restarts == max_restarts) break;   // then e is added again below (P2:2466)
+                norm[0] = residual();
+                rho[1] = rho[2] = rho[3] = 0.0;
+                alpha[0] = beta[0] = omg[0] = 0.0;
+                restarts = restarts + 1;
+                init = 1;
+            }
+        }
+    }
+    add();
+    return isfinite(norm[0]) ? DST_OK : DST_NONFINITE;
+}
+constexpr int kCellsMost = 3;   // cells a thread of cell_bicgstab
+
+__device__ __forceinline__ int held_bicgstab(const Lv& L, int dd, double* sh, HeldWork& H) {
+    const int c = (L.nx * L.ny + kCoarseThreads - 1) / kCoarseThreads;
+    if (dd) return c == 1 ? cell_bicgstab<true, 1>(L, sh, H) : c == 2 ? cell_bicgstab<true, 2>(L, sh, H)
+                                                                      : cell_bicgstab<true, 3>(L, sh, H);
+    return c == 1 ? cell_bicgstab<false, 1>(L, sh, H) : c == 2 ? cell_bicgstab<false, 2>(L, sh, H)
+                                                               : cell_bicgstab<false, 3>(L, sh, H);
 }
 
 // ---------------------------------------------------------------------------
@@ -2060,6 +2279,7 @@ visit:
             int s;
             if constexpr (S::kGrid) s = b_bicgstab<S>(L, L.e, L.r, 1, 1.0e-6, 80, 5, 0, a.dd, sh);
             else s = is_tiny(d) ? tiny_bicgstab(tiny[d], L, a.dd, *W)
+                   : W && L.nx * L.ny <= kCellsMost * kCoarseThreads ? held_bicgstab(L, a.dd, sh, *H)
                                 : b_bicgstab<S>(L, L.e, L.r, 1, 1.0e-6, 80, 5, 0, a.dd, sh, H);
             if (s) st = s;
             goto up;
