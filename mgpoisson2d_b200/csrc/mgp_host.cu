@@ -936,24 +936,22 @@ int solver_build(mgp_solver* s, const mgp_box* valid, const mgp_geo* geo, const 
             Lv& L = sh[d];
             place(L.e, L.nx, L.ny, 1);
             place(L.r, L.nx, L.ny, 0);
-            place(L.w, L.nx, L.ny, 0);
+            if (d < md || s->kind == MGP_KIND_DD) place(L.w, L.nx, L.ny, 0);
             place(L.invd, L.nx, L.ny, 0);
-            place(L.g.J, L.nx, L.ny, 0);
+            if (d < md) place(L.g.J, L.nx, L.ny, 0);
             place(L.g.xx, L.nx + 1, L.ny, 0);
             place(L.g.xy, L.nx + 1, L.ny, 0);
             place(L.g.yx, L.nx, L.ny + 1, 0);
             place(L.g.yy, L.nx, L.ny + 1, 0);
-            if (d == md) {
-                place(L.ea, L.nx, L.ny, 1);
+            if (d == md) {   // of the BiCGStab fields the two cell_bicgstab keeps outside registers
                 place(L.pt, L.nx, L.ny, 1);
-                place(L.st, L.nx, L.ny, 1);
-                place(L.rr, L.nx, L.ny, 0);
-                place(L.rt, L.nx, L.ny, 0);
                 place(L.pp, L.nx, L.ny, 0);
-                place(L.tt, L.nx, L.ny, 0);
-                place(L.vv, L.nx, L.ny, 0);
             }
         }
+        // Bottoms one CTA holds, though a cluster could share them: 37 x 50 cells
+        // take 68 us a BiCGStab iteration in shared memory (87 in global memory),
+        // and a cluster's seventy-odd barriers an iteration alone cost 2 us each.
+        if ((long)s->lv[md].nx * s->lv[md].ny > kHeldBottomCells) off = (size_t)kCoarseSmemMax;   // not staged
         if (md - s->dc + 1 <= kMaxCoarseLevels && off * sizeof(double) <= (size_t)kCoarseSmemMax)
             RC(build_tiny(s, &off, st));
         const size_t bytes = off * sizeof(double);
@@ -2029,11 +2027,43 @@ bool fill_one_phase(const BCd& b, int do_neum) {   // no side's fill reads anoth
     return true;
 }
 
-// A level's sweep jobs: one sweep per launch, two per launch, and levels of a
+// A level's sweep jobs: one, two or four sweeps per launch, and levels of a
 // single tile, whose launch makes the whole smoothing call in place.
 template <class T>
 struct SweepGroups {
-    Table<SweepJobT<T>> one, two, all;
+    Table<SweepJobT<T>> one, two, four, all;
+    std::vector<SweepJobT<T>> open;   // until all are known (settle)
+
+    // As sweep_plan for one level, over the tiles of all: the most sweeps a launch
+    // whose tiles do not outnumber the SMs, else one sweep by the large shape's
+    // persistent CTAs: 11 us a sweep however small the level, against 3 to 4 with
+    // four sweeps a launch (32 problems of up to 1024 cells a side: 226 -> 212 ms).
+    // The counts must leave every correction in its first buffer: an even number
+    // of launches.
+    void settle(int nd, int nu) {
+        for (int k : {4, 2}) {
+            if (nd % (2 * k) || nu % (2 * k)) continue;
+            long tiles = 0;
+            for (const auto& J : open) {
+                const SweepPlan p = sweep_tiles<T>(J.nx, J.ny, k);
+                tiles += p.k ? (long)p.gx * p.gy : 1L << 40;
+            }
+            if (tiles > sweep_wave()) continue;
+            for (auto& J : open) {
+                const SweepPlan p = sweep_tiles<T>(J.nx, J.ny, k);
+                J.gx = p.gx;
+                J.gy = p.gy;
+                (k == 4 ? four : two).push(J, J.gx * J.gy);
+            }
+            open.clear();
+            return;
+        }
+        for (auto& J : open) {
+            J.tiles = sweep_large_tiles<T>(J.nx, J.ny);
+            one.push(J, J.tiles.total);
+        }
+        open.clear();
+    }
 };
 
 template <class T>
@@ -2053,7 +2083,7 @@ void add_sweep_job(SweepGroups<T>& sg, const LevelMaps& m, const DFT<T>& e, cons
     J.nx = nx;
     J.ny = ny;
     // one tile: the whole call in a launch; `pairs`: two sweeps a launch on small
-    // levels; else one sweep with the large shape's tiles
+    // levels, however many; else as settle finds
     const SweepPlan p = sweep_plan<T>(nx, ny, b, 2, &m);
     J.in_place = p.gx * p.gy == 1;
     if (J.in_place || (pairs && p.k == 2)) {
@@ -2061,8 +2091,7 @@ void add_sweep_job(SweepGroups<T>& sg, const LevelMaps& m, const DFT<T>& e, cons
         J.gy = p.gy;
         (J.in_place ? sg.all : sg.two).push(J, J.gx * J.gy);
     } else {
-        J.tiles = sweep_large_tiles<T>(nx, ny);
-        sg.one.push(J, J.tiles.total);
+        sg.open.push_back(J);
     }
 }
 
@@ -2200,12 +2229,14 @@ void build_plan(Plan& P, const std::vector<mgp_solver*>& ss, const std::vector<i
         P.norm.push(NormJob{s->phi0, s->rhs0, L0.r, L0.g, ubc[p], nx, ny, homog, bx0}, bx0 * by0);
         P.vol.push_back(s->valid.dx * s->valid.dy);
     }
+    for (auto& g : P.sw64) g.settle(nd, nu);
+    for (auto& g : P.sw32) g.settle(nd, nu);
 }
 
 template <class F>
 void for_tables(Plan& P, F f) {
-    for (auto& g : P.sw64) { f(g.one); f(g.two); f(g.all); }
-    for (auto& g : P.sw32) { f(g.one); f(g.two); f(g.all); }
+    for (auto& g : P.sw64) { f(g.one); f(g.two); f(g.four); f(g.all); }
+    for (auto& g : P.sw32) { f(g.one); f(g.two); f(g.four); f(g.all); }
     for (auto& t : P.fpre64) f(t);
     for (auto& t : P.fpre32) f(t);
     for (auto& t : P.fpost64) f(t);
@@ -2255,8 +2286,8 @@ int upload_plan(Plan& P, Lockstep* ls, cudaStream_t st) {
     return MGP_OK;
 }
 
-// n sweeps of every job of a level (n even; with two-sweep jobs a multiple of
-// 4, so every job's correction ends in its first buffer).
+// n sweeps of every job of a level (n even; with two- or four-sweep jobs a
+// multiple of 4 or 8, so every job's correction ends in its first buffer).
 template <class T>
 int sweeps(SweepGroups<T>& g, int n, Lockstep* ls, cudaStream_t st) {
     for (int k = 0; k < n; ++k)
@@ -2264,6 +2295,9 @@ int sweeps(SweepGroups<T>& g, int n, Lockstep* ls, cudaStream_t st) {
                                  st));
     for (int k = 0; k < n / 2; ++k)
         CK(launch_sweep9_jobs<T>(g.two.dj, g.two.dp, g.two.n(), g.two.blocks(), 2, 1, k & 1, ls->status,
+                                 st));
+    for (int k = 0; k < n / 4; ++k)
+        CK(launch_sweep9_jobs<T>(g.four.dj, g.four.dp, g.four.n(), g.four.blocks(), 4, 1, k & 1, ls->status,
                                  st));
     if (n > 0) CK(launch_sweep9_jobs<T>(g.all.dj, g.all.dp, g.all.n(), g.all.blocks(), n, 1, 0, ls->status, st));
     return MGP_OK;

@@ -1816,7 +1816,7 @@ __device__ __noinline__ int cell_bicgstab(const Lv& L_, double* sh, HeldWork& H)
     const double tol = 1.0e-6, reps = 1.0e-12, hang = 1.0e-7, small = 1.0e-30;
     const int max_iters = 80, max_restarts = 5;
     const Lv& L = L_;
-    const DF phi = L.e, pt = L.pt, st = L.st, pp = L.pp, rr = L.rr;
+    const DF phi = L.e, z = L.pt, f = L.pp;
     const int nx = L.nx, ny = L.ny, n = nx * ny;
     const double vol = L.g.dx * L.g.dy;
     int ci[kCells], cj[kCells];
@@ -1833,8 +1833,7 @@ __device__ __noinline__ int cell_bicgstab(const Lv& L_, double* sh, HeldWork& H)
     }
     for (int k = threadIdx.x; k < (nx + 2) * (ny + 2); k += kCoarseThreads) {
         const int j = k / (nx + 2) - 1, i = k - (j + 1) * (nx + 2) - 1;
-        AT(pt, i, j) = 0.0;
-        AT(st, i, j) = 0.0;
+        AT(z, i, j) = 0.0;
     }
     int flip = 0;
     const auto each = [&](auto f) {
@@ -1872,8 +1871,8 @@ __device__ __noinline__ int cell_bicgstab(const Lv& L_, double* sh, HeldWork& H)
         __syncthreads();
         if (kDd) b_fill<BlockScope>(phi, L.g, L.bc, 1, 1, nx, ny);
     };
-    // z = two sweeps for the right-hand side x (in f), w = L[z]
-    const auto precondition = [&](const DF& z, const DF& f, const double* x, double* w, double* zv) {
+    // z = two sweeps for the right-hand side x, w = L[z].  A Neumann ghost of z stays zero.
+    const auto precondition = [&](const double* x, double* w, double* zv) {
         each([&](int q, int i, int j) {
             AT(z, i, j) = x[q] * d[q];
             AT(f, i, j) = x[q];
@@ -1910,8 +1909,8 @@ __device__ __noinline__ int cell_bicgstab(const Lv& L_, double* sh, HeldWork& H)
         if (!init) beta[1] = (rho[1] / rho[2]) * (alpha[1] / omg[1]);
         each([&](int q, int, int) { p[q] = init ? r[q] : beta[1] * (p[q] - omg[1] * v[q]) + r[q]; });
         init = 0;
-        double z[kCells];
-        precondition(pt, pp, p, v, z);
+        double zv[kCells];
+        precondition(p, v, zv);
         double m = 0.0, unused = 0.0;
         each([&](int q, int, int) { m = m + rt[q] * v[q]; });
         cell_reduce<false>(m, unused, sh, flip);
@@ -1920,7 +1919,7 @@ __device__ __noinline__ int cell_bicgstab(const Lv& L_, double* sh, HeldWork& H)
         if (fabs(m) > small * fabs(rho[1])) {
             each([&](int q, int, int) {
                 r[q] = r[q] + -alpha[0] * v[q];
-                e[q] = e[q] + alpha[0] * z[q];
+                e[q] = e[q] + alpha[0] * zv[q];
             });
             norm[0] = norm_rho();
         } else {
@@ -1930,7 +1929,7 @@ __device__ __noinline__ int cell_bicgstab(const Lv& L_, double* sh, HeldWork& H)
         }
         if ((norm[0] > tol * initial_norm) && (norm[0] > reps * initial_rnorm)) {
             double t[kCells];
-            precondition(st, rr, r, t, z);
+            precondition(r, t, zv);
             double tr = 0.0, tt = 0.0;
             each([&](int q, int, int) {
                 tr = tr + t[q] * r[q];
@@ -1939,7 +1938,7 @@ __device__ __noinline__ int cell_bicgstab(const Lv& L_, double* sh, HeldWork& H)
             cell_reduce<false>(tr, tt, sh, flip);
             omg[0] = (vol * tr) / (vol * tt);
             each([&](int q, int, int) {
-                e[q] = e[q] + omg[0] * z[q];
+                e[q] = e[q] + omg[0] * zv[q];
                 r[q] = r[q] + -omg[0] * t[q];
             });
             norm[0] = norm_rho();
@@ -1963,14 +1962,12 @@ __device__ __noinline__ int cell_bicgstab(const Lv& L_, double* sh, HeldWork& H)
     add();
     return isfinite(norm[0]) ? DST_OK : DST_NONFINITE;
 }
-constexpr int kCellsMost = 3;   // cells a thread of cell_bicgstab
 
-__device__ __forceinline__ int held_bicgstab(const Lv& L, int dd, double* sh, HeldWork& H) {
+template <bool kDd>
+__device__ __forceinline__ int held_bicgstab(const Lv& L, double* sh, HeldWork& H) {
     const int c = (L.nx * L.ny + kCoarseThreads - 1) / kCoarseThreads;
-    if (dd) return c == 1 ? cell_bicgstab<true, 1>(L, sh, H) : c == 2 ? cell_bicgstab<true, 2>(L, sh, H)
-                                                                      : cell_bicgstab<true, 3>(L, sh, H);
-    return c == 1 ? cell_bicgstab<false, 1>(L, sh, H) : c == 2 ? cell_bicgstab<false, 2>(L, sh, H)
-                                                               : cell_bicgstab<false, 3>(L, sh, H);
+    return c == 1 ? cell_bicgstab<kDd, 1>(L, sh, H) : c == 2 ? cell_bicgstab<kDd, 2>(L, sh, H)
+         : c == 3 ? cell_bicgstab<kDd, 3>(L, sh, H) : cell_bicgstab<kDd, kHeldBottomCells / kCoarseThreads>(L, sh, H);
 }
 
 // ---------------------------------------------------------------------------
@@ -2279,8 +2276,8 @@ visit:
             int s;
             if constexpr (S::kGrid) s = b_bicgstab<S>(L, L.e, L.r, 1, 1.0e-6, 80, 5, 0, a.dd, sh);
             else s = is_tiny(d) ? tiny_bicgstab(tiny[d], L, a.dd, *W)
-                   : W && L.nx * L.ny <= kCellsMost * kCoarseThreads ? held_bicgstab(L, a.dd, sh, *H)
-                                : b_bicgstab<S>(L, L.e, L.r, 1, 1.0e-6, 80, 5, 0, a.dd, sh, H);
+                   : W ? (a.dd ? held_bicgstab<true>(L, sh, *H) : held_bicgstab<false>(L, sh, *H))
+                       : b_bicgstab<S>(L, L.e, L.r, 1, 1.0e-6, 80, 5, 0, a.dd, sh, H);
             if (s) st = s;
             goto up;
         }
@@ -2350,9 +2347,8 @@ __device__ __forceinline__ void coarse_cycle_smem(const CoarseArgs& a, double* s
         Lv L = a.shadow[a.d0 + threadIdx.x];
         rebase(L.e, smem); rebase(L.r, smem); rebase(L.w, smem); rebase(L.invd, smem);
         rebase(L.g.J, smem); rebase(L.g.xx, smem); rebase(L.g.xy, smem); rebase(L.g.yx, smem); rebase(L.g.yy, smem);
-        if (a.d0 + (int)threadIdx.x == a.maxdepth && !a.ainv) {
-            rebase(L.ea, smem); rebase(L.pt, smem); rebase(L.st, smem);
-            rebase(L.rr, smem); rebase(L.rt, smem); rebase(L.pp, smem); rebase(L.tt, smem); rebase(L.vv, smem);
+        if (a.d0 + (int)threadIdx.x == a.maxdepth && !a.ainv) {   // cell_bicgstab's two fields
+            rebase(L.pt, smem); rebase(L.pp, smem);
         }
         sl[threadIdx.x] = L;
     }
@@ -2362,7 +2358,7 @@ __device__ __forceinline__ void coarse_cycle_smem(const CoarseArgs& a, double* s
         const int nx = S.nx, ny = S.ny;
         b_copy_in(S.e, G.e, -1, nx + 1, -1, ny + 1);
         b_copy_in(S.invd, G.invd, 0, nx, 0, ny);
-        b_copy_in(S.g.J, G.g.J, 0, nx, 0, ny);
+        if (k + 1 < nl) b_copy_in(S.g.J, G.g.J, 0, nx, 0, ny);
         b_copy_in(S.g.xx, G.g.xx, 0, nx + 1, 0, ny);
         b_copy_in(S.g.xy, G.g.xy, 0, nx + 1, 0, ny);
         b_copy_in(S.g.yx, G.g.yx, 0, nx, 0, ny + 1);

@@ -113,6 +113,7 @@ struct BicgArgs {
 };
 
 constexpr int kCoarseThreads = 512;   // of the one-CTA coarse cycle: the shape of mgp_sweep.cuh's windows
+constexpr int kHeldBottomCells = 5 * kCoarseThreads;   // largest bottom it holds in shared memory
 constexpr int kReduceThreads = 256;   // of them that accumulate its reductions
 constexpr int kGridThreads = 256;     // threads per CTA of the cooperative-grid coarse cycle
 constexpr int kClusterThreads = 256;   // threads per CTA of the cluster coarse cycle
@@ -255,6 +256,10 @@ struct SweepPlan {
     int k, gx, gy;
     bool small;
 };
+// The small shape's tiles for k sweeps a launch (k = 0: none), and the CTAs of it that run at once.
+template <class T>
+SweepPlan sweep_tiles(int nx, int ny, int k);
+int sweep_wave();
 template <class T>
 SweepTiles sweep_large_tiles(int nx, int ny);
 // A level's descriptors with phi in either of its two buffers.  Built when the

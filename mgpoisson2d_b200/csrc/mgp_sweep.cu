@@ -632,6 +632,17 @@ SweepPlan sweep_plan(int nx, int ny, const BCd& b, int left, const LevelMaps* ma
     if (maps && maps->ok) return SweepPlan{1, 0, 0, false};
     return tiles_of<S>(nx, ny, periodic || left < 2 || S::ty(2) < 12 ? 1 : 2);
 }
+
+template <class T>
+SweepPlan sweep_tiles(int nx, int ny, int k) {
+    using S = typename Shapes<T>::Small;
+    if (S::tx(k) < 12 || S::ty(k) < 12) return SweepPlan{0, 0, 0, true};
+    return tiles_of<S>(nx, ny, k);
+}
+template SweepPlan sweep_tiles<float>(int, int, int);
+template SweepPlan sweep_tiles<double>(int, int, int);
+int sweep_wave() { return sm_count(); }
+
 template SweepPlan sweep_plan<float>(int, int, const BCd&, int, const LevelMaps*);
 template SweepPlan sweep_plan<double>(int, int, const BCd&, int, const LevelMaps*);
 
