@@ -31,13 +31,13 @@
 // Two shapes, chosen by sweep_plan.  Levels whose sweeps last one CTA's latency
 // take several sweeps a launch, with four warps of their own for the sides:
 // measured per sweep of an n^2 level, FP32 / FP64, before (operator in shared
-// memory, two sweeps a launch) and now: 128^2 8.4 / 8.3 -> 2.7 / 3.7 us, 256^2
-// 8.5 / 8.3 -> 2.9 / 5.3 us, 512^2 8.7 / 11 -> 5.7 / 10 us.  Large levels take
+// memory, two sweeps a launch) and now: 128^2 8.4 / 8.3 -> 2.2 / 3.4 us, 256^2
+// 8.5 / 8.3 -> 2.3 / 5.2 us, 512^2 8.7 / 11 -> 5.7 / 9.9 us.  Large levels take
 // one sweep a launch by persistent CTAs that load the next tile while they
-// sweep one: 1024^2 17.2 / 32 -> 13.5 / 22 us, 2048^2 41 / 88 -> 38 / 72 us
-// (0.55 / 0.58 of the copy rate by the 8 words a cell of a sweep).  They are
+// sweep one: 1024^2 17.2 / 32 -> 13 / 22 us, 2048^2 41 / 88 -> 37 / 72 us
+// (0.57 / 0.58 of the copy rate by the 8 words a cell of a sweep).  They are
 // bound by the barriers between colour passes (5 of 18 cycles between a warp's
-// issues), not by the bytes.
+// issues), not by the bytes; the small ones by the sides (mgp_sweep.cuh).
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
@@ -250,8 +250,10 @@ __device__ __forceinline__ void sweep_stream(int total, int homog, double omega,
             load_fields(tiles[it ^ 1]);
         }
         if (any_side) {
-            with_side<C>(warp, [&](auto L) {
+            with_side<C>(warp, w, L0.nx, L0.ny, [&](auto L) {
                 L.place(w, *L0.g, *L0.b, homog, L0.nx, L0.ny, om, om1);
+                L.grab(s);
+                L.put(s);
                 L.fill(s, *L0.pin, w, *L0.b, homog, L0.nx, L0.ny, 0);
             });
             cta_sync();
@@ -259,7 +261,7 @@ __device__ __forceinline__ void sweep_stream(int total, int homog, double omega,
         }
         colours<C>(k, own, mask, idx, idy, om, om1);
         if (any_side) {
-            with_side<C>(warp, [&](auto L) {
+            with_side<C>(warp, w, L0.nx, L0.ny, [&](auto L) {
                 L.place(w, *L0.g, *L0.b, homog, L0.nx, L0.ny, om, om1);
                 L.take(strips, w, *L0.b, homog);
                 L.pass(s, strips, w, *L0.g, *L0.b, homog, L0.nx, L0.ny);

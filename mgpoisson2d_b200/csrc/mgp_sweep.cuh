@@ -161,15 +161,20 @@ __device__ __forceinline__ T update(const Block<T>& k, const T* s, T idx, T idy,
 // (x on the y sides, y on the x sides) and its normal n; the cell formulas are
 // gather9's and lap9f's with t for x and n for y, which on the x sides are the
 // same operations by the symmetry of the operator under exchanging x and y.
-// A lane keeps two neighbouring cells of the side, one of each colour: their
-// operator and the sixteen plane addresses they read.  These passes are a
-// serial chain of single warps (about 4 cycles an instruction), so every
-// instruction that does not depend on phi is made once, before the sweeps.
+// A lane keeps two neighbouring cells of the side, one of each colour, and their
+// operator.  These passes are a serial chain of single warps (about 4 cycles an
+// instruction), four times the interior's 745 cycles a sweep in FP64, so every
+// instruction that does not depend on phi is made once, before the sweeps, and
+// the rest are few: places known at compile time, ghosts read before the interior
+// colours and written beside them, the FP32 operator folded into nine weights.  A
+// sweep of 32^2 cells: 2.6 -> 2.05 us in FP64, 2.0 -> 1.3 in FP32.
 //
 // The operator at a side's cells comes from their owners through shared
 // memory: value q of cell a along side t at [(t * kStrip + q) * kAlong + a].
 constexpr int kStrip = 10, kAlong = 64;
 enum { Q_TT1, Q_TT0, Q_TN1, Q_TN0, Q_NN1, Q_NN0, Q_NT1, Q_NT0, Q_D, Q_F };   // 1: the high face, 0: the low face
+// Weights by cell: plus and minus along the side; the cell itself, one and two inward; the ghost.
+enum { W_PP, W_PM, W_P1, W_M1, W_P2, W_M2, W_I1, W_I2, W_GH, W_D, W_F };
 
 template <int CX, int CY, class T>
 __device__ __forceinline__ void strip_write(T* q, const Block<T>& k, bool yside) {
@@ -227,16 +232,45 @@ __device__ __forceinline__ void corner_cell(T* S, const T* q, const int* x, cons
     S[x[1] + y[1]] = om * newphi + om1 * p;
 }
 
-// What a lane keeps of its side (kY: a y side; kHigh: at the high end).
-template <class C, bool kY, bool kHigh>
+// What a lane keeps of its side (kY: a y side; kHigh: at the high end, in an odd
+// row or column of the window if kOdd).  With the side's parity known, the plane
+// places of the sixteen cells a lane reads are constants from one address and the
+// two colours whose turns its cells have are too: as registers they were made
+// again, some hundred instructions a colour, each time.
+template <class C, bool kY, bool kHigh, bool kOdd>
 struct SideLane {
     using T = typename C::T;
     static constexpr int sd = (kY ? S_YLO : S_XLO) + (kHigh ? 1 : 0);
+    // the colours (0,0),(1,1),(1,0),(0,1): the one with this normal parity and tangential parity c
+    __host__ __device__ static constexpr int ph(int c) {
+        return kY ? (kOdd ? (c ? 1 : 3) : (c ? 2 : 0)) : (kOdd ? (c ? 1 : 2) : (c ? 3 : 0));
+    }
+    // Term of row r across the side, at its block (the ghost, the side, one and two inward).
+    __host__ __device__ static constexpr int across(int r) {
+        constexpr int NQ = kY ? 2 * C::PS : C::PS, NB = kY ? C::P : 1;
+        const int low = r == 0 ? NQ - NB : r == 1 ? 0 : r == 2 ? NQ : NB;
+        const int odd = r == 0 ? NB : r == 1 ? NQ : r == 2 ? 0 : NQ - NB;
+        const int even = r == 0 ? NQ : r == 1 ? 0 : r == 2 ? NQ - NB : -NB;
+        return !kHigh ? low : kOdd ? odd : even;
+    }
+    // Place of column t - 1 of the lane's (its cells are 0 and 1) in row r (the ghost, the side, one and two inward).
+    __host__ __device__ static constexpr int at(int t, int r) {
+        constexpr int TQ = kY ? C::PS : 2 * C::PS, TB = kY ? 1 : C::P;   // planes and blocks along the side
+        return across(r) + (t == 0 ? TQ - TB : t == 1 ? 0 : t == 2 ? TQ : TB);
+    }
+    // The warp's corner of the domain: (low, low), (high, high), (low, high), (high,
+    // low) for y low, y high, x low, x high, so that at most one direction's places
+    // depend on the other side's parity (cz).
+    static constexpr bool hx = kHigh, hy = kY ? kHigh : !kHigh;
     bool on, plain, neum;      // the window holds the side; its ghosts follow from three rows; a Neumann side
+    bool all_plain, corner;    // so do every side's; the window holds the corner and it is to update
+    int cz[4];
     bool ok[2], in[2];         // the lane's cells: edge cells to update, cells of the window
-    int ad[4][4];              // plane index of (column - 1, the two cells, column + 2; ghost, side, one, two inward)
-    int ph[2];                 // the colour in whose turn each cell is
-    T q[2][kStrip], nb[2];     // operators; the Neumann side's boundary fluxes
+    int base;
+    // FP64: the operators (Q_*) and the Neumann side's fluxes.  FP32: the weights W_*
+    // of the differences to the cell's own value, the operator folded once a call.
+    T q[2][11], nb[2];
+    T g0[2], g1[2], g2[2];     // what the next sweep's ghosts are made of
     T idt, idn, om, om1;
 
     __device__ __forceinline__ void place(const Window& w, const GeoT<T>& g, const BCd& b, int homog, int nx, int ny,
@@ -249,24 +283,23 @@ struct SideLane {
                 (b.type[sd] == T_NEUM || (b.type[sd] == T_DIRI && homog && b.mode[sd] != M_LAH));
         neum = b.type[sd] == T_NEUM;
         const int ot = kY ? w.ox : w.oy, et = kY ? w.wx1 : w.wy1, nt = kY ? nx : ny;
-        const int at = kHigh ? (kY ? ny : nx) - 1 : 0, in_ = kHigh ? -1 : 1;
-        const int n = at - (kY ? w.oy : w.ox), a = 2 * lane;
+        const int m = kHigh ? ((kY ? ny - w.oy : nx - w.ox) - 1) >> 1 : 0;   // the side's block, 0 at the low end
         const int lo = (kY ? pr.xl : pr.yl) ? 0 : 1, hi = (kY ? pr.xh : pr.yh) ? nt : nt - 1;   // corners left out
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
-            const int t = ot + a + c;
+            const int t = ot + 2 * lane + c;
             in[c] = on && t < et;
             ok[c] = in[c] && !periodic && t >= lo && t < hi;
-            // colours (0,0),(1,1),(1,0),(0,1): the one with this normal parity and tangential parity c
-            ph[c] = kY ? ((at & 1) ? (c ? 1 : 3) : (c ? 2 : 0)) : ((at & 1) ? (c ? 1 : 2) : (c ? 3 : 0));
         }
+        base = C::P + 1 + (kY ? lane + m * C::P : lane * C::P + m);
+        all_plain = !(pr.xl || pr.xh || pr.yl || pr.yh);
 #pragma unroll
-        for (int t = 0; t < 4; ++t)
+        for (int s = 0; s < 4; ++s)
+            all_plain = all_plain && (b.type[s] == T_NEUM || (b.type[s] == T_DIRI && homog && b.mode[s] != M_LAH));
+        corner = lane == 0 && (hx ? w.xh && !pr.xh : w.xl && !pr.xl) && (hy ? w.yh && !pr.yh : w.yl && !pr.yl);
 #pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                const int tt = a - 1 + t, nn = n + (r - 1) * in_;
-                ad[t][r] = kY ? x_term<C>(tt) + y_term<C>(nn) : x_term<C>(nn) + y_term<C>(tt);
-            }
+        for (int r = 0; r < 4; ++r)   // the direction along the side: the other sides' terms
+            cz[r] = kY ? x_term<C>(hx ? nx - 1 - w.ox - (r - 1) : r - 1) : y_term<C>(hy ? ny - 1 - w.oy - (r - 1) : r - 1);
         idt = T(kY ? g.idx : g.idy);
         idn = T(kY ? g.idy : g.idx);
         om = om_;
@@ -275,48 +308,97 @@ struct SideLane {
     // The operators, once their owners have written the strips.
     __device__ __forceinline__ void take(const T* strips, const Window& w, const BCd& b, int homog) {
         const int lane = threadIdx.x & 31, side = (kY ? 0 : 2) + (kHigh ? 1 : 0);
-#pragma unroll
-        for (int c = 0; c < 2; ++c)
-#pragma unroll
-            for (int v = 0; v < kStrip; ++v) {
-                q[c][v] = T(0.0);
-                if (ok[c]) q[c][v] = strips[(side * kStrip + v) * kAlong + 2 * lane + c];
-                if (v == Q_TN1 || v == Q_TN0 || v == Q_NT1 || v == Q_NT0) q[c][v] = q[c][v] * T(0.25);
-            }
+        const T quarter = T(0.25);
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
             const int t = (kY ? w.ox : w.oy) + 2 * lane + c;
             nb[c] = T(0.0);
             if (neum && ok[c]) nb[c] = T(nbval(b, homog, sd, sd == S_YHI ? b.kyhi : t));
+            T v[kStrip];
+#pragma unroll
+            for (int r = 0; r < kStrip; ++r) {
+                v[r] = T(0.0);
+                if (ok[c]) v[r] = strips[(side * kStrip + r) * kAlong + 2 * lane + c];
+                if (r == Q_TN1 || r == Q_TN0 || r == Q_NT1 || r == Q_NT0) v[r] = v[r] * quarter;
+            }
+            if constexpr (sizeof(T) == 8) {
+#pragma unroll
+                for (int r = 0; r < kStrip; ++r) q[c][r] = v[r];
+            } else {
+                // lphi = sum of W (phi - p): the extrapolations are sums of such differences, and the sign s turns the
+                // high side's normal inward (in: the face towards the interior, out: the domain's side)
+                const T s = kHigh ? T(-1.0) : T(1.0), tt = idt * idt, tn = s * idt * idn, nn = idn * idn;
+                const T a1 = v[Q_TT1] * tt, a0 = v[Q_TT0] * tt, b1 = v[Q_TN1] * tn, b0 = v[Q_TN0] * tn;
+                const T ci = v[kHigh ? Q_NN0 : Q_NN1] * nn, ei = v[kHigh ? Q_NT0 : Q_NT1] * tn;
+                const T co = neum ? T(0.0) : v[kHigh ? Q_NN1 : Q_NN0] * nn;
+                const T eo = neum ? T(0.0) : v[kHigh ? Q_NT1 : Q_NT0] * tn;
+                q[c][W_PP] = a1 - T(3.0) * b1 + ei - T(4.0) * eo;
+                q[c][W_PM] = a0 + T(3.0) * b0 - ei + T(4.0) * eo;
+                q[c][W_P1] = T(4.0) * b1 + ei + T(3.0) * eo;
+                q[c][W_M1] = -(T(4.0) * b0 + ei + T(3.0) * eo);
+                q[c][W_P2] = -(b1 + eo);
+                q[c][W_M2] = b0 + eo;
+                q[c][W_I1] = T(4.0) * (b1 - b0) + ci;
+                q[c][W_I2] = b0 - b1;
+                q[c][W_GH] = co;
+                q[c][W_D] = v[Q_D] * om;
+                q[c][W_F] = v[Q_F] + s * nb[c] * idn;
+            }
         }
     }
-    // A sweep's ghosts (fill_ghosts without do_neum, P2:1556).
+    // A sweep's ghosts (fill_ghosts without do_neum, P2:1556), of the values at its
+    // start.  Where they follow from three rows, grab reads these before the interior
+    // colours change them (and may do so before the corners, whose values put reads
+    // again) and put writes the ghosts beside the colours, since only the sides' cells
+    // read them.  Otherwise fill, between barriers.
+    __device__ __forceinline__ void grab(const T* S) {
+        if (!plain || neum) return;   // a Neumann side's stay as stored
+#pragma unroll
+        for (int c = 0; c < 2; ++c)
+            if (in[c]) {
+                g0[c] = S[base + at(1 + c, 1)];
+                g1[c] = S[base + at(1 + c, 2)];
+                g2[c] = S[base + at(1 + c, 3)];
+            }
+    }
+    __device__ __forceinline__ void put(T* S) {
+        if (!plain || neum) return;
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {   // AU:1161-1177, homogeneous
+            if (in[c] && !ok[c]) g0[c] = S[base + at(1 + c, 1)];
+            if (in[c]) S[base + at(1 + c, 0)] = -(T(3.0) * g0[c]) + g1[c] - T(1.0 / 5.0) * g2[c];
+        }
+    }
     __device__ __forceinline__ void fill(T* S, const DFT<T>& pin, const Window& w, const BCd& b, int homog, int nx,
                                          int ny, int sw) const {
-        if (!on) return;
-        if (plain) {
-            if (neum) return;   // as stored
-#pragma unroll
-            for (int c = 0; c < 2; ++c)   // AU:1161-1177, homogeneous
-                if (in[c])
-                    S[ad[1 + c][0]] = -(T(3.0) * S[ad[1 + c][1]]) + S[ad[1 + c][2]] - T(1.0 / 5.0) * S[ad[1 + c][3]];
-        } else if (!(sw > 0 && neum)) {
-            const StartLoad<C> P{S, w, pin};
-            const int lo = kY ? (w.xl ? -1 : w.ox) : w.oy, hi = kY ? (w.xh ? nx + 1 : w.wx1) : w.wy1;
-            const int at = kHigh ? (kY ? ny : nx) : -1;
-            for (int v = lo + (threadIdx.x & 31); v < hi; v += 32) {
-                const int i = kY ? v : at, j = kY ? at : v;
-                S[x_term<C>(i - w.ox) + y_term<C>(j - w.oy)] = sweep_ghost(P, b, homog, nx, ny, i, j);
-            }
+        if (!on || plain || (sw > 0 && neum)) return;
+        const StartLoad<C> P{S, w, pin};
+        const int lo = kY ? (w.xl ? -1 : w.ox) : w.oy, hi = kY ? (w.xh ? nx + 1 : w.wx1) : w.wy1;
+        const int side = kHigh ? (kY ? ny : nx) : -1;
+        for (int v = lo + (threadIdx.x & 31); v < hi; v += 32) {
+            const int i = kY ? v : side, j = kY ? side : v;
+            S[x_term<C>(i - w.ox) + y_term<C>(j - w.oy)] = sweep_ghost(P, b, homog, nx, ny, i, j);
         }
     }
     // gs9's update of the lane's cell c.
     template <int c>
     __device__ __forceinline__ void cell(T* S) const {
         const T three = T(3.0);
-        const T p = S[ad[1 + c][1]], i1 = S[ad[1 + c][2]], i2 = S[ad[1 + c][3]], gh = S[ad[1 + c][0]];
-        const T pm = S[ad[c][1]], m1 = S[ad[c][2]], m2 = S[ad[c][3]];
-        const T pp = S[ad[2 + c][1]], p1 = S[ad[2 + c][2]], p2 = S[ad[2 + c][3]];
+        T* B = S + base;
+        const T p = B[at(1 + c, 1)], i1 = B[at(1 + c, 2)], i2 = B[at(1 + c, 3)], gh = B[at(1 + c, 0)];
+        const T pm = B[at(c, 1)], m1 = B[at(c, 2)], m2 = B[at(c, 3)];
+        const T pp = B[at(2 + c, 1)], p1 = B[at(2 + c, 2)], p2 = B[at(2 + c, 3)];
+        if constexpr (sizeof(T) == 4) {
+            T x = q[c][W_PP] * (pp - p), y = q[c][W_PM] * (pm - p), z = q[c][W_GH] * (gh - p);
+            x = __fmaf_rn(q[c][W_P1], p1 - p, x);
+            y = __fmaf_rn(q[c][W_M1], m1 - p, y);
+            z = __fmaf_rn(q[c][W_I1], i1 - p, z);
+            x = __fmaf_rn(q[c][W_P2], p2 - p, x);
+            y = __fmaf_rn(q[c][W_M2], m2 - p, y);
+            z = __fmaf_rn(q[c][W_I2], i2 - p, z);
+            B[at(1 + c, 1)] = __fmaf_rn(q[c][W_F] - ((x + y) + z), q[c][W_D], p);
+            return;
+        }
         const T x0 = three * (p - i1) + i2, xm = three * (pm - m1) + m2, xp = three * (pp - p1) + p2;
         const T N0 = kHigh ? x0 : i1, S0 = kHigh ? i1 : x0, Np = kHigh ? xp : p1, Sp = kHigh ? p1 : xp;
         const T Nm = kHigh ? xm : m1, Sm = kHigh ? m1 : xm, gn = kHigh ? gh : i1, gs = kHigh ? i1 : gh;
@@ -328,44 +410,49 @@ struct SideLane {
         else n0 = neum ? nb[c] : n0;
         const T lphi = (t1 - t0) * idt + (n1 - n0) * idn;
         const T newphi = p + (q[c][Q_F] - lphi) * q[c][Q_D];
-        S[ad[1 + c][1]] = om * newphi + om1 * p;
+        B[at(1 + c, 1)] = om * newphi + om1 * p;
     }
-    // The edge cells colour by colour, then the corners: warps y low, y high, x
-    // low, x high take the corners (low, low), (low, high), (high, low), (high,
-    // high); on a grid of at least 4 x 4 they do not read each other.
-    __device__ __forceinline__ void pass(T* S, const T* strips, const Window& w, const GeoT<T>& g, const BCd& b,
-                                         int homog, int nx, int ny) const {
-#pragma unroll 1
-        for (int c = 0; c < 4; ++c) {
-            if (c == ph[0]) {
-                if (ok[0]) cell<0>(S);
-            } else if (c == ph[1]) {
-                if (ok[1]) cell<1>(S);
-            }
-            boundary_sync();
+    // The edge cells colour by colour, then the corners, which on a grid of at least
+    // 4 x 4 do not read each other.
+    template <int kPhase>
+    __device__ __forceinline__ void phase(T* S) const {
+        if (ph(0) == kPhase) {
+            if (ok[0]) cell<0>(S);
+        } else if (ph(1) == kPhase) {
+            if (ok[1]) cell<1>(S);
         }
-        constexpr bool hx = !kY, hy = kHigh;
-        const Per pr = periodic_of(b);
-        if ((threadIdx.x & 31) == 0 && (hx ? w.xh && !pr.xh : w.xl && !pr.xl) && (hy ? w.yh && !pr.yh : w.yl && !pr.yl)) {
+        boundary_sync();
+    }
+    __device__ __forceinline__ void pass(T* S, const T* strips, const Window& w, const GeoT<T>& g, const BCd& b,
+                                         int homog, int nx, int ny) {
+        phase<0>(S);
+        phase<1>(S);
+        phase<2>(S);
+        phase<3>(S);
+        grab(S);   // for the next sweep
+        if (corner) {
             const int i = hx ? nx - 1 : 0, j = hy ? ny - 1 : 0;
+            T* B = S + base - (kY ? 0 : C::P + 1);   // lane 0's place
             int x[4], y[4];
 #pragma unroll
             for (int r = 0; r < 4; ++r) {
-                x[r] = x_term<C>(i - w.ox + (r - 1) * (hx ? -1 : 1));
-                y[r] = y_term<C>(j - w.oy + (r - 1) * (hy ? -1 : 1));
+                x[r] = kY ? cz[r] : across(r);
+                y[r] = kY ? across(r) : cz[r];
             }
-            corner_cell<hx, hy>(S, strips + (hy ? kStrip * kAlong : 0) + i - w.ox, x, y, g, b, homog, i, j, om, om1);
+            corner_cell<hx, hy>(B, strips + (hy ? kStrip * kAlong : 0) + i - w.ox, x, y, g, b, homog, i, j, om, om1);
         }
     }
 };
 
-// Calls f with the side of warp v (0-3: y low, y high, x low, x high).
+// Calls f with the side of warp v (0-3: y low, y high, x low, x high) of window w.
 template <class C, class F>
-__device__ __forceinline__ void with_side(int v, F f) {
-    if (v == 0) f(SideLane<C, true, false>());
-    else if (v == 1) f(SideLane<C, true, true>());
-    else if (v == 2) f(SideLane<C, false, false>());
-    else if (v == 3) f(SideLane<C, false, true>());
+__device__ __forceinline__ void with_side(int v, const Window& w, int nx, int ny, F f) {
+    if (v == 0) f(SideLane<C, true, false, false>());
+    else if (v == 1 && ((ny - 1 - w.oy) & 1)) f(SideLane<C, true, true, true>());
+    else if (v == 1) f(SideLane<C, true, true, false>());
+    else if (v == 2) f(SideLane<C, false, false, false>());
+    else if (v == 3 && ((nx - 1 - w.ox) & 1)) f(SideLane<C, false, true, true>());
+    else if (v == 3) f(SideLane<C, false, true, false>());
 }
 
 // Ghosts no sweep changes, by warps 0-3: a Neumann side's, as stored, and the
@@ -542,20 +629,22 @@ __device__ __forceinline__ void sweep_window(T* s, T* strips, const DFT<T>& pin,
     const bool any_side = w.any();
     const T idx = T(g.idx), idy = T(g.idy), om = T(omega), om1 = T(1.0 - omega);
     if (warp >= C::NI) {   // the counterpart of the blocks' loop below, with the same CTA barriers
-        with_side<C>(warp - C::NI, [&](auto L) {
+        with_side<C>(warp - C::NI, w, nx, ny, [&](auto L) {
             L.place(w, g, b, homog, nx, ny, om, om1);
             cta_sync();   // phi and the strips are in place
             if (any_side) {
-                L.take(strips, w, b, homog);
+                L.grab(s);
                 L.fill(s, pin, w, b, homog, nx, ny, 0);
                 cta_sync();
+                L.take(strips, w, b, homog);
             }
 #pragma unroll 1
             for (int sw = 0; sw < K; ++sw) {
+                if (any_side) L.put(s);
                 for (int c = 0; c < 4; ++c) cta_sync();   // the interior colours
                 if (!any_side) continue;
                 L.pass(s, strips, w, g, b, homog, nx, ny);
-                if (sw + 1 < K) {
+                if (sw + 1 < K && !L.all_plain) {
                     boundary_sync();
                     L.fill(s, pin, w, b, homog, nx, ny, sw + 1);
                 }
@@ -612,7 +701,7 @@ __device__ __forceinline__ void sweep_window(T* s, T* strips, const DFT<T>& pin,
     }
     const unsigned mask = settle<C, false>(k, s, strips, w, kbx, kby, idx, idy, om, b, nx, ny);
     cta_sync();
-    if (any_side) cta_sync();   // 2. the sides' warps fill the first sweep's ghosts
+    if (any_side) cta_sync();   // 2. the sides' warps have read what the first sweep's ghosts are made of
 #pragma unroll 1
     for (int sw = 0; sw < K; ++sw) {
         // the boundary pass of the sweep before changed cells their owners hold
