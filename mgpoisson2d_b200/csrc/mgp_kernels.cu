@@ -927,23 +927,60 @@ cudaError_t launch_mdot(const DF& w, const MVec& V, int nv, int nx, int ny, doub
 // The multi-dot with kDotVecs basis vectors per launch row: a thread reads
 // w at a cell once for all of its row's vectors, so a pass reads w
 // ceil(nv / kDotVecs) times and each v_k once, where one row per vector read
-// w nv times.  partials[k * gridDim.x + b] = block b's sum of w * v_k.
+// w nv times.  partials[k * gridDim.x + b] = block b's sum of w * v_k.  The next
+// cell's place follows by addition (two 64-bit divisions a cell, for nine loads,
+// made it issue-bound) and two cells' loads are in flight at once: 50 vectors of
+// 1024^2 cells 98 -> 86 us (they are 66 us of memory).
 constexpr int kDotVecs = 8;
 
 __global__ void __launch_bounds__(kMdotThreads) k_mdot8(DF w, MVec V, int nv, int nx, int ny, double* partials) {
     __shared__ double sh[kDotVecs][kMdotThreads];
     const int k0 = blockIdx.y * kDotVecs, kn = min(kDotVecs, nv - k0);
-    const long n = (long)nx * ny;
+    const long n = (long)nx * ny, step = (long)gridDim.x * blockDim.x;
+    const int di = (int)(step % nx), dj = (int)(step / nx);
     double acc[kDotVecs];
 #pragma unroll
     for (int q = 0; q < kDotVecs; ++q) acc[q] = 0.0;
-    for (long c = (long)blockIdx.x * blockDim.x + threadIdx.x; c < n; c += (long)gridDim.x * blockDim.x) {
-        const int i = (int)(c % nx), j = (int)(c / nx);
+    const long c0 = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    int i = (int)(c0 % nx), j = (int)(c0 / nx);
+    const double* base = V.p + (long)k0 * V.stride;
+    const auto next = [&]() {
+        i += di;
+        j += dj;
+        if (i >= nx) {
+            i -= nx;
+            ++j;
+        }
+    };
+    long c = c0;
+    if (kn == kDotVecs) {
+        for (; c + step < n; c += 2 * step) {
+            const double w0 = AT(w, i, j);
+            const double* v0 = base + i + (long)j * V.ld;
+            next();
+            const double w1 = AT(w, i, j);
+            const double* v1 = base + i + (long)j * V.ld;
+            next();
+            double a[kDotVecs], b[kDotVecs];
+#pragma unroll
+            for (int q = 0; q < kDotVecs; ++q) {
+                a[q] = v0[(long)q * V.stride];
+                b[q] = v1[(long)q * V.stride];
+            }
+#pragma unroll
+            for (int q = 0; q < kDotVecs; ++q) {
+                acc[q] = acc[q] + w0 * a[q];
+                acc[q] = acc[q] + w1 * b[q];
+            }
+        }
+    }
+    for (; c < n; c += step) {
         const double wv = AT(w, i, j);
-        const double* v = V.p + (long)k0 * V.stride + i + (long)j * V.ld;
+        const double* v = base + i + (long)j * V.ld;
 #pragma unroll
         for (int q = 0; q < kDotVecs; ++q)
             if (q < kn) acc[q] = acc[q] + wv * v[(long)q * V.stride];
+        next();
     }
 #pragma unroll
     for (int q = 0; q < kDotVecs; ++q) sh[q][threadIdx.x] = acc[q];
