@@ -1071,19 +1071,6 @@ int smooth_body(mgp_solver* s, int d, int nu) {
     return MGP_OK;
 }
 
-int residual_level(mgp_solver* s, int d) {
-    Lv& L = s->lv[d];
-    cudaStream_t st = s->stream;
-    if (s->kind == MGP_KIND_DD) {
-        CK(launch_dd_apply(L.w, L.e, L.r, L.g, L.bc, L.nx, L.ny, 1, st));
-        CK(launch_fill(L.e, L.g, L.bc, 1, 1, L.nx, L.ny, st));
-    } else {
-        CK(launch_fill(L.e, L.g, L.bc, 1, 0, L.nx, L.ny, st));
-        CK(launch_apply(L.w, L.e, L.r, L.g, L.bc, 1, L.nx, L.ny, 1, 0, st));
-    }
-    return MGP_OK;
-}
-
 // prolong(e(d), e(d+1), ..., order), MG:262-394.
 int prolong_level(mgp_solver* s, int d, int order) {
     Lv &F = s->lv[d], &Cl = s->lv[d + 1];
@@ -1142,23 +1129,26 @@ int coarse_cycle(mgp_solver* s, int d, int numcycles, int nd, int nu, int nb) {
     return MGP_OK;
 }
 
-// vcycle_noinit(depth), MG:675-854 / DD:867-1045.
-int vcycle_noinit(mgp_solver* s, int d, int numcycles, int nd, int nu, int nb) {
+// vcycle_noinit(depth), MG:675-854 / DD:867-1045.  guessed: the level's guess
+// (DD:971) was made with its right-hand side.
+int vcycle_noinit(mgp_solver* s, int d, int numcycles, int nd, int nu, int nb, bool guessed = false) {
     if (d >= s->dc) return coarse_cycle(s, d, numcycles, nd, nu, nb);
     Lv &L = s->lv[d], &Cl = s->lv[d + 1];
     cudaStream_t st = s->stream;
     const bool dd = (s->kind == MGP_KIND_DD);
-    if (dd) CK(launch_set_guess(L.e, L.r, L.invd, L.nx, L.ny, st));   // DD:971
+    if (dd && !guessed) CK(launch_set_guess(L.e, L.r, L.invd, L.nx, L.ny, st));   // DD:971
     RC(smooth(s, d, nd));
-    if (dd) {
-        RC(residual_level(s, d));
-        CK(launch_restrict(L.w, Cl.r, Cl.nx, Cl.ny, s->refx[d], s->refy[d], 0, st));
+    const bool guess = numcycles > 0 && d + 1 < s->dc;   // (the coarse cycle makes its own; a level not visited has none)
+    if (dd) {   // residual (DD:99), restriction and the coarse guess in one pass, then the ghosts it leaves
+        CK(launch_dd_resid_restrict(L.e, L.r, L.g, L.bc, L.nx, L.ny, Cl.r, Cl.e, Cl.invd, Cl.nx, Cl.ny, s->refx[d],
+                                    s->refy[d], guess, st));
+        CK(launch_fill(L.e, L.g, L.bc, 1, 1, L.nx, L.ny, st));
     } else {   // residual (MG:793-795), restriction and the coarse guess (MG:805-806) in one pass
         CK(launch_fill(L.e, L.g, L.bc, 1, 0, L.nx, L.ny, st));
         CK(launch_resid_restrict(L.e, L.r, L.g, L.bc, 1, L.nx, L.ny, Cl.r, Cl.e, Cl.invd, Cl.nx, Cl.ny, s->refx[d],
                                  s->refy[d], 1, st));
     }
-    for (int c = 1; c <= numcycles; ++c) RC(vcycle_noinit(s, d + 1, numcycles, nd, nu, nb));
+    for (int c = 1; c <= numcycles; ++c) RC(vcycle_noinit(s, d + 1, numcycles, nd, nu, nb, dd && guess && c == 1));
     RC(prolong_level(s, d, 1));
     RC(smooth(s, d, nu));
     return MGP_OK;
@@ -1170,7 +1160,7 @@ int vcycle_noinit(mgp_solver* s, int d, int numcycles, int nd, int nu, int nb) {
 // restriction into level dc writes the FP64 right-hand side of the coarse
 // CTA's levels (which, with the bottom solve, stay FP64) and the prolongation
 // from level dc reads its FP64 correction.
-int vcycle32(mgp_solver* s, int d, int numcycles, int nd, int nu, int nb) {
+int vcycle32(mgp_solver* s, int d, int numcycles, int nd, int nu, int nb, bool guessed = false) {
     auto& L = s->lv32[d];
     const Lv& F = s->lv[d];   // BCs of the level
     cudaStream_t st = s->stream;
@@ -1181,7 +1171,7 @@ int vcycle32(mgp_solver* s, int d, int numcycles, int nd, int nu, int nb) {
     auto round16 = [&](const DF32& f, int lvl, int nx_, int ny_, int g) -> cudaError_t {
         return (b16 && lvl >= 1) ? launch_round_bf16(f, nx_, ny_, g, st) : cudaSuccess;
     };
-    if (dd) CK(launch_set_guess(L.e, L.r, L.invd, L.nx, L.ny, st));   // DD:971
+    if (dd && !guessed) CK(launch_set_guess(L.e, L.r, L.invd, L.nx, L.ny, st));   // DD:971
     auto smooth32 = [&](int nu_) -> int {
         return timed_smooth(s, d, nu_, [&]() -> int {
             if (dd) {
@@ -1225,16 +1215,16 @@ int vcycle32(mgp_solver* s, int d, int numcycles, int nd, int nu, int nb) {
     const int rx = s->refx[d], ry = s->refy[d];
     const bool fine_next = d + 1 < s->dc;
     Lv& C = s->lv[d + 1];
+    const bool guess = dd && !b16 && numcycles > 0 && fine_next;
     if (dd) {
-        CK(launch_dd_apply(L.w, L.e, L.r, L.g, F.bc, L.nx, L.ny, 1, st));
-        CK(launch_fill(L.e, L.g, F.bc, 1, 1, L.nx, L.ny, st));
-        if (fine_next) {
+        if (fine_next) {   // the BF16 study makes the guess of the rounded right-hand side
             auto& N = s->lv32[d + 1];
-            CK(launch_restrict(L.w, N.r, N.nx, N.ny, rx, ry, st));
+            CK(launch_dd_resid_restrict(L.e, L.r, L.g, F.bc, L.nx, L.ny, N.r, N.e, N.invd, N.nx, N.ny, rx, ry, guess, st));
             CK(round16(N.r, d + 1, N.nx, N.ny, 0));
         } else {
-            CK(launch_restrict(L.w, C.r, C.nx, C.ny, rx, ry, st));
+            CK(launch_dd_resid_restrict(L.e, L.r, L.g, F.bc, L.nx, L.ny, C.r, C.e, C.invd, C.nx, C.ny, rx, ry, 0, st));
         }
+        CK(launch_fill(L.e, L.g, F.bc, 1, 1, L.nx, L.ny, st));
     } else {   // residual (MG:793-795), restriction and the coarse guess (MG:805-806) in one pass
         CK(launch_fill(L.e, L.g, F.bc, 1, 0, L.nx, L.ny, st));
         if (fine_next) {
@@ -1248,7 +1238,7 @@ int vcycle32(mgp_solver* s, int d, int numcycles, int nd, int nu, int nb) {
     }
     if (fine_next) {
         auto& N = s->lv32[d + 1];
-        for (int c = 1; c <= numcycles; ++c) RC(vcycle32(s, d + 1, numcycles, nd, nu, nb));
+        for (int c = 1; c <= numcycles; ++c) RC(vcycle32(s, d + 1, numcycles, nd, nu, nb, guess && c == 1));
         CK(launch_fill(N.e, N.g, C.bc, 1, 1, N.nx, N.ny, st));    // MG:318
         CK(round16(N.e, d + 1, N.nx, N.ny, 1));
         CK(launch_prolong(L.e, N.e, N.nx, N.ny, rx, ry, 1, st));

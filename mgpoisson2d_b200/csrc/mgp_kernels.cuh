@@ -132,8 +132,6 @@ cudaError_t launch_fill(const DF32& p, const Geo32& g, const BCd& b, int homog, 
 cudaError_t launch_apply(const DF32& out, const DF32& phi, const DF32& rhs, const Geo32& g, const BCd& b, int homog,
                          int nx, int ny, int mode, int jscale, cudaStream_t st);
 // Cell-centred restriction into an FP32 or an FP64 coarse field.
-cudaError_t launch_restrict(const DF32& f, const DF32& c, int ncx, int ncy, int refx, int refy, cudaStream_t st);
-cudaError_t launch_restrict(const DF32& f, const DF& c, int ncx, int ncy, int refx, int refy, cudaStream_t st);
 // Prolongation from an FP32 or an FP64 coarse field (arithmetic in the coarse type).
 cudaError_t launch_prolong(const DF32& fine, const DF32& crse, int ncx, int ncy, int refx, int refy, int order,
                            cudaStream_t st);
@@ -152,6 +150,16 @@ cudaError_t launch_resid_restrict(const DF32& phi, const DF32& rhs, const Geo32&
 cudaError_t launch_resid_restrict(const DF32& phi, const DF32& rhs, const Geo32& g, const BCd& b, int homog, int nx,
                                   int ny, const DF& rc, const DF& ec, const DF& invdc, int ncx, int ncy, int refx,
                                   int refy, int guess, cudaStream_t st);
+// The same with the deferred-correction operator.
+cudaError_t launch_dd_resid_restrict(const DF& phi, const DF& rhs, const Geo& g, const BCd& b, int nx, int ny,
+                                     const DF& rc, const DF& ec, const DF& invdc, int ncx, int ncy, int refx, int refy,
+                                     int guess, cudaStream_t st);
+cudaError_t launch_dd_resid_restrict(const DF32& phi, const DF32& rhs, const Geo32& g, const BCd& b, int nx, int ny,
+                                     const DF32& rc, const DF32& ec, const DF32& invdc, int ncx, int ncy, int refx, int refy,
+                                     int guess, cudaStream_t st);
+cudaError_t launch_dd_resid_restrict(const DF32& phi, const DF32& rhs, const Geo32& g, const BCd& b, int nx, int ny,
+                                     const DF& rc, const DF& ec, const DF& invdc, int ncx, int ncy, int refx, int refy,
+                                     int guess, cudaStream_t st);
 cudaError_t launch_sub_mean(const DF32& y, const double* out, int nx, int ny, int gx, int gy, cudaStream_t st);
 cudaError_t launch_reduce(int kind, const DF32& a, const DF32& b, int nx, int ny, double vol, double* partials,
                           double* out, cudaStream_t st);
@@ -362,8 +370,6 @@ cudaError_t launch_div(const DF& div, const DF& xflux, const DF& yflux, int nx, 
                        cudaStream_t st);
 // Deferred-correction operators.
 cudaError_t launch_dd_invdiag(const DF& invd, const Geo& g, int nx, int ny, cudaStream_t st);
-cudaError_t launch_dd_apply(const DF& out, const DF& phi, const DF& rhs, const Geo& g, const BCd& b, int nx, int ny,
-                            int mode, cudaStream_t st);
 cudaError_t launch_dd_modrhs(const DF& out, const DF& phi, const DF& rhs, const Geo& g, int nx, int ny,
                              cudaStream_t st);
 cudaError_t launch_dd_colour(const DF& phi, const DF& modrhs, const DF& invd, const Geo& g, int nx, int ny,
@@ -379,8 +385,6 @@ cudaError_t launch_dd_sweeps(const DF& pin, const DF& pout, const DF& m, const D
 cudaError_t launch_dd_sweeps(const DF32& pin, const DF32& pout, const DF32& m, const DF32& invd, const Geo32& g,
                              const BCd& b, int nx, int ny, double omega, int left, int* done, cudaStream_t st);
 // The same three on FP32 fields (the grid levels of a mixed-precision DD V-cycle).
-cudaError_t launch_dd_apply(const DF32& out, const DF32& phi, const DF32& rhs, const Geo32& g, const BCd& b, int nx,
-                            int ny, int mode, cudaStream_t st);
 cudaError_t launch_dd_modrhs(const DF32& out, const DF32& phi, const DF32& rhs, const Geo32& g, int nx, int ny,
                              cudaStream_t st);
 cudaError_t launch_dd_colour(const DF32& phi, const DF32& modrhs, const DF32& invd, const Geo32& g, int nx, int ny,
