@@ -15,8 +15,10 @@
  *    element of the allocation (bx%ilo, bx%jlo) plus its leading dimension and
  *    ghost counts, so a Fortran caller passes c_loc(bd%data) without a copy.
  *  - Pointers may be host or device memory; the library asks the CUDA driver
- *    which one each pointer is (cudaPointerGetAttributes).  Host arrays are
- *    staged through device buffers inside the call.
+ *    which one each pointer is.  Operator-level calls work on a device array
+ *    where it lies, if it has the ghost layers the call needs and, where it is
+ *    written, shares no memory with another array of the call; other arrays
+ *    are staged through device buffers inside the call.
  *  - All arithmetic is IEEE FP64 without fused multiply-add, in the same
  *    operation order as the Fortran routines (MGP_FLAG_MIXED, an opt-in
  *    extension, runs the V-cycle's grid levels in FP32).
@@ -437,8 +439,9 @@ int mgp_batch_vcycle(mgp_batch *b, mgp_array *phi, mgp_array *rhs, const mgp_bdr
  * results: groups = how many groups of problems run their lockstep loops
  * concurrently, each on its own stream (1 .. nstreams; 0 restores the
  * default, min(4, nstreams)); pairs = 1 runs two sweeps per launch on the
- * levels whose descriptors allow it (when the smoothing counts are multiples
- * of 4).  mgpoisson2d_b200.api.Batch.autotune times the combinations and
+ * levels whose descriptors allow it, however many tiles they have (when the
+ * smoothing counts are multiples of 4; without it a level takes four or two
+ * sweeps a launch where the group's tiles do not outnumber the SMs).  mgpoisson2d_b200.api.Batch.autotune times the combinations and
  * caches the fastest.  No reference counterpart. */
 int mgp_batch_set_tuning(mgp_batch *b, int groups, int pairs);
 int mgp_batch_get_tuning(const mgp_batch *b, int *groups, int *pairs);
