@@ -177,10 +177,11 @@ typedef struct mgp_report {
  * than 1024 cells (the schedule stops at an odd side, so it is the coarsest),
  * the exact bottom is a block cyclic reduction over its lines (2 log2(lines) + 1
  * launches a solve; 40 cells x shorter side bytes of factors), if the shorter
- * side has 5 to 160 cells, not both axes are periodic, the factors take at most
- * 256 MB that the device has, and the factorisation, tried on a right-hand side,
- * solves to 1e-8.  Otherwise, or where that level lies below one of at most 64
- * cells, MGP_FLAG_DIRECT_COARSE alone applies.  No reference counterpart. */
+ * side has 5 to 160 cells and the longer at most 16384, not both axes are
+ * periodic, the factors take at most 256 MB that the device has, and the
+ * factorisation, tried on a right-hand side, solves to 1e-8.  Otherwise, or
+ * where that level lies below one of at most 64 cells, MGP_FLAG_DIRECT_COARSE
+ * alone applies.  No reference counterpart. */
 #define MGP_FLAG_DIRECT_LARGE 64
 /* mgp_batch only: solve the batch in lockstep.  Every phase of the V-cycle --
  * a level's smoothing sweeps, its ghost fill, the residual restricted to the

@@ -293,7 +293,8 @@ bool block_bottom_shape(int nx, int ny, const BCd& bc, BlockBottom* b) {
     b->along_y = px ? 1 : py ? 0 : nx <= ny;
     b->m = b->along_y ? nx : ny;
     b->lines = b->along_y ? ny : nx;
-    return b->m >= 5 && b->lines >= 6 && b->m <= kBlockLineMax &&
+    // (lines: a launch has a block of the grid's second dimension per product, at most two a line)
+    return b->m >= 5 && b->lines >= 6 && b->m <= kBlockLineMax && b->lines <= kBlockLinesMax &&
            5.0 * b->lines * b->m * b->m * sizeof(double) <= (double)kBlockBytesMax;
 }
 

@@ -423,6 +423,7 @@ cudaError_t launch_relax_block(const Lv& L, const DF& phi, const DF& rhs, int ho
 // The exact bottom of a level of more than kDirectLargeCells cells (mgp_bottom.cu):
 // block cyclic reduction over its lines of m cells.
 constexpr int kBlockLineMax = 160;                  // an inverted block fits one CTA's shared memory
+constexpr int kBlockLinesMax = 16384;
 constexpr int kBlockStepsMax = 16;
 constexpr size_t kBlockBytesMax = 256ull << 20;     // of factors
 struct BlockBottom {
