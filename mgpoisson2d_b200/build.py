@@ -17,7 +17,7 @@ INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 LIB = os.path.join(HERE, "libmgp2d.so")
 SOURCES = ["mgp_kernels.cu", "mgp_sweep.cu", "mgp_ddsweep.cu", "mgp_bottom.cu", "mgp_host.cu", "mgp_noalloc.cu", "mgp_batch.cu", "mgp_geometry.cu",
            "mgp_lockstep.cu"]
-HEADERS = ["mgp_core.cuh", "mgp_kernels.cuh", "mgp_sweep.cuh", "mgp_ddsweep.cuh"]
+HEADERS = ["mgp_core.cuh", "mgp_kernels.cuh", "mgp_stage.cuh", "mgp_sweep.cuh", "mgp_ddsweep.cuh"]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",

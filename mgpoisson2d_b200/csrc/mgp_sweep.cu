@@ -46,6 +46,7 @@
 #include <type_traits>
 
 #include "mgp_kernels.cuh"
+#include "mgp_stage.cuh"
 #include "mgp_sweep.cuh"
 
 namespace mgp {
@@ -207,11 +208,10 @@ __device__ __forceinline__ void sweep_stream(int total, int homog, double omega,
     grid_dependency_wait();
     if (issuer) load_fields(tiles[0]);
     cta_sync();
-    unsigned parity = 0;
     // One tile; kInner: of the inner region, without sides.  (Two copies: the
     // sides' code takes so many registers that the FP32 kernel spills, which the
-    // inner tiles then do not see.)  False after the last one.
-    const auto tile = [&](auto inner_tag, int it) -> bool {
+    // inner tiles then do not see.)
+    const auto tile = [&](auto inner_tag, int it) -> TileEnd {
         constexpr bool kInner = decltype(inner_tag)::value;
         const Window& w = tiles[it].w;
         const LevelRef<T>& L0 = levels[it];
@@ -244,8 +244,12 @@ __device__ __forceinline__ void sweep_stream(int total, int homog, double omega,
         const unsigned mask =
             settle<C, kInner>(k, s, strips, w, kbx, kby, idx, idy, om, *L0.b, L0.nx, L0.ny);
         cta_sync();   // the planes are in place, the staging buffer is read and the next tile placed
+        // A thread gave up on the loads, so what was read may be anything: nothing is
+        // stored.  (Decided at this barrier, which the tile needs anyway, not at one
+        // of its own before the staging buffer is read.)
+        if (bad) return TILE_LOST;
         const bool more = tiles[it ^ 1].t >= 0;
-        if (issuer && more && !bad) {
+        if (issuer && more) {
             load_const(tiles[it ^ 1]);
             load_fields(tiles[it ^ 1]);
         }
@@ -271,11 +275,12 @@ __device__ __forceinline__ void sweep_stream(int total, int homog, double omega,
             store_ghosts<C>(s, *L0.pout, w, warp, L0.nx, L0.ny);
         }
         store_block<true>(k, *L0.pout, w, w.ox + 2 * kbx, w.oy + 2 * kby);
-        return more;
+        if (more) cta_sync();   // the planes are read no more
+        return more ? TILE_MORE : TILE_LAST;
     };
-#pragma unroll 1
-    for (int it = 0;; it ^= 1) {
-        if (issuer) {   // the tile after this one, while this one's loads are in flight
+    walk_tiles(
+        [&](int it) {   // the tile after this one, while this one's loads are in flight
+            if (!issuer) return;
             NextTile& n = tiles[it ^ 1];
             n.t = tiles[it].t + gridDim.x;
             n.job = tiles[it].job;
@@ -285,19 +290,16 @@ __device__ __forceinline__ void sweep_stream(int total, int homog, double omega,
             } else {
                 n.t = -1;
             }
-        }
-        if (!mbar_wait(bar, parity)) {   // never seen: report, finish the tile (its result is void) and stop
-            bad = 1;
+        },
+        [&](unsigned parity) {
+            if (mbar_wait(bar, parity)) return;
+            bad = 1;   // never seen
             if (lane == 0) set_status(status, DST_TIMEOUT);
-        }
-        parity ^= 1;
-        if (!(tiles[it].inner ? tile(std::true_type(), it) : tile(std::false_type(), it))) break;
-        cta_sync();   // the planes are read no more
-        if (bad) {
-            if (issuer) mbar_wait(bar, parity);   // let copies still in flight land before the CTA exits
-            break;
-        }
-    }
+        },
+        [&](int it) { return tiles[it].inner ? tile(std::true_type(), it) : tile(std::false_type(), it); },
+        [&](unsigned parity) {   // let copies still in flight land before the CTA exits
+            if (issuer) mbar_wait(bar, parity);
+        });
 }
 
 template <class C>
