@@ -451,7 +451,10 @@ typedef struct mgp_server mgp_server;
 /* A solve server with nworkers slots.  Requests start in arrival order as a
  * slot frees up and the device memory their hierarchy needs fits within
  * mem_budget bytes (0: 90% of the memory free at creation), evicting idle
- * cached hierarchies first.  The hierarchy of a request with a nonzero key
+ * cached hierarchies first.  The factors of an exact bottom of more than 1024
+ * cells (MGP_FLAG_DIRECT_LARGE) count with their set-up's scratch; a request
+ * that fits the budget only without them is solved with the reference bottom.
+ * The hierarchy of a request with a nonzero key
  * stays resident and serves later requests with the same key and box. */
 int mgp_server_create(int nworkers, size_t mem_budget, int flags, mgp_server **out);
 /* Queue one vcycle solve (the mgp_solver_vcycle arguments).  Every array the

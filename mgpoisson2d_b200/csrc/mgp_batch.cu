@@ -32,6 +32,7 @@ int record_error(int code, const char* msg);
 int solver_create_on(const mgp_box* valid, const mgp_geo* geo, const mgp_bdry* bc, int kind, int flags,
                      int maxdepth_user, cudaStream_t st, mgp_solver** out);
 size_t solver_device_bytes(const mgp_solver* s);
+size_t solver_block_bottom_bytes(const mgp_box* v, const mgp_bdry* bc, int kind, int flags);
 size_t solver_pool_cached_bytes();
 struct Lockstep;
 Lockstep* lockstep_new();
@@ -54,7 +55,8 @@ double now_s() {
 // fields ~21 per cell over all levels (geometry, inverse diagonal,
 // corrections, residuals, the BiCGStab vectors), FP32 copies ~14, with
 // MGP_FLAG_GMRES the 2m + 1 = 257 stored fields of GMRES(128), plus padding
-// and the small buffers.
+// and the small buffers.  (The factors of an exact bottom of more than 1024 cells
+// are solver_block_bottom_bytes.)
 size_t estimate_bytes(const mgp_box* v, int flags) {
     const double n = (double)v->nx * (double)v->ny;
     const double per = 8.0 * 21.0 + ((flags & MGP_FLAG_MIXED) ? 4.0 * 14.0 : 0.0) +
@@ -332,7 +334,7 @@ void serve(mgp_server* S) {
         mgp_solver* sv = nullptr;
         size_t bytes = 0;
         bool cached = false;
-        int rc = MGP_OK;
+        int rc = MGP_OK, flags = S->flags;
         std::vector<mgp_solver*> doomed;
         {
             std::unique_lock<std::mutex> lock(S->mu);
@@ -348,6 +350,13 @@ void serve(mgp_server* S) {
             }
             if (!sv) {   // admission by device memory
                 bytes = estimate_bytes(&r->valid, S->flags);
+                // The factors of a large exact bottom are optional: counted where
+                // the budget holds them beside the hierarchy, else left out.  Only
+                // the request and the budget decide, so a result does not depend on
+                // what else runs.
+                const size_t factors = solver_block_bottom_bytes(&r->valid, &r->bc, MGP_KIND_MG, S->flags);
+                if (bytes + factors <= S->budget) bytes += factors;
+                else if (factors) flags &= ~MGP_FLAG_DIRECT_LARGE;
                 if (bytes > S->budget) {   // could never fit, even with every other hierarchy gone
                     rc = record_error(MGP_ENOMEM, "server: the request's hierarchy is larger than the memory budget");
                 } else {
@@ -371,7 +380,7 @@ void serve(mgp_server* S) {
         const bool held = !rc;
         for (mgp_solver* d : doomed) mgp_solver_destroy(d);
         if (!sv && !rc) {
-            rc = solver_create_on(&r->valid, &r->geo, &r->bc, MGP_KIND_MG, S->flags, -1, st, &sv);
+            rc = solver_create_on(&r->valid, &r->geo, &r->bc, MGP_KIND_MG, flags, -1, st, &sv);
             const size_t actual = rc ? 0 : solver_device_bytes(sv);
             std::lock_guard<std::mutex> lock(S->mu);
             S->used = S->used - bytes + actual;

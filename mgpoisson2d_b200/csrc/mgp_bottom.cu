@@ -283,39 +283,8 @@ struct Step {
     std::vector<BlockMul> first, second;
 };
 
-}  // namespace
-
-bool block_bottom_shape(int nx, int ny, const BCd& bc, BlockBottom* b) {
-    for (int k = 0; k < 4; ++k)
-        if (bc.type[k] != T_DIRI && bc.type[k] != T_NEUM && bc.type[k] != T_PERIODIC) return false;
-    const bool px = bc.type[0] == T_PERIODIC, py = bc.type[2] == T_PERIODIC;
-    if ((px && py) || px != (bc.type[1] == T_PERIODIC) || py != (bc.type[3] == T_PERIODIC)) return false;
-    b->along_y = px ? 1 : py ? 0 : nx <= ny;
-    b->m = b->along_y ? nx : ny;
-    b->lines = b->along_y ? ny : nx;
-    // (lines: a launch has a block of the grid's second dimension per product, at most two a line)
-    return b->m >= 5 && b->lines >= 6 && b->m <= kBlockLineMax && b->lines <= kBlockLinesMax &&
-           5.0 * b->lines * b->m * b->m * sizeof(double) <= (double)kBlockBytesMax;
-}
-
-cudaError_t launch_block_bottom(const BlockBottom& b, const DF& e, const DF& r, cudaStream_t st) {
-    const unsigned rows = (b.m + kRowsPerCta - 1) / kRowsPerCta;
-    cudaError_t err = cudaSuccess;
-    for (int l = 0; l < b.steps && err == cudaSuccess; ++l)
-        err = launch_step(k_bb_down, dim3(rows, b.ndown[l]), st, b, r, (int)(l == 0), b.items + b.odown[l]);
-    for (int l = b.steps; l >= 0 && err == cudaSuccess; --l)
-        err = launch_step(k_bb_up, dim3(rows, b.nup[l]), st, b, e, r, (int)(l == 0), b.items + b.oup[l]);
-    return err;
-}
-
-cudaError_t block_bottom_build(BlockBottom* b, const Geo& g, const BCd& bc, int nx, int ny, const BlockAlloc& mem,
-                               cudaStream_t st, bool* ok) {
-    *ok = false;
-    const int m = b->m, B = b->lines;
-    const size_t mm = (size_t)m * m;
-    const bool px = bc.type[0] == T_PERIODIC, py = bc.type[2] == T_PERIODIC;
-    const bool pc = b->along_y ? px : py;
-    // the order of elimination
+// The order of elimination of B lines.
+std::vector<Step> elimination(int B) {
     std::vector<Step> steps;
     std::vector<int> act(B);
     for (int k = 0; k < B; ++k) act[k] = k;
@@ -343,9 +312,73 @@ cudaError_t block_bottom_build(BlockBottom* b, const Geo& g, const BCd& bc, int 
         steps.push_back(s);
         act = keep;
     }
+    return steps;
+}
+
+// Doubles of memory: what the solves read (keep), and the set-up's own (temp).
+struct Sizes {
+    int nfg, nc, nl, np;   // blocks of F and G; probing colours across and along the lines, and fields
+    bool pc;               // the lines close on themselves
+    size_t ld, field, keep, temp;
+    Sizes(const BlockBottom& b, int nx, int ny, bool px, bool py) {
+        const size_t mm = (size_t)b.m * b.m;
+        nfg = 0;
+        for (const Step& s : elimination(b.lines)) nfg += 2 * (int)s.down.size();
+        pc = b.along_y ? px : py;
+        nc = probe_colours(b.m, pc);
+        nl = probe_colours(b.lines, false);
+        np = nc * nl;
+        ld = nx + 2;
+        field = ld * (ny + 2);
+        keep = (size_t)(3 * b.lines + nfg) * mm + (size_t)b.lines * b.m;
+        temp = (size_t)(2 * b.lines + 2) * mm + (size_t)(np + 3) * field;
+    }
+};
+
+}  // namespace
+
+bool block_bottom_shape(int nx, int ny, const BCd& bc, BlockBottom* b) {
+    for (int k = 0; k < 4; ++k)
+        if (bc.type[k] != T_DIRI && bc.type[k] != T_NEUM && bc.type[k] != T_PERIODIC) return false;
+    const bool px = bc.type[0] == T_PERIODIC, py = bc.type[2] == T_PERIODIC;
+    if ((px && py) || px != (bc.type[1] == T_PERIODIC) || py != (bc.type[3] == T_PERIODIC)) return false;
+    b->along_y = px ? 1 : py ? 0 : nx <= ny;
+    b->m = b->along_y ? nx : ny;
+    b->lines = b->along_y ? ny : nx;
+    // (lines: a launch has a block of the grid's second dimension per product, at most two a line)
+    return b->m >= 5 && b->lines >= 6 && b->m <= kBlockLineMax && b->lines <= kBlockLinesMax &&
+           5.0 * b->lines * b->m * b->m * sizeof(double) <= (double)kBlockBytesMax;
+}
+
+size_t block_bottom_peak_bytes(int nx, int ny, const BCd& bc) {
+    BlockBottom b = {};
+    if (!block_bottom_shape(nx, ny, bc, &b)) return 0;
+    const Sizes z(b, nx, ny, bc.type[0] == T_PERIODIC, bc.type[2] == T_PERIODIC);
+    // the launches' items and the products' jobs: at most one and five a line and step
+    return (z.keep + z.temp) * sizeof(double) + (size_t)2 * b.lines * (sizeof(int4) + 5 * sizeof(BlockMul));
+}
+
+cudaError_t launch_block_bottom(const BlockBottom& b, const DF& e, const DF& r, cudaStream_t st) {
+    const unsigned rows = (b.m + kRowsPerCta - 1) / kRowsPerCta;
+    cudaError_t err = cudaSuccess;
+    for (int l = 0; l < b.steps && err == cudaSuccess; ++l)
+        err = launch_step(k_bb_down, dim3(rows, b.ndown[l]), st, b, r, (int)(l == 0), b.items + b.odown[l]);
+    for (int l = b.steps; l >= 0 && err == cudaSuccess; --l)
+        err = launch_step(k_bb_up, dim3(rows, b.nup[l]), st, b, e, r, (int)(l == 0), b.items + b.oup[l]);
+    return err;
+}
+
+cudaError_t block_bottom_build(BlockBottom* b, const Geo& g, const BCd& bc, int nx, int ny, const BlockAlloc& mem,
+                               cudaStream_t st, bool* ok) {
+    *ok = false;
+    const int m = b->m, B = b->lines;
+    const size_t mm = (size_t)m * m;
+    const bool px = bc.type[0] == T_PERIODIC, py = bc.type[2] == T_PERIODIC;
+    const Sizes sz(*b, nx, ny, px, py);
+    std::vector<Step> steps = elimination(B);
     if ((int)steps.size() > kBlockStepsMax) return cudaSuccess;
     Step top;
-    top.up.push_back(int4{act[0], -1, -1, 0});
+    top.up.push_back(int4{steps.back().down[0].x, -1, -1, 0});   // the line that is left
     steps.push_back(top);
     b->steps = (int)steps.size() - 1;
     std::vector<int4> items;
@@ -357,15 +390,12 @@ cudaError_t block_bottom_build(BlockBottom* b, const Geo& g, const BCd& bc, int 
         b->nup[l] = (int)steps[l].up.size();
         items.insert(items.end(), steps[l].up.begin(), steps[l].up.end());
     }
-    // memory: what the solves read, and the set-up's own
-    const int nc = probe_colours(m, pc), nl = probe_colours(B, false), np = nc * nl;
-    const size_t ld = nx + 2, field = ld * (ny + 2);
-    const size_t keep_d = (size_t)(3 * B + nfg) * mm + (size_t)B * m;
-    const size_t temp_d = (size_t)(2 * B + 2) * mm + (size_t)(np + 3) * field;
-    double* keep = (double*)mem.get(mem.ctx, keep_d * sizeof(double));
+    const int nc = sz.nc, nl = sz.nl, np = sz.np;
+    const size_t ld = sz.ld, field = sz.field;
+    double* keep = (double*)mem.get(mem.ctx, sz.keep * sizeof(double));
     b->mem = keep;
     b->items = (int4*)mem.get(mem.ctx, items.size() * sizeof(int4));
-    double* temp = (double*)mem.get(mem.ctx, temp_d * sizeof(double));
+    double* temp = (double*)mem.get(mem.ctx, sz.temp * sizeof(double));
     std::vector<BlockMul> jobs;
     std::vector<int> n1, n2;
     double *D = keep, *P = keep + B * mm, *Q = keep + 2 * B * mm, *FG = keep + 3 * B * mm;
@@ -410,11 +440,11 @@ cudaError_t block_bottom_build(BlockBottom* b, const Geo& g, const BCd& bc, int 
         b->p = P;
         b->q = Q;
         b->fg = FG;
-        b->r = keep + (size_t)(3 * B + nfg) * mm;
-        b->bytes = keep_d * sizeof(double) + items.size() * sizeof(int4);
+        b->r = keep + (size_t)(3 * B + sz.nfg) * mm;
+        b->bytes = sz.keep * sizeof(double) + items.size() * sizeof(int4);
         step(cudaMemsetAsync(fail, 0, sizeof(int), st));
-        step(cudaMemsetAsync(keep, 0, keep_d * sizeof(double), st));
-        step(cudaMemsetAsync(temp, 0, temp_d * sizeof(double), st));
+        step(cudaMemsetAsync(keep, 0, sz.keep * sizeof(double), st));
+        step(cudaMemsetAsync(temp, 0, sz.temp * sizeof(double), st));
         step(cudaMemcpyAsync(b->items, items.data(), items.size() * sizeof(int4), cudaMemcpyHostToDevice, st));
         step(cudaMemcpyAsync(djobs, jobs.data(), jobs.size() * sizeof(BlockMul), cudaMemcpyHostToDevice, st));
         const auto at = [&](int k) { return DF{out + field * k + ld + 1, (int)ld}; };
@@ -428,7 +458,7 @@ cudaError_t block_bottom_build(BlockBottom* b, const Geo& g, const BCd& bc, int 
             step(launch_apply(at(k), phi, rhs, g, bc, 1, nx, ny, 0, 0, st));
         }
         if (err == cudaSuccess) {
-            k_bb_gather<<<B, 256, 0, st>>>(out, field, (int)ld, b->along_y, m, B, pc, nc, nl, D, A, C, e0, e1);
+            k_bb_gather<<<B, 256, 0, st>>>(out, field, (int)ld, b->along_y, m, B, sz.pc, nc, nl, D, A, C, e0, e1);
             step(cudaGetLastError());
         }
         const size_t smem = (size_t)m * (m | 1) * sizeof(double);

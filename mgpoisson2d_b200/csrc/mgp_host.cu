@@ -405,6 +405,7 @@ struct mgp_solver {
     Lv* d_shadow = nullptr; // coarse levels' shared-memory layout (offsets), or nullptr
     TinyLv* d_tiny = nullptr;       // the tiny coarse levels' dense forms, or nullptr
     double* d_tinymat = nullptr;
+    size_t tiny_bytes = 0;
     int shadow_bytes = 0;
     // MGP_FLAG_DIRECT_COARSE: level db (>= dc) is the V-cycle's bottom, solved
     // with d_ainv, its operator's inverse (transposed); db = -1 without.
@@ -578,13 +579,24 @@ int build_direct_large(mgp_solver* s, cudaStream_t st) {
     return MGP_OK;
 }
 
+// Whether the flags ask for the exact bottom of a level dc of so many cells below.
+bool block_bottom_wanted(int kind, int flags, const int* types, long cells) {
+    bool diri = false;
+    for (int k = 0; k < 4; ++k) diri = diri || types[k] == MGP_BCTYPE_DIRI;
+    return kind == MGP_KIND_MG && (flags & MGP_FLAG_DIRECT_COARSE) && (flags & MGP_FLAG_DIRECT_LARGE) && diri &&
+           cells > kDirectLargeCells;
+}
+
 // MGP_FLAG_DIRECT_LARGE on a level dc of more cells, which is then the
 // coarsest: its exact bottom by block cyclic reduction (mgp_bottom.cu), where
-// that has its memory and solves; else the reference bottom stays.  The line lies
+// that has its memory and solves; else the reference bottom stays.  Made when the
+// solver has all else it needs, so that the factors take memory from nothing the
+// solve cannot do without (GMRES's vectors are as many as without them).  The line lies
 // at kDirectLargeCells because one launch of the dense inverse (8 MB, 5 us) beats
 // the reduction there (21 us on 33 x 35) and its inversion grows with the cube.
 int build_block_bottom(mgp_solver* s, cudaStream_t st) {
     const Lv& L = s->lv[s->dc];
+    if (!block_bottom_wanted(s->kind, s->flags, s->types, (long)L.nx * L.ny)) return MGP_OK;
     if (s->dc != s->maxdepth || !block_bottom_shape(L.nx, L.ny, L.bc, &s->bb)) {
         s->bb = BlockBottom{};
         return MGP_OK;
@@ -614,9 +626,7 @@ int build_direct_coarse(mgp_solver* s, cudaStream_t st) {
     if ((s->flags & MGP_FLAG_DIRECT_LARGE) && (long)s->lv[s->dc].nx * s->lv[s->dc].ny <= kDirectLargeCells &&
         (long)s->lv[s->dc].nx * s->lv[s->dc].ny > kDirectCells)
         return build_direct_large(s, st);
-    if ((s->flags & MGP_FLAG_DIRECT_LARGE) && (long)s->lv[s->dc].nx * s->lv[s->dc].ny > kDirectLargeCells)
-        return build_block_bottom(s, st);
-    int db = -1;
+    int db = -1;   // (none where dc has more than kDirectLargeCells: it is the coarsest level)
     for (int d = s->dc; d <= s->maxdepth; ++d)
         if ((long)s->lv[d].nx * s->lv[d].ny <= kDirectCells) {
             db = d;
@@ -706,6 +716,7 @@ int build_tiny(mgp_solver* s, size_t* off, cudaStream_t st) {
         cudaGetLastError();
         return set_err(MGP_ENOMEM, "device allocation failed");
     }
+    s->tiny_bytes = total * sizeof(double) + sizeof(TinyLv) * (md + 1);
     cudaError_t e = cudaSuccess;
     for (int d = 0; d <= md && e == cudaSuccess; ++d) {
         TinyLv& T = tiny[d];
@@ -1003,6 +1014,7 @@ int solver_build(mgp_solver* s, const mgp_box* valid, const mgp_geo* geo, const 
         if (L.e2.p) sweep_maps_prepare(&s->maps[d], L.e, L.e2, L.r, L.invd, L.g, L.nx, L.ny);
     }
     if (mixed(s)) RC(build_fp32_levels(s));
+    RC(build_block_bottom(s, st));
     std::vector<int> ref(2 * (md + 1), 0);
     for (int d = 0; d < md; ++d) { ref[d] = s->refx[d]; ref[md + 1 + d] = s->refy[d]; }
     CK(cudaMemcpyAsync(s->d_lv, s->lv.data(), sizeof(Lv) * (md + 1), cudaMemcpyHostToDevice, st));
@@ -1930,8 +1942,26 @@ size_t solver_device_bytes(const mgp_solver* s) {
         const size_t n = (size_t)s->lv[s->db].nx * s->lv[s->db].ny;
         bytes += n * n * sizeof(double);
     }
-    bytes += s->bb.bytes;
+    bytes += s->tiny_bytes + s->bb.bytes;
     return bytes;
+}
+// Device bytes a solver of all levels takes at its most beside its fields for the
+// exact bottom of more than kDirectLargeCells cells; 0 where it has none.
+size_t solver_block_bottom_bytes(const mgp_box* v, const mgp_bdry* bc, int kind, int flags) {
+    if (!v || !bc || v->nx < 4 || v->ny < 4) return 0;
+    std::vector<int> refx, refy;
+    int md = 1000;
+    estimate_maxdepth(&md, v);
+    create_mgschedule(refx, refy, &md, v);
+    int nx = v->nx, ny = v->ny;
+    for (int d = 0; d < md && (long)nx * ny > kCoarseCells; ++d) {
+        nx /= refx[d];
+        ny /= refy[d];
+    }
+    if (!block_bottom_wanted(kind, flags, bc->type, (long)nx * ny)) return 0;
+    BCd b = {};
+    for (int k = 0; k < 4; ++k) b.type[k] = bc->type[k];
+    return block_bottom_peak_bytes(nx, ny, b);
 }
 // Memory the solvers' pool on the current device holds but no solver uses
 // (freed, kept for reuse; see solver_pool): free for the next solver.

@@ -440,6 +440,8 @@ struct BlockAlloc {
 };
 // Whether a level of these sides and types has such a bottom; sets its shape.
 bool block_bottom_shape(int nx, int ny, const BCd& bc, BlockBottom* b);
+// Device bytes its set-up needs at its most (the factors and the scratch beside them); 0 without such a bottom.
+size_t block_bottom_peak_bytes(int nx, int ny, const BCd& bc);
 // Factorises the level's operator (homogeneous sides) and tries it; synchronises st.
 // *ok: it solves.  Without memory or a sound factorisation *b is empty.
 cudaError_t block_bottom_build(BlockBottom* b, const Geo& g, const BCd& bc, int nx, int ny, const BlockAlloc& mem,
