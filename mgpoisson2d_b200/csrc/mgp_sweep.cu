@@ -616,12 +616,18 @@ template SweepTiles sweep_large_tiles<double>(int, int);
 // Sweeps of the next launch, of `left` still to do.  A level inside one window
 // takes all of them; a level whose tiles for 4 (2, 1) sweeps do not outnumber
 // the SMs takes that many in the small shape, since its launch lasts one CTA's
-// latency whatever it recomputes in the halo (256^2 in FP32: 2.9 us a sweep at
-// 4, 3.5 at 2, 5.0 at 1; 512^2, where 4 and 2 need a second round: 7.6, 6.1 and
-// 5.7).  A larger one takes one in the large shape (1024^2: 13.5 us against
-// 14.1 for two a launch, 2048^2: 38 against 49).  A caller's arrays, without
-// descriptors, stay with the small shape.  A periodic side's ghosts come from
-// global memory as they stand at the start of the launch, so it takes one.
+// latency whatever it recomputes in the halo (256^2 in FP32: 2.3 us a sweep at
+// 4, 3.0 at 2, 4.6 at 1; 512^2, where 4 and 2 need a second round: 7.0, 5.6 and
+// 5.8).  A larger one takes one in the large shape (1024^2 in FP32: 13.0 us against
+// 13.5 for two a launch, 2048^2: 36.7 against 48.1).  A caller's arrays (FP64), without
+// descriptors, stay with the small shape, two sweeps a launch up to six rounds of
+// its tiles: a pair shares one read of the operands, but a window of 32 x 48 holds
+// 14 x 28 cells of a pair's tile and 22 x 36 of a single sweep's, so with many
+// rounds the pair sweeps twice as many windows (us a sweep, pairs / singles, by the
+// pairs' rounds: 384^2 at 2.6 9.3 / 11.5, 512^2 at 4.8 14.4 / 14.4, 577^2 at 6.0
+// 17.5 / 18.4, 640^2 at 7.1 19.5 / 18.5, 1024^2 at 18.5 45 / 39, 2048^2 at 74
+// 166 / 139).  A periodic side's ghosts come from global memory as they stand at
+// the start of the launch, so it takes one.
 template <class T>
 SweepPlan sweep_plan(int nx, int ny, const BCd& b, int left, const LevelMaps* maps) {
     using S = typename Shapes<T>::Small;
@@ -634,7 +640,9 @@ SweepPlan sweep_plan(int nx, int ny, const BCd& b, int left, const LevelMaps* ma
         if ((long)p.gx * p.gy <= sm_count()) return p;
     }
     if (maps && maps->ok) return SweepPlan{1, 0, 0, false};
-    return tiles_of<S>(nx, ny, periodic || left < 2 || S::ty(2) < 12 ? 1 : 2);
+    const SweepPlan two = tiles_of<S>(nx, ny, 2);
+    const bool pair = !periodic && left >= 2 && S::ty(2) >= 12 && (long)two.gx * two.gy <= 6L * sm_count();
+    return pair ? two : tiles_of<S>(nx, ny, 1);
 }
 
 template <class T>
