@@ -48,9 +48,8 @@ __device__ __forceinline__ double row_sum(double s) {
 // One step down: the lines that stay take up their eliminated neighbours,
 // r_p -= F r_l + G r_r.  item: line, eliminated neighbours (-1: none), F's index.
 // The factors do not depend on the step ahead: they are read before the wait.
-__global__ void __launch_bounds__(kRowThreads) k_bb_down(BlockBottom b, DF r, int first, const int4* __restrict__ items) {
-    const int lane = threadIdx.x & 31, row = blockIdx.x * kRowsPerCta + (threadIdx.x >> 5), m = b.m;
-    const int4 it = __ldg(items + blockIdx.y);
+__device__ __forceinline__ void step_down(const BlockBottom& b, const DF& r, int first, int4 it, int row) {
+    const int lane = threadIdx.x & 31, m = b.m;
     const double* F = b.fg + ((long)it.w * m + row) * m;
     double f[kVec], g[kVec];
     const bool here = row < m;
@@ -68,10 +67,8 @@ __global__ void __launch_bounds__(kRowThreads) k_bb_down(BlockBottom b, DF r, in
 }
 
 // One step up: the eliminated lines from their neighbours, x_p = D^-1 r_p - P x_l - Q x_r.
-__global__ void __launch_bounds__(kRowThreads) k_bb_up(BlockBottom b, DF e, DF r, int first,
-                                                       const int4* __restrict__ items) {
-    const int lane = threadIdx.x & 31, row = blockIdx.x * kRowsPerCta + (threadIdx.x >> 5), m = b.m;
-    const int4 it = __ldg(items + blockIdx.y);
+__device__ __forceinline__ void step_up(const BlockBottom& b, const DF& e, const DF& r, int first, int4 it, int row) {
+    const int lane = threadIdx.x & 31, m = b.m;
     const long o = ((long)it.x * m + row) * m;
     double d[kVec], p[kVec], q[kVec];
     const bool here = row < m;
@@ -89,6 +86,34 @@ __global__ void __launch_bounds__(kRowThreads) k_bb_up(BlockBottom b, DF e, DF r
     s = row_dot(s, q, e.p + it.z * el, ec, it.z >= 0, m, lane);
     const double x = row_sum(t - s);
     if (lane == 0) e.p[it.x * el + row * ec] = x;
+}
+
+__global__ void __launch_bounds__(kRowThreads) k_bb_down(BlockBottom b, DF r, int first, const int4* __restrict__ items) {
+    step_down(b, r, first, __ldg(items + blockIdx.y), blockIdx.x * kRowsPerCta + (threadIdx.x >> 5));
+}
+__global__ void __launch_bounds__(kRowThreads) k_bb_up(BlockBottom b, DF e, DF r, int first,
+                                                       const int4* __restrict__ items) {
+    step_up(b, e, r, first, __ldg(items + blockIdx.y), blockIdx.x * kRowsPerCta + (threadIdx.x >> 5));
+}
+
+// Step l of many problems (lockstep batches): job k owns blocks [pre[k], pre[k + 1]),
+// none where its reduction has fewer steps.  The factors and the tables do not
+// depend on the launch ahead.
+template <bool kUp>
+__global__ void __launch_bounds__(kRowThreads) k_bb_jobs(const BlockJob* __restrict__ jobs, const int* __restrict__ pre,
+                                                         int njobs, int l) {
+    int lo = 0, hi = njobs - 1;
+    while (lo < hi) {   // the last job with pre[job] <= the block
+        const int mid = (lo + hi + 1) >> 1;
+        if (__ldg(pre + mid) <= (int)blockIdx.x) lo = mid;
+        else hi = mid - 1;
+    }
+    const BlockJob& J = jobs[lo];
+    const int rows = (J.b.m + kRowsPerCta - 1) / kRowsPerCta, q = blockIdx.x - __ldg(pre + lo);
+    const int4 it = __ldg(J.b.items + (kUp ? J.b.oup[l] : J.b.odown[l]) + q / rows);
+    const int row = (q % rows) * kRowsPerCta + (threadIdx.x >> 5);
+    if (kUp) step_up(J.b, J.e, J.r, l == 0, it, row);
+    else step_down(J.b, J.r, l == 0, it, row);
 }
 
 template <class... KArgs, class... Args>
@@ -366,6 +391,18 @@ cudaError_t launch_block_bottom(const BlockBottom& b, const DF& e, const DF& r, 
     for (int l = b.steps; l >= 0 && err == cudaSuccess; --l)
         err = launch_step(k_bb_up, dim3(rows, b.nup[l]), st, b, e, r, (int)(l == 0), b.items + b.oup[l]);
     return err;
+}
+
+int block_bottom_blocks(const BlockBottom& b, int l, bool up) {
+    const int rows = (b.m + kRowsPerCta - 1) / kRowsPerCta;
+    return up ? (l <= b.steps ? rows * b.nup[l] : 0) : (l < b.steps ? rows * b.ndown[l] : 0);
+}
+
+cudaError_t launch_block_jobs(const BlockJob* jobs, const int* pre, int njobs, int nblocks, int l, bool up,
+                              cudaStream_t st) {
+    if (njobs < 1 || nblocks < 1) return cudaSuccess;
+    return up ? launch_step(k_bb_jobs<true>, dim3(nblocks), st, jobs, pre, njobs, l)
+              : launch_step(k_bb_jobs<false>, dim3(nblocks), st, jobs, pre, njobs, l);
 }
 
 cudaError_t block_bottom_build(BlockBottom* b, const Geo& g, const BCd& bc, int nx, int ny, const BlockAlloc& mem,

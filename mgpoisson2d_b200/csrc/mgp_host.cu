@@ -2036,6 +2036,49 @@ struct Table {
     }
 };
 
+// The problems whose bottom is solved by block cyclic reduction: their jobs, and
+// for each step down and up the blocks of every problem in it.
+struct BlockTable {
+    std::vector<BlockJob> jobs;
+    std::vector<std::vector<int>> pre[2];   // [up][step]
+    size_t oj = 0;
+    std::vector<size_t> op[2];
+    const BlockJob* dj = nullptr;
+    std::vector<const int*> dp[2];
+    void push(const BlockJob& j) {
+        for (int up = 0; up < 2; ++up) {
+            while ((int)pre[up].size() < j.b.steps + up) pre[up].emplace_back(jobs.size() + 1, 0);
+            for (size_t l = 0; l < pre[up].size(); ++l)
+                pre[up][l].push_back(pre[up][l].back() + block_bottom_blocks(j.b, (int)l, up != 0));
+        }
+        jobs.push_back(j);
+    }
+    void pack(Packer& pk) {
+        oj = pk.add(jobs.data(), jobs.size() * sizeof(BlockJob));
+        for (int up = 0; up < 2; ++up) {
+            op[up].clear();
+            for (const auto& p : pre[up]) op[up].push_back(pk.add(p.data(), p.size() * sizeof(int)));
+        }
+    }
+    void bind(char* base) {
+        dj = reinterpret_cast<const BlockJob*>(base + oj);
+        for (int up = 0; up < 2; ++up) {
+            dp[up].clear();
+            for (size_t o : op[up]) dp[up].push_back(reinterpret_cast<const int*>(base + o));
+        }
+    }
+    cudaError_t launch(cudaStream_t st) const {
+        cudaError_t e = cudaSuccess;
+        const auto step = [&](int l, int up) {
+            if (e == cudaSuccess)
+                e = launch_block_jobs(dj, dp[up][l], (int)jobs.size(), pre[up][l].back(), l, up != 0, st);
+        };
+        for (int l = 0; l < (int)pre[0].size(); ++l) step(l, 0);
+        for (int l = (int)pre[1].size() - 1; l >= 0; --l) step(l, 1);
+        return e;
+    }
+};
+
 int cdiv(long a, long b) { return (int)((a + b - 1) / b); }
 
 bool fill_one_phase(const BCd& b, int do_neum) {   // no side's fill reads another side's ghosts
@@ -2132,7 +2175,7 @@ struct Plan {
     std::vector<Table<ProlongJob<float, double>>> pro3264;
     Table<CoarseJob> coarse;
     int coarse_smem = 0;
-    std::vector<mgp_solver*> block;   // problems whose bottom is solved by block cyclic reduction, in turn
+    BlockTable block;
     Table<DirectJob> direct;   // problems whose bottom is the coarse-cycle level, solved by its inverse
     Table<CellJob<float, double>> r_to32;   // mixed: level-0 rhs rounded to FP32
     Table<CellJob<float, float>> guess32;   // e = r invd on FP32 level 0
@@ -2225,7 +2268,7 @@ void build_plan(Plan& P, const std::vector<mgp_solver*>& ss, const std::vector<i
             const Lv& B = s->lv[s->dc];
             P.direct.push(DirectJob{B.e, B.r, s->d_ainv, B.nx, B.ny}, direct_apply_blocks(B.nx, B.ny));
         } else if (s->bb.mem) {
-            P.block.push_back(s);
+            P.block.push(BlockJob{s->bb, s->lv[s->dc].e, s->lv[s->dc].r});
         } else {
             CoarseJob cj;
             cj.a = coarse_args_of(s, s->dc, nd, nu, nb);
@@ -2267,7 +2310,7 @@ void for_tables(Plan& P, F f) {
     for (auto& t : P.pro64) f(t);
     for (auto& t : P.pro32) f(t);
     for (auto& t : P.pro3264) f(t);
-    f(P.coarse); f(P.direct); f(P.r_to32); f(P.guess32); f(P.guess64); f(P.e_to64); f(P.update); f(P.fill_phi); f(P.norm);
+    f(P.coarse); f(P.direct); f(P.block); f(P.r_to32); f(P.guess32); f(P.guess64); f(P.e_to64); f(P.update); f(P.fill_phi); f(P.norm);
 }
 
 int upload_plan(Plan& P, Lockstep* ls, cudaStream_t st) {
@@ -2339,7 +2382,7 @@ int lockstep_iteration(Plan& P, Lockstep* ls, int nd, int nu, cudaStream_t st) {
     }
     CK(launch_coarse_jobs(P.coarse.dj, P.coarse.n(), P.coarse_smem, st));
     CK(launch_direct_jobs(P.direct.dj, P.direct.dp, P.direct.n(), P.direct.blocks(), st));
-    for (mgp_solver* s : P.block) CK(launch_block_bottom(s->bb, s->lv[s->dc].e, s->lv[s->dc].r, st));
+    CK(P.block.launch(st));
     for (int d = P.D - 1; d >= 0; --d) {   // up: fill the coarse correction, prolong, smooth (MG:818-845)
         CK(launch_fill_jobs(P.fpost64[d].dj, P.fpost64[d].dp, P.fpost64[d].n(), P.fpost64[d].blocks(), P.fpost_ph[d],
                             st));

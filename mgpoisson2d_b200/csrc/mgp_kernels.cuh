@@ -448,5 +448,15 @@ cudaError_t block_bottom_build(BlockBottom* b, const Geo& g, const BCd& bc, int 
                                cudaStream_t st, bool* ok);
 // e = A^-1 r on the level's cells (ghosts untouched).
 cudaError_t launch_block_bottom(const BlockBottom& b, const DF& e, const DF& r, cudaStream_t st);
+// The same for many levels at once (lockstep batches): the launches of the longest
+// reduction, each a step of every problem that has it, steps 0 .. down and then
+// .. 0 up, in the same bits.  Blocks of a problem in a step, and the step's launch.
+struct BlockJob {
+    BlockBottom b;
+    DF e, r;
+};
+int block_bottom_blocks(const BlockBottom& b, int l, bool up);
+cudaError_t launch_block_jobs(const BlockJob* jobs, const int* pre, int njobs, int nblocks, int l, bool up,
+                              cudaStream_t st);
 
 }  // namespace mgp
