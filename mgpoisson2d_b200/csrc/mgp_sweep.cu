@@ -254,13 +254,14 @@ __device__ __forceinline__ void sweep_stream(int total, int homog, double omega,
             load_fields(tiles[it ^ 1]);
         }
         if (any_side) {
-            with_side<C>(warp, w, L0.nx, L0.ny, [&](auto L) {
-                L.place(w, *L0.g, *L0.b, homog, L0.nx, L0.ny, om, om1);
-                L.grab(s);
-                L.put(s);
-                L.fill(s, *L0.pin, w, *L0.b, homog, L0.nx, L0.ny, 0);
-            });
-            cta_sync();
+            if (any_plain(*L0.b, homog)) {
+                with_side<C>(warp, w, L0.nx, L0.ny, [&](auto L) {
+                    L.place(w, *L0.g, *L0.b, homog, L0.nx, L0.ny, om, om1);
+                    L.grab(s);
+                    L.put(s);
+                });
+                cta_sync();
+            }
             reload<C>(k, own);
         }
         colours<C>(k, own, mask, idx, idy, om, om1);
@@ -279,7 +280,10 @@ __device__ __forceinline__ void sweep_stream(int total, int homog, double omega,
         return more ? TILE_MORE : TILE_LAST;
     };
     walk_tiles(
-        [&](int it) {   // the tile after this one, while this one's loads are in flight
+        [&](int it) {   // while this tile's loads are in flight: ghosts they do not make, and the next tile
+            const LevelRef<T>& L0 = levels[it];
+            if (warp < 4 && !tiles[it].inner)
+                start_ghosts<C>(s, tiles[it].w, *L0.pin, *L0.b, homog, L0.nx, L0.ny, warp);
             if (!issuer) return;
             NextTile& n = tiles[it ^ 1];
             n.t = tiles[it].t + gridDim.x;

@@ -98,8 +98,9 @@ struct Window {
     }
 };
 
-// phi at the start of a sweep: the window where it holds (i,j), else global
-// memory (a stored ghost, or the far side of a periodic domain).
+// phi at the start of a launch's second and later sweeps: the window where it
+// holds (i,j), else global memory (a stored ghost; a launch of several sweeps has
+// a periodic side only where one window holds the level).
 template <class C>
 struct StartLoad {
     using T = typename C::T;
@@ -232,6 +233,39 @@ __device__ __forceinline__ void corner_cell(T* S, const T* q, const int* x, cons
     S[x[1] + y[1]] = om * newphi + om1 * p;
 }
 
+// Whether a side's ghosts follow from three rows of the window beside it, or stay
+// as stored (SideLane::put); the others are filled from phi as a whole.
+__device__ __forceinline__ bool side_plain(const BCd& b, int homog, int sd) {
+    for (int s = 0; s < 4; ++s)
+        if (b.type[s] == T_PERIODIC) return false;
+    return b.type[sd] == T_NEUM || (b.type[sd] == T_DIRI && homog && b.mode[sd] != M_LAH);
+}
+__device__ __forceinline__ bool any_plain(const BCd& b, int homog) {
+    bool p = false;
+    for (int s = 0; s < 4; ++s) p = p || side_plain(b, homog, s);
+    return p;
+}
+
+// The first sweep's ghosts of a side that is not plain, by the warp of side v (0-3:
+// y low, y high, x low, x high), read from pin beside the window's own loads.  (Read
+// after them, the far side of a periodic domain was a second round trip to memory and
+// a barrier: a sweep of 132 x 140 doubly periodic cells 5.2 -> 4.2 us in FP64, of
+// 264 x 280 with one periodic direction 5.5 -> 4.6, of 1024^2 22.2 -> 20.9.)
+template <class C, class T>
+__device__ __forceinline__ void start_ghosts(T* S, const Window& w, const DFT<T>& pin, const BCd& b, int homog, int nx,
+                                             int ny, int v) {
+    const bool yside = v < 2, high = v & 1;
+    const bool on = v == 0 ? w.yl : v == 1 ? w.yh : v == 2 ? w.xl : w.xh;
+    if (!on || side_plain(b, homog, (yside ? S_YLO : S_XLO) + (high ? 1 : 0))) return;
+    const DFLoadT<T> P{pin};
+    const int lo = yside ? (w.xl ? -1 : w.ox) : w.oy, hi = yside ? (w.xh ? nx + 1 : w.wx1) : w.wy1;
+    const int side = high ? (yside ? ny : nx) : -1;
+    for (int q = lo + (threadIdx.x & 31); q < hi; q += 32) {
+        const int i = yside ? q : side, j = yside ? side : q;
+        S[x_term<C>(i - w.ox) + y_term<C>(j - w.oy)] = sweep_ghost(P, b, homog, nx, ny, i, j);
+    }
+}
+
 // What a lane keeps of its side (kY: a y side; kHigh: at the high end, in an odd
 // row or column of the window if kOdd).  With the side's parity known, the plane
 // places of the sixteen cells a lane reads are constants from one address and the
@@ -279,8 +313,7 @@ struct SideLane {
         on = kY ? (kHigh ? w.yh : w.yl) : (kHigh ? w.xh : w.xl);
         const Per pr = periodic_of(b);
         const bool periodic = kY ? (kHigh ? pr.yh : pr.yl) : (kHigh ? pr.xh : pr.xl);
-        plain = !(pr.xl || pr.xh || pr.yl || pr.yh) &&
-                (b.type[sd] == T_NEUM || (b.type[sd] == T_DIRI && homog && b.mode[sd] != M_LAH));
+        plain = side_plain(b, homog, sd);
         neum = b.type[sd] == T_NEUM;
         const int ot = kY ? w.ox : w.oy, et = kY ? w.wx1 : w.wy1, nt = kY ? nx : ny;
         const int m = kHigh ? ((kY ? ny - w.oy : nx - w.ox) - 1) >> 1 : 0;   // the side's block, 0 at the low end
@@ -292,10 +325,9 @@ struct SideLane {
             ok[c] = in[c] && !periodic && t >= lo && t < hi;
         }
         base = C::P + 1 + (kY ? lane + m * C::P : lane * C::P + m);
-        all_plain = !(pr.xl || pr.xh || pr.yl || pr.yh);
+        all_plain = true;
 #pragma unroll
-        for (int s = 0; s < 4; ++s)
-            all_plain = all_plain && (b.type[s] == T_NEUM || (b.type[s] == T_DIRI && homog && b.mode[s] != M_LAH));
+        for (int s = 0; s < 4; ++s) all_plain = all_plain && side_plain(b, homog, s);
         corner = lane == 0 && (hx ? w.xh && !pr.xh : w.xl && !pr.xl) && (hy ? w.yh && !pr.yh : w.yl && !pr.yl);
 #pragma unroll
         for (int r = 0; r < 4; ++r)   // the direction along the side: the other sides' terms
@@ -350,7 +382,8 @@ struct SideLane {
     // start.  Where they follow from three rows, grab reads these before the interior
     // colours change them (and may do so before the corners, whose values put reads
     // again) and put writes the ghosts beside the colours, since only the sides' cells
-    // read them.  Otherwise fill, between barriers.
+    // read them.  Otherwise start_ghosts and, from the second sweep of a launch on,
+    // fill, between barriers.
     __device__ __forceinline__ void grab(const T* S) {
         if (!plain || neum) return;   // a Neumann side's stay as stored
 #pragma unroll
@@ -370,8 +403,8 @@ struct SideLane {
         }
     }
     __device__ __forceinline__ void fill(T* S, const DFT<T>& pin, const Window& w, const BCd& b, int homog, int nx,
-                                         int ny, int sw) const {
-        if (!on || plain || (sw > 0 && neum)) return;
+                                         int ny) const {
+        if (!on || plain || neum) return;
         const StartLoad<C> P{S, w, pin};
         const int lo = kY ? (w.xl ? -1 : w.ox) : w.oy, hi = kY ? (w.xh ? nx + 1 : w.wx1) : w.wy1;
         const int side = kHigh ? (kY ? ny : nx) : -1;
@@ -456,7 +489,7 @@ __device__ __forceinline__ void with_side(int v, const Window& w, int nx, int ny
 }
 
 // Ghosts no sweep changes, by warps 0-3: a Neumann side's, as stored, and the
-// corners' marker.
+// corners' marker (with a periodic side they are start_ghosts' instead).
 template <class C, class T>
 __device__ __forceinline__ void fixed_ghosts(T* s, const Window& w, const DFT<T>& pin, const BCd& b, int nx, int ny) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -476,7 +509,8 @@ __device__ __forceinline__ void fixed_ghosts(T* s, const Window& w, const DFT<T>
             }
         }
     }
-    if (on && yside && lane < 2 && (lane ? w.xh : w.xl))
+    const bool periodic = b.type[S_XLO] == T_PERIODIC || b.type[S_YLO] == T_PERIODIC;
+    if (on && yside && !periodic && lane < 2 && (lane ? w.xh : w.xl))
         s[x_term<C>(lane ? nx - w.ox : -1) + y_term<C>(gt)] = bogus<T>();
 }
 
@@ -626,18 +660,21 @@ __device__ __forceinline__ void sweep_window(T* s, T* strips, const DFT<T>& pin,
     Window w;
     w.set(2 * (bx * hx / gx), min(nx, 2 * ((bx + 1) * hx / gx)), 2 * (by * hy / gy), min(ny, 2 * ((by + 1) * hy / gy)),
           4 * K + 2, 4 * K, 4 * K + 2, 4 * K + 2, nx, ny);
-    const bool any_side = w.any();
+    const bool any_side = w.any(), grabs = any_side && any_plain(b, homog);
     const T idx = T(g.idx), idy = T(g.idy), om = T(omega), om1 = T(1.0 - omega);
     if (warp >= C::NI) {   // the counterpart of the blocks' loop below, with the same CTA barriers
         with_side<C>(warp - C::NI, w, nx, ny, [&](auto L) {
             L.place(w, g, b, homog, nx, ny, om, om1);
-            cta_sync();   // phi and the strips are in place
-            if (any_side) {
-                L.grab(s);
-                L.fill(s, pin, w, b, homog, nx, ny, 0);
-                cta_sync();
-                L.take(strips, w, b, homog);
+            if (any_side && !L.all_plain) {
+                if (!kHeld) grid_dependency_wait();
+                start_ghosts<C>(s, w, pin, b, homog, nx, ny, warp - C::NI);
             }
+            cta_sync();   // phi, the strips and these ghosts are in place
+            if (grabs) {
+                L.grab(s);
+                cta_sync();
+            }
+            if (any_side) L.take(strips, w, b, homog);
 #pragma unroll 1
             for (int sw = 0; sw < K; ++sw) {
                 if (any_side) L.put(s);
@@ -646,7 +683,7 @@ __device__ __forceinline__ void sweep_window(T* s, T* strips, const DFT<T>& pin,
                 L.pass(s, strips, w, g, b, homog, nx, ny);
                 if (sw + 1 < K && !L.all_plain) {
                     boundary_sync();
-                    L.fill(s, pin, w, b, homog, nx, ny, sw + 1);
+                    L.fill(s, pin, w, b, homog, nx, ny);
                 }
                 cta_sync();
             }
@@ -701,7 +738,7 @@ __device__ __forceinline__ void sweep_window(T* s, T* strips, const DFT<T>& pin,
     }
     const unsigned mask = settle<C, false>(k, s, strips, w, kbx, kby, idx, idy, om, b, nx, ny);
     cta_sync();
-    if (any_side) cta_sync();   // 2. the sides' warps have read what the first sweep's ghosts are made of
+    if (grabs) cta_sync();   // 2. the sides' warps have read what the first sweep's ghosts are made of
 #pragma unroll 1
     for (int sw = 0; sw < K; ++sw) {
         // the boundary pass of the sweep before changed cells their owners hold
