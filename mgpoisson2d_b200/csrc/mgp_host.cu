@@ -405,7 +405,7 @@ struct mgp_solver {
     Lv* d_shadow = nullptr; // coarse levels' shared-memory layout (offsets), or nullptr
     TinyLv* d_tiny = nullptr;       // the tiny coarse levels' dense forms, or nullptr
     double* d_tinymat = nullptr;
-    size_t tiny_bytes = 0;
+    size_t tiny_bytes = 0, tiny_at = 0;   // their bytes; doubles of the staged coarse cycle ahead of their place
     int shadow_bytes = 0;
     // MGP_FLAG_DIRECT_COARSE: level db (>= dc) is the V-cycle's bottom, solved
     // with d_ainv, its operator's inverse (transposed); db = -1 without.
@@ -963,7 +963,9 @@ int solver_build(mgp_solver* s, const mgp_box* valid, const mgp_geo* geo, const 
         // take 68 us a BiCGStab iteration in shared memory (87 in global memory),
         // and a cluster's seventy-odd barriers an iteration alone cost 2 us each.
         if ((long)s->lv[md].nx * s->lv[md].ny > kHeldBottomCells) off = (size_t)kCoarseSmemMax;   // not staged
-        if (md - s->dc + 1 <= kMaxCoarseLevels && off * sizeof(double) <= (size_t)kCoarseSmemMax)
+        // (under an exact bottom on level dc no V-cycle goes below it: fmg asks for them, solver_solve)
+        s->tiny_at = off;
+        if (md - s->dc + 1 <= kMaxCoarseLevels && off * sizeof(double) <= (size_t)kCoarseSmemMax && !s->direct_large)
             RC(build_tiny(s, &off, st));
         const size_t bytes = off * sizeof(double);
         if (md - s->dc + 1 <= kMaxCoarseLevels && bytes <= (size_t)kCoarseSmemMax) {
@@ -1605,6 +1607,11 @@ int solver_solve(mgp_solver* s, int which, mgp_array* phi, mgp_array* rhs, const
     if (!bc) return set_err(MGP_EINVAL, "null bdry_data");
     for (int k = 0; k < 4; ++k)
         if (bc->type[k] != s->types[k]) return set_err(MGP_EINVAL, "BC types differ from the ones the solver was built with");
+    if (which == 1 && s->direct_large && s->shadow_bytes > 0 && !s->d_tiny) {   // fmg's first cycles lie below dc
+        size_t off = s->tiny_at;
+        RC(build_tiny(s, &off, st));
+        s->shadow_bytes = (int)(off * sizeof(double));
+    }
     BCd ubc;
     RC(make_bc(bc, &s->valid, homog, s->d_bcbuf, &ubc, st));
     Lv& L0 = s->lv[0];
