@@ -1210,16 +1210,20 @@ int vcycle32(mgp_solver* s, int d, int numcycles, int nd, int nu, int nb, bool g
                 }
                 return MGP_OK;
             }
+            // The BF16 study rounds after two sweeps where 32 x 32 tiles are at most two
+            // an SM of a B200 and no side is periodic, else after each, however many
+            // launches the sweeps take.
+            bool twice = (long)((L.nx + 31) / 32) * ((L.ny + 31) / 32) <= 296;
+            for (int k = 0; k < 4; ++k) twice = twice && F.bc.type[k] != T_PERIODIC;
+            const int most = !(b16 && d >= 1) ? nu_ : twice ? 2 : 1;
             for (int k = 0; k < nu_;) {
-                // the BF16 study rounds what a kernel writes: after two sweeps
-                // where 32 x 32 tiles are at most two an SM, else after each
-                const long t32 = (long)((L.nx + 31) / 32) * ((L.ny + 31) / 32);
-                const int left = !(b16 && d >= 1) ? nu_ - k : std::min(nu_ - k, t32 <= 296 ? 2 : 1);
-                const SweepPlan p = sweep_plan<float>(L.nx, L.ny, F.bc, left, &s->maps32[d]);
-                CK(launch_sweep9(L.e, L.e2, L.r, L.invd, L.g, F.bc, 1, L.nx, L.ny, 1.0, p, 1, &s->maps32[d],
-                                 s->d_status, st));
-                k += p.k;
-                std::swap(L.e, L.e2);
+                for (const int end = k + std::min(most, nu_ - k); k < end;) {
+                    const SweepPlan p = sweep_plan<float>(L.nx, L.ny, F.bc, end - k, &s->maps32[d]);
+                    CK(launch_sweep9(L.e, L.e2, L.r, L.invd, L.g, F.bc, 1, L.nx, L.ny, 1.0, p, 1, &s->maps32[d],
+                                     s->d_status, st));
+                    k += p.k;
+                    std::swap(L.e, L.e2);
+                }
                 CK(round16(L.e, d, L.nx, L.ny, 1));
             }
             return MGP_OK;
