@@ -1538,17 +1538,24 @@ __device__ __forceinline__ bool fusable_sides(const BCd& b) {
 // arrays in every phase: 32^2 cells, nine points, 5.5 -> 2.2 us a sweep; the cycle
 // below 32^2 (nine-point, eight sweeps a visit) 261 -> 146 us.  Bound by the
 // barriers and the latency of the chains between them.  The same operations in the
-// same order, so the same bits.
+// same order, so the same bits.  The shapes leave out few levels of less than 1400
+// cells: those whose BiCGStab's sweeps ran the general phases in this kernel's 512
+// threads took up to 7 % longer than in the 256 of a kernel without windows, since the
+// phases are chains of barriers (a V-cycle with a bottom of 33 x 33 cells 1.73 -> 1.81
+// ms, 41 x 25 1.81 -> 1.93; in a window of their own 1.37 and 1.43).
 using DdFlat64 = DdShape<double, 32>;   // 64 x 32
 using DdTall64 = DdShape<double, 16>;   // 32 x 64
+constexpr int most(int a, int b) { return a > b ? a : b; }
 union HeldWork {
     struct {
-        double planes[4 * (Small64::PS > Flat64::PS ? Small64::PS : Flat64::PS)];
+        double planes[4 * most(most(most(Small64::PS, Flat64::PS), most(Square64::PS, Wide64::PS)), Broad64::PS)];
         double strips[4 * kStrip * kAlong];
     };
     double dd[4 * (DdFlat64::PS > DdTall64::PS ? DdFlat64::PS : DdTall64::PS)];
 };
 static_assert(Small64::kThreads == kCoarseThreads && Flat64::kThreads == kCoarseThreads &&
+                  Square64::kThreads == kCoarseThreads && Broad64::kThreads == kCoarseThreads &&
+                  Wide64::kThreads == kCoarseThreads &&
                   32 * DdFlat64::NW == kCoarseThreads && 32 * DdTall64::NW == kCoarseThreads,
               "a window takes the CTA");
 template <class C>
@@ -1565,14 +1572,13 @@ __device__ void b_relax9(const Lv& L, const DF& phi, const DF& rhs, int homog, d
     if (fusable_sides(L.bc)) {
         if constexpr (!S::kGrid) {
             if (H && sweeps > 0 && nx >= 4 && ny >= 4) {
-                if (nx <= Small64::WX && ny <= Small64::WY) {
-                    held_sweeps<Small64>(*H, phi, rhs, L.invd, L.g, L.bc, homog, nx, ny, omega, sweeps);
-                    return;
-                }
-                if (nx <= Flat64::WX && ny <= Flat64::WY) {
-                    held_sweeps<Flat64>(*H, phi, rhs, L.invd, L.g, L.bc, homog, nx, ny, omega, sweeps);
-                    return;
-                }
+                const auto held = [&](auto shape) {
+                    using C = decltype(shape);
+                    if (nx > C::WX || ny > C::WY) return false;
+                    held_sweeps<C>(*H, phi, rhs, L.invd, L.g, L.bc, homog, nx, ny, omega, sweeps);
+                    return true;
+                };
+                if (held(Small64()) || held(Flat64()) || held(Square64()) || held(Broad64()) || held(Wide64())) return;
             }
         }
         for (int it = 0; it < sweeps; ++it) b_sweep9<S>(phi, rhs, L.invd, L.g, L.bc, homog, nx, ny, omega);

@@ -174,7 +174,7 @@ __device__ __forceinline__ void sweep_stream(int total, int homog, double omega,
     __shared__ __align__(8) unsigned long long barrier_word;
     extern __shared__ unsigned char stage_raw[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int kbx = lane % C::LB, kby = warp * C::RB + lane / C::LB;
+    const int kbx = tid % C::LB, kby = tid / C::LB;
     T* stage = reinterpret_cast<T*>(stage_raw + ((128 - ((unsigned)__cvta_generic_to_shared(stage_raw) & 127)) & 127));
     const unsigned sb = (unsigned)__cvta_generic_to_shared(stage), bar = (unsigned)__cvta_generic_to_shared(&barrier_word);
     T* own = s + (kby + 1) * C::P + kbx + 1;

@@ -9,18 +9,19 @@ namespace mgp {
 
 namespace {
 
-// A CTA's shape: NI warps own the window's blocks, LB blocks (2 LB columns) a
-// row, 32 / LB rows a warp; with kSep four more warps serve the domain's sides.
+// A CTA's shape: NI warps own the window's blocks, a thread a block, LB blocks (2
+// LB columns) a row (threads past the last whole row have none); with kSep four
+// more warps serve the domain's sides.
 template <class T_, int NI_, int LB_, bool kSep_, int kMinBlocks_>
 struct Shape {
     using T = T_;
     static constexpr int NI = NI_, LB = LB_, kMinBlocks = kMinBlocks_;
     static constexpr bool kSep = kSep_;
-    static constexpr int RB = 32 / LB;                       // block rows a warp
+    static constexpr int NR = 32 * NI / LB;                  // block rows
     static constexpr int kThreads = 32 * (NI + (kSep ? 4 : 0));
-    static constexpr int WX = 2 * LB, WY = 2 * NI * RB;      // window
+    static constexpr int WX = 2 * LB, WY = 2 * NR;           // window
     static constexpr int P = LB + 2;                         // blocks per plane row, one spare either side
-    static constexpr int PS = P * (NI * RB + 2);             // one plane
+    static constexpr int PS = P * (NR + 2);                  // one plane
     static_assert(WX <= 64 && WY <= 64 && NI >= 4, "a warp holds a side, two cells a lane");
     // largest tile for K sweeps a launch
     static constexpr int tx(int k) { return WX - (8 * k + 2); }
@@ -691,7 +692,8 @@ __device__ __forceinline__ void sweep_window(T* s, T* strips, const DFT<T>& pin,
         store_ghosts<C>(s, pout, w, warp - C::NI, nx, ny);
         return;
     }
-    const int kbx = lane % C::LB, kby = warp * C::RB + lane / C::LB;   // the thread's block
+    const int kbx = threadIdx.x % C::LB, kby = threadIdx.x / C::LB;   // the thread's block
+    const bool ahead = kbx == C::LB - 1 || lane == 31;                // its east neighbour is not the next lane's
     const int i0 = w.ox + 2 * kbx, j0 = w.oy + 2 * kby;
     const bool c0 = i0 < w.wx1, c1 = i0 + 1 < w.wx1;
     T* own = s + (kby + 1) * C::P + kbx + 1;
@@ -706,7 +708,7 @@ __device__ __forceinline__ void sweep_window(T* s, T* strips, const DFT<T>& pin,
         load_pair<kVec, !kHeld>(&AT(g.xx, i0, j), f0, f1, k.xx[r][0], k.xx[r][1]);
         load_pair<kVec, !kHeld>(&AT(g.xy, i0, j), f0, f1, k.xy[r][0], k.xy[r][1]);
         load_pair<kVec, !kHeld>(&AT(invd, i0, j), in && c0, in && c1, k.d[r][0], k.d[r][1]);
-        if (kbx == C::LB - 1 && in && c1) {   // the window's last face has no neighbour lane
+        if (ahead && in && c1) {
             k.xx[r][2] = kHeld ? AT(g.xx, i0 + 2, j) : __ldg(&AT(g.xx, i0 + 2, j));
             k.xy[r][2] = kHeld ? AT(g.xy, i0 + 2, j) : __ldg(&AT(g.xy, i0 + 2, j));
         }
@@ -731,7 +733,7 @@ __device__ __forceinline__ void sweep_window(T* s, T* strips, const DFT<T>& pin,
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
         const T a = __shfl_down_sync(0xffffffffu, k.xx[r][0], 1), c = __shfl_down_sync(0xffffffffu, k.xy[r][0], 1);
-        if (kbx < C::LB - 1) {
+        if (!ahead) {
             k.xx[r][2] = a;
             k.xy[r][2] = c;
         }
@@ -751,9 +753,12 @@ __device__ __forceinline__ void sweep_window(T* s, T* strips, const DFT<T>& pin,
     store_block<kVec>(k, pout, w, i0, j0);
 }
 
-// FP64 shapes of sixteen warps: windows of 32 x 48 and 64 x 24 cells.
+// FP64 shapes of sixteen warps: windows of 32 x 48, 64 x 24, 40 x 38, 48 x 32 and 52 x 28 cells.
 using Small64 = Shape<double, 12, 16, true, 1>;
 using Flat64 = Shape<double, 12, 32, true, 1>;
+using Square64 = Shape<double, 12, 20, true, 1>;
+using Broad64 = Shape<double, 12, 24, true, 1>;
+using Wide64 = Shape<double, 12, 26, true, 1>;
 
 }  // namespace
 
