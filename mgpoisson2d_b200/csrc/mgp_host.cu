@@ -3091,6 +3091,8 @@ int mgp_restrict(const mgp_box* fine_valid, const mgp_array* fine, const mgp_box
     const int rx = fine_valid->nx / crse_valid->nx, ry = fine_valid->ny / crse_valid->ny;
     if (rx < 1 || ry < 1 || rx * crse_valid->nx != fine_valid->nx || ry * crse_valid->ny != fine_valid->ny)
         return set_err(MGP_EINVAL, "restrict: boxes are not refinements of each other");
+    if ((offi != 0 && offi != 1) || (offj != 0 && offj != 1))   // an array's extents follow from them
+        return set_err(MGP_EINVAL, "restrict: offi and offj must be 0 (node) or 1 (cell)");
     const int kind = (offi == 1 && offj == 1) ? 0 : (offi == 0 && offj == 1) ? 1 : (offi == 1 && offj == 0) ? 2 : 3;
     const int fx = fine_valid->nx + (offi == 0), fy = fine_valid->ny + (offj == 0);
     const int cx = crse_valid->nx + (offi == 0), cy = crse_valid->ny + (offj == 0);
