@@ -370,19 +370,9 @@ struct DFLoadT {
 };
 using DFLoad = DFLoadT<double>;
 
-// k / d by a multiply: exact for 0 <= k < 65536 and 1 <= d <= 1024 (every
-// pair checked on the host).  The magic number costs one divide; compute it
-// off the critical path.
-__device__ __forceinline__ unsigned long long fastdiv_magic(int d) {
-    return ((1ull << 32) + (unsigned)d - 1) / (unsigned)d;
-}
-__device__ __forceinline__ int fastdiv(int k, unsigned long long m) {
-    return (int)(((unsigned long long)(unsigned)k * m) >> 32);
-}
-
-// The same with a 24-bit magic number, which one 32-bit divide makes:
-// m = ceil(2^24 / d), and floor(k * m / 2^24) = floor(k / d) whenever
-// k * (d - 1) < 2^24 (so for k < 16384 with d <= 1024, and k < 65536 with
+// k / d by a multiply with a 24-bit magic number, which one 32-bit divide makes
+// (off the critical path): m = ceil(2^24 / d), and floor(k * m / 2^24) = floor(k / d)
+// whenever k * (d - 1) < 2^24 (so for k < 16384 with d <= 1024, and k < 65536 with
 // d <= 256; both ranges checked exhaustively on the host).
 __device__ __forceinline__ unsigned fastdiv24_magic(int d) {
     return ((1u << 24) + (unsigned)d - 1u) / (unsigned)d;

@@ -3030,17 +3030,4 @@ cudaError_t launch_bicgstab(const BicgArgs& a, cudaStream_t st) {
     return cudaGetLastError();
 }
 
-__global__ void __launch_bounds__(kCoarseThreads) k_relax_block(Lv L, DF phi, DF rhs, int homog, double omega,
-                                                               int sweeps, int dd) {
-    b_relax<BlockScope>(L, phi, rhs, homog, omega, sweeps, dd);
-}
-
-cudaError_t launch_relax_block(const Lv& L, const DF& phi, const DF& rhs, int homog, double omega, int sweeps,
-                               int dd, int* status, cudaStream_t st) {
-    (void)status;
-    k_relax_block<<<1, kCoarseThreads, 0, st>>>(L, phi, rhs, homog, omega, sweeps, dd);
-    count_launch();
-    return cudaGetLastError();
-}
-
 }  // namespace mgp

@@ -131,7 +131,6 @@ cudaError_t launch_fill(const DF32& p, const Geo32& g, const BCd& b, int homog, 
                         cudaStream_t st);
 cudaError_t launch_apply(const DF32& out, const DF32& phi, const DF32& rhs, const Geo32& g, const BCd& b, int homog,
                          int nx, int ny, int mode, int jscale, cudaStream_t st);
-// Cell-centred restriction into an FP32 or an FP64 coarse field.
 // Prolongation from an FP32 or an FP64 coarse field (arithmetic in the coarse type).
 cudaError_t launch_prolong(const DF32& fine, const DF32& crse, int ncx, int ncy, int refx, int refy, int order,
                            cudaStream_t st);
@@ -384,7 +383,7 @@ cudaError_t launch_dd_sweeps(const DF& pin, const DF& pout, const DF& m, const D
                              int nx, int ny, double omega, int left, int* done, cudaStream_t st);
 cudaError_t launch_dd_sweeps(const DF32& pin, const DF32& pout, const DF32& m, const DF32& invd, const Geo32& g,
                              const BCd& b, int nx, int ny, double omega, int left, int* done, cudaStream_t st);
-// The same three on FP32 fields (the grid levels of a mixed-precision DD V-cycle).
+// modrhs and colour on FP32 fields (the grid levels of a mixed-precision DD V-cycle).
 cudaError_t launch_dd_modrhs(const DF32& out, const DF32& phi, const DF32& rhs, const Geo32& g, int nx, int ny,
                              cudaStream_t st);
 cudaError_t launch_dd_colour(const DF32& phi, const DF32& modrhs, const DF32& invd, const Geo32& g, int nx, int ny,
@@ -417,8 +416,6 @@ cudaError_t launch_invert(const double* A, int n, double* ainv, double* work, in
 // numbered i fastest), one warp per row.
 cudaError_t launch_direct_apply(const DF& e, const DF& r, const double* ainv, int nx, int ny, cudaStream_t st);
 cudaError_t launch_bicgstab(const BicgArgs& a, cudaStream_t st);
-cudaError_t launch_relax_block(const Lv& L, const DF& phi, const DF& rhs, int homog, double omega, int sweeps,
-                               int dd, int* status, cudaStream_t st);
 
 // The exact bottom of a level of more than kDirectLargeCells cells (mgp_bottom.cu):
 // block cyclic reduction over its lines of m cells.

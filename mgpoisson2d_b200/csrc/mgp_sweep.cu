@@ -20,8 +20,8 @@
 //
 // The operator lives in registers.  A thread owns a 2 x 2 block of cells -- one
 // of each colour -- and keeps their face coefficients, inverse diagonals and
-// right-hand sides (36 values) through all K sweeps.  Shared memory holds phi
-// alone, as four planes, one per colour (i mod 2, j mod 2), so a colour pass
+// right-hand sides (32 values, 36 with phi) through all K sweeps.  Shared memory holds
+// phi alone, as four planes, one per colour (i mod 2, j mod 2), so a colour pass
 // reads its five neighbours outside the block with consecutive lanes on
 // consecutive words.  (With the whole operator in shared memory at one word a
 // cell, a colour reads 19 values an update at stride two: 640 of the ~900
