@@ -2184,7 +2184,7 @@ struct Plan {
     std::vector<Table<ProlongJob<double, double>>> pro64;
     std::vector<Table<ProlongJob<float, float>>> pro32;
     std::vector<Table<ProlongJob<float, double>>> pro3264;
-    Table<CoarseJob> coarse;
+    Table<CoarseJob> coarse, plain;   // plain: a bottom of at most kPlainCells cells in global memory
     int coarse_smem = 0;
     BlockTable block;
     Table<DirectJob> direct;   // problems whose bottom is the coarse-cycle level, solved by its inverse
@@ -2283,7 +2283,9 @@ void build_plan(Plan& P, const std::vector<mgp_solver*>& ss, const std::vector<i
         } else {
             CoarseJob cj;
             cj.a = coarse_args_of(s, s->dc, nd, nu, nb);
-            P.coarse.push(cj, 1);
+            const Lv& B = s->lv[s->dc];
+            const bool plain = !s->d_shadow && s->dc == s->maxdepth && !s->d_ainv && B.nx * B.ny <= kPlainCells;
+            (plain ? P.plain : P.coarse).push(cj, 1);
             if (s->d_shadow) P.coarse_smem = std::max(P.coarse_smem, s->shadow_bytes);
         }
         const Lv& L0 = s->lv[0];
@@ -2321,7 +2323,7 @@ void for_tables(Plan& P, F f) {
     for (auto& t : P.pro64) f(t);
     for (auto& t : P.pro32) f(t);
     for (auto& t : P.pro3264) f(t);
-    f(P.coarse); f(P.direct); f(P.block); f(P.r_to32); f(P.guess32); f(P.guess64); f(P.e_to64); f(P.update); f(P.fill_phi); f(P.norm);
+    f(P.coarse); f(P.plain); f(P.direct); f(P.block); f(P.r_to32); f(P.guess32); f(P.guess64); f(P.e_to64); f(P.update); f(P.fill_phi); f(P.norm);
 }
 
 int upload_plan(Plan& P, Lockstep* ls, cudaStream_t st) {
@@ -2391,7 +2393,7 @@ int lockstep_iteration(Plan& P, Lockstep* ls, int nd, int nu, cudaStream_t st) {
         CK(launch_resid_jobs(P.res32[d].dj, P.res32[d].dp, P.res32[d].n(), P.res32[d].blocks(), st));
         CK(launch_resid_jobs(P.res3264[d].dj, P.res3264[d].dp, P.res3264[d].n(), P.res3264[d].blocks(), st));
     }
-    CK(launch_coarse_jobs(P.coarse.dj, P.coarse.n(), P.coarse_smem, st));
+    CK(launch_coarse_jobs(P.coarse.dj, P.coarse.n(), P.coarse_smem, P.plain.dj, P.plain.n(), st));
     CK(launch_direct_jobs(P.direct.dj, P.direct.dp, P.direct.n(), P.direct.blocks(), st));
     CK(P.block.launch(st));
     for (int d = P.D - 1; d >= 0; --d) {   // up: fill the coarse correction, prolong, smooth (MG:818-845)

@@ -481,6 +481,7 @@ __device__ void grid_barrier() {
 // per-thread partial sums (RLOOP).
 struct BlockScope {
     static constexpr bool kGrid = false;
+    static constexpr bool kWhole = true;   // has the threads that the windows of held levels take
     static constexpr bool kCluster = false;
     __device__ static int rank() { return threadIdx.x; }
     __device__ static int size() { return blockDim.x; }
@@ -489,10 +490,26 @@ struct BlockScope {
     __device__ static int rsize() { return kReduceThreads; }
     __device__ static bool ractive() { return threadIdx.x < kReduceThreads; }
 };
+// BlockScope in a kernel of kReduceThreads threads, which may have twice the
+// registers each: the general phases of small levels (k_bicgstab_plain,
+// k_coarse_jobs_plain).  A scope of its own, so that its routines are compiled for those
+// registers.
+struct PlainScope {
+    static constexpr bool kGrid = false;
+    static constexpr bool kWhole = false;
+    static constexpr bool kCluster = false;
+    __device__ static int rank() { return threadIdx.x; }
+    __device__ static int size() { return kReduceThreads; }
+    __device__ static void sync() { __syncthreads(); }
+    __device__ static int rrank() { return threadIdx.x; }
+    __device__ static int rsize() { return kReduceThreads; }
+    __device__ static bool ractive() { return true; }
+};
 struct GridScope {
     __device__ static int cta() { return blockIdx.x; }
     __device__ static int ncta() { return gridDim.x; }
     static constexpr bool kGrid = true;
+    static constexpr bool kWhole = false;
     static constexpr bool kCluster = false;
     __device__ static int rank() { return blockIdx.x * blockDim.x + threadIdx.x; }
     __device__ static int size() { return gridDim.x * blockDim.x; }
@@ -525,6 +542,7 @@ __device__ __forceinline__ void cluster_barrier() {
 template <bool kOrdered>
 struct ClusterScope {
     static constexpr bool kGrid = true;
+    static constexpr bool kWhole = false;
     static constexpr bool kCluster = kOrdered;
     __device__ static int cta() {
         unsigned r;
@@ -1570,7 +1588,7 @@ __device__ void b_relax9(const Lv& L, const DF& phi, const DF& rhs, int homog, d
                          HeldWork* H = nullptr) {
     const int nx = L.nx, ny = L.ny;
     if (fusable_sides(L.bc)) {
-        if constexpr (!S::kGrid) {
+        if constexpr (S::kWhole) {
             if (H && sweeps > 0 && nx >= 4 && ny >= 4) {
                 const auto held = [&](auto shape) {
                     using C = decltype(shape);
@@ -1626,7 +1644,7 @@ __device__ __noinline__ void held_dd_sweeps(HeldWork& H, const DF& phi, const Lv
 template <class S>
 __device__ void b_dd_sweeps(const Lv& L, const DF& phi, int homog, double omega, int sweeps, HeldWork* H) {
     const int nx = L.nx, ny = L.ny;
-    if constexpr (!S::kGrid) {
+    if constexpr (S::kWhole) {
         bool lah = true;   // the ghosts dd_window knows
         for (int s = 0; s < 4; ++s)
             lah = lah && (L.bc.type[s] == T_DIRI || L.bc.type[s] == T_NEUM) && L.bc.mode[s] == M_LAH;
@@ -2426,9 +2444,33 @@ __global__ void __launch_bounds__(kCoarseThreads, 1) k_coarse_jobs(const CoarseJ
         const int s = coarse_body<BlockScope>(a.lv, a, sh, nullptr, nullptr, &work.held);
         if (threadIdx.x == 0) set_status(a.status, s);
     }
+    pdl_wait();   // for the plain jobs, which this kernel runs beside
 }
 
-cudaError_t launch_coarse_jobs(const CoarseJob* jobs, int njobs, int smem_bytes, cudaStream_t st) {
+// The bottoms among them that no CTA stages and no window holds, of at most
+// kPlainCells cells: coarse cycles of that level alone.  Their phases are chains of
+// barriers and loads in which 512 threads help less than the registers they halve cost
+// (128 with spills against 214): two V-cycles of a bottom of 51 x 53 cells 10.9 -> 9.9
+// ms, 61 x 45 10.6 -> 9.9, 61 x 61 14.6 either way, 65 x 65 21.3 here against 20.5.
+__global__ void __launch_bounds__(kReduceThreads, 1) k_coarse_jobs_plain(const CoarseJob* __restrict__ jobs) {
+    __shared__ double sh[64];
+    pdl_allow();
+    const CoarseArgs& a = jobs[blockIdx.x].a;
+    const Lv& L = a.lv[a.d0];
+    if (a.dd) b_set_guess<PlainScope>(L);
+    b_relax<PlainScope>(L, L.e, L.r, 1, a.dd ? 4.0 / 5.0 : 1.0, a.nb, a.dd);
+    const int s = b_bicgstab<PlainScope>(L, L.e, L.r, 1, 1.0e-6, 80, 5, 0, a.dd, sh);
+    if (threadIdx.x == 0) set_status(a.status, s);
+}
+
+cudaError_t launch_coarse_jobs(const CoarseJob* jobs, int njobs, int smem_bytes, const CoarseJob* plain, int nplain,
+                               cudaStream_t st) {
+    if (nplain > 0) {
+        k_coarse_jobs_plain<<<nplain, kReduceThreads, 0, st>>>(plain);
+        count_launch();
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
+    }
     if (njobs < 1) return cudaSuccess;
     static std::mutex mu;
     static unsigned long long done = 0;
@@ -2443,8 +2485,10 @@ cudaError_t launch_coarse_jobs(const CoarseJob* jobs, int njobs, int smem_bytes,
             if (dev < 64) done |= 1ull << dev;
         }
     }
-    k_coarse_jobs<<<njobs, kCoarseThreads, smem_bytes, st>>>(jobs);
     count_launch();
+    // (what both read was complete when the plain jobs' kernel began)
+    if (nplain > 0) return launch_dep(k_coarse_jobs, dim3(njobs), dim3(kCoarseThreads), smem_bytes, st, jobs);
+    k_coarse_jobs<<<njobs, kCoarseThreads, smem_bytes, st>>>(jobs);
     return cudaGetLastError();
 }
 
@@ -3024,8 +3068,27 @@ __global__ void __launch_bounds__(kCoarseThreads, 1) k_bicgstab(BicgArgs a) {
     if (threadIdx.x == 0) set_status(a.status, s);
 }
 
+__global__ void __launch_bounds__(kReduceThreads, 1) k_bicgstab_plain(BicgArgs a) {
+    __shared__ double sh[64];
+    const int s = b_bicgstab<PlainScope>(a.L, a.phi, a.rhs, a.homog, a.tol, a.max_iters, a.max_restarts, a.zerophi,
+                                         a.dd, sh);
+    if (threadIdx.x == 0) set_status(a.status, s);
+}
+
+// The windows pay off in a BiCGStab of more than 64 cells without periodic sides, whose
+// ghosts cost them two more barriers a sweep (six iterations, windows / plain, us: 16 x
+// 16 periodic 274 / 212, 31 x 31 318 / 294, 8 x 8 264 / 256; 20 x 20 Dirichlet 257 /
+// 266); without them 512 threads do above kPlainCells
+// (45 x 45 567 / 507).
 cudaError_t launch_bicgstab(const BicgArgs& a, cudaStream_t st) {
-    k_bicgstab<<<1, kCoarseThreads, 0, st>>>(a);
+    const int nx = a.L.nx, ny = a.L.ny;
+    bool periodic = false;
+    for (int s = 0; s < 4; ++s) periodic = periodic || a.L.bc.type[s] == T_PERIODIC;
+    const auto fits = [&](auto shape) { return nx <= decltype(shape)::WX && ny <= decltype(shape)::WY; };
+    const bool window = !periodic && nx * ny > 64 &&
+                        (fits(Small64()) || fits(Flat64()) || fits(Square64()) || fits(Broad64()) || fits(Wide64()));
+    if (window || nx * ny > kPlainCells) k_bicgstab<<<1, kCoarseThreads, 0, st>>>(a);
+    else k_bicgstab_plain<<<1, kReduceThreads, 0, st>>>(a);
     count_launch();
     return cudaGetLastError();
 }

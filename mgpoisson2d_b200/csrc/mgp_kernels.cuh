@@ -115,6 +115,7 @@ struct BicgArgs {
 constexpr int kCoarseThreads = 512;   // of the one-CTA coarse cycle: the shape of mgp_sweep.cuh's windows
 constexpr int kHeldBottomCells = 5 * kCoarseThreads;   // largest bottom it holds in shared memory
 constexpr int kReduceThreads = 256;   // of them that accumulate its reductions
+constexpr int kPlainCells = 3600;     // largest level whose general phases are faster in a CTA of that many (mgp_kernels.cu)
 constexpr int kGridThreads = 256;     // threads per CTA of the cooperative-grid coarse cycle
 constexpr int kClusterThreads = 256;   // threads per CTA of the cluster coarse cycle
 
@@ -315,7 +316,8 @@ cudaError_t launch_cell_jobs(const CellJob<TD, TS>* jobs, const int* pre, int nj
 // r = rhs - L[phi], then norms[k] = sqrt(vol_k * sum of job k's r^2) in block order (vol in volk).
 cudaError_t launch_norm_jobs(const NormJob* jobs, const int* pre, int njobs, int nblocks, double* partials,
                              const double* volk, double* norms, cudaStream_t st);
-cudaError_t launch_coarse_jobs(const CoarseJob* jobs, int njobs, int smem_bytes, cudaStream_t st);
+cudaError_t launch_coarse_jobs(const CoarseJob* jobs, int njobs, int smem_bytes, const CoarseJob* plain, int nplain,
+                               cudaStream_t st);
 int direct_apply_blocks(int nx, int ny);
 cudaError_t launch_direct_jobs(const DirectJob* jobs, const int* pre, int njobs, int nblocks, cudaStream_t st);
 cudaError_t launch_invdiag(const DF& invd, const Geo& g, const BCd& b, int homog, int nx, int ny, int coupled,
