@@ -216,7 +216,7 @@ int mgp_map_geometry(const mgp_box* valid, int map, const double* params, mgp_ge
             k_metric<<<grd, blk>>>(f, a.what, m, valid->ilo, valid->jlo, valid->dx, valid->dy, a.nvx, a.nvy, gx,
                                    gy);
             count_launch();
-            if (cudaGetLastError() != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess) {
+            if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(0) != cudaSuccess) {
                 cudaGetLastError();
                 return record_error(MGP_ECUDA, "map_geometry: kernel failed");
             }
@@ -267,7 +267,7 @@ int mgp_map_fourier_rhs(const mgp_box* valid, int map, const double* params, int
                 return record_error(MGP_ECUDA, "map_fourier_rhs: reduction failed");
             k_center_scale<<<grd, blk>>>(f, jd, out, nx, ny);
             count_launch();
-            if (cudaGetLastError() != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess) {
+            if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(0) != cudaSuccess) {
                 cudaGetLastError();
                 return record_error(MGP_ECUDA, "map_fourier_rhs: kernel failed");
             }

@@ -233,7 +233,7 @@ struct ArenaT {
         CK(cudaMemsetAsync(base, 0, elems * sizeof(T), st));   // fresh arrays start at zero
         return MGP_OK;
     }
-    void release() {   // after a device synchronisation (solver_free)
+    void release() {   // when nothing that uses it runs (solver_free)
         dfree(base, nullptr);
         base = nullptr;
         specs.clear();
@@ -470,12 +470,22 @@ namespace {
 
 constexpr int kRedSlots = 2 * kRedBlocksMax + 8;   // two partials per reduction block, then the outputs
 
+// On every way out of a call, its stream is idle: a solver's memory may go back to
+// the pool after any call on it.  (Waiting for the device when a solver is freed
+// instead breaks a stream capture that another thread has under way, as every
+// solver's first V-cycle does.)
+struct Quiesce {
+    cudaStream_t st;
+    bool idle = false;
+    ~Quiesce() {
+        if (!idle) cudaStreamSynchronize(st);
+    }
+};
+
+// Nothing of the solver's runs (Quiesce); its stream may already be gone: a server
+// worker's, say.
 void solver_free(mgp_solver* s) {
     if (!s) return;
-    // nothing of the solver's may still run when its memory goes back to the
-    // pool (its stream may already be gone: a server worker's, say), as
-    // cudaFree would have waited for the device
-    cudaDeviceSynchronize();
     for (void* p : {(void*)s->d_lv, (void*)s->d_shadow, (void*)s->d_tiny, (void*)s->d_tinymat, (void*)s->d_ainv, (void*)s->bb.mem, (void*)s->bb.items, (void*)s->gm_base, (void*)s->gm_red,
                     (void*)s->gctl.bar, (void*)s->gctl.part, (void*)s->d_ref, (void*)s->d_status,
                     (void*)s->d_bcbuf, (void*)s->d_red})
@@ -1611,6 +1621,7 @@ int solver_solve(mgp_solver* s, int which, mgp_array* phi, mgp_array* rhs, const
     if (!bc) return set_err(MGP_EINVAL, "null bdry_data");
     for (int k = 0; k < 4; ++k)
         if (bc->type[k] != s->types[k]) return set_err(MGP_EINVAL, "BC types differ from the ones the solver was built with");
+    Quiesce q{st};
     if (which == 1 && s->direct_large && s->shadow_bytes > 0 && !s->d_tiny) {   // fmg's first cycles lie below dc
         size_t off = s->tiny_at;
         RC(build_tiny(s, &off, st));
@@ -1692,6 +1703,7 @@ int solver_solve(mgp_solver* s, int which, mgp_array* phi, mgp_array* rhs, const
     }
     CK(cudaEventRecord(s->ev1, st));
     CK(cudaStreamSynchronize(st));
+    q.idle = true;
     if (status == MGP_OK && dstat)
         status = (dstat == DST_TIMEOUT) ? MGP_ETIMEOUT : MGP_EDIVERGED;
     if (status == MGP_OK && (s->flags & MGP_FLAG_REPORT_MAXITER) && !diverged && !(relres[iters] <= tol))
@@ -1732,7 +1744,12 @@ int solver_new(const mgp_box* valid, const mgp_geo* geo, const mgp_bdry* bc, int
     s->kind = kind;
     s->flags = flags;
     s->stream = stream;
-    const int rc = solver_build(s, valid, geo, bc, maxdepth_user);
+    int rc;
+    {
+        Quiesce q{stream};
+        rc = solver_build(s, valid, geo, bc, maxdepth_user);
+        q.idle = !rc;
+    }
     if (rc) {
         solver_free(s);
         return rc;
@@ -2418,9 +2435,8 @@ int lockstep_iteration(Plan& P, Lockstep* ls, int nd, int nu, cudaStream_t st) {
 
 Lockstep* lockstep_new() { return new Lockstep(); }
 
-void lockstep_free(Lockstep* ls) {
+void lockstep_free(Lockstep* ls) {   // nothing of its runs (Quiesce)
     if (!ls) return;
-    cudaDeviceSynchronize();
     if (ls->exec) cudaGraphExecDestroy(ls->exec);
     if (ls->capture) cudaStreamDestroy(ls->capture);
     dfree(ls->dev, nullptr);
@@ -2466,6 +2482,7 @@ int lockstep_vcycle(const std::vector<mgp_solver*>& ss, Lockstep* ls, mgp_array*
     const int n = (int)ss.size();
     const bool pairs = pairs_wanted && nd % 4 == 0 && nu % 4 == 0;
     if (maxiters < 0 || nb < 0) return set_err(MGP_EINVAL, "negative count");
+    Quiesce q{st};
     if (ls->ncap < n) {
         dfree(ls->norms, st);
         if (ls->h_norms) cudaFreeHost(ls->h_norms);
