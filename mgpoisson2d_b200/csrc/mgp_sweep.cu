@@ -254,7 +254,7 @@ __device__ __forceinline__ void sweep_stream(int total, int homog, double omega,
             load_fields(tiles[it ^ 1]);
         }
         if (any_side) {
-            if (any_plain(*L0.b, homog)) {
+            if (plain_sides(*L0.b, homog)) {
                 with_side<C>(warp, w, L0.nx, L0.ny, [&](auto L) {
                     L.place(w, *L0.g, *L0.b, homog, L0.nx, L0.ny, om, om1);
                     L.grab(s);

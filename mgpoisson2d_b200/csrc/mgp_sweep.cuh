@@ -234,17 +234,17 @@ __device__ __forceinline__ void corner_cell(T* S, const T* q, const int* x, cons
     S[x[1] + y[1]] = om * newphi + om1 * p;
 }
 
-// Whether a side's ghosts follow from three rows of the window beside it, or stay
-// as stored (SideLane::put); the others are filled from phi as a whole.
-__device__ __forceinline__ bool side_plain(const BCd& b, int homog, int sd) {
-    for (int s = 0; s < 4; ++s)
-        if (b.type[s] == T_PERIODIC) return false;
-    return b.type[sd] == T_NEUM || (b.type[sd] == T_DIRI && homog && b.mode[sd] != M_LAH);
-}
-__device__ __forceinline__ bool any_plain(const BCd& b, int homog) {
-    bool p = false;
-    for (int s = 0; s < 4; ++s) p = p || side_plain(b, homog, s);
-    return p;
+// The sides (bit S_*) whose ghosts follow from three rows of the window beside them, or
+// stay as stored (SideLane::put); the others' are filled from phi as a whole.
+__device__ __forceinline__ unsigned plain_sides(const BCd& b, int homog) {
+    unsigned m = 0;
+    bool periodic = false;
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+        periodic = periodic || b.type[s] == T_PERIODIC;
+        if (b.type[s] == T_NEUM || (b.type[s] == T_DIRI && homog && b.mode[s] != M_LAH)) m |= 1u << s;
+    }
+    return periodic ? 0u : m;
 }
 
 // The first sweep's ghosts of a side that is not plain, by the warp of side v (0-3:
@@ -257,7 +257,7 @@ __device__ __forceinline__ void start_ghosts(T* S, const Window& w, const DFT<T>
                                              int ny, int v) {
     const bool yside = v < 2, high = v & 1;
     const bool on = v == 0 ? w.yl : v == 1 ? w.yh : v == 2 ? w.xl : w.xh;
-    if (!on || side_plain(b, homog, (yside ? S_YLO : S_XLO) + (high ? 1 : 0))) return;
+    if (!on || (plain_sides(b, homog) >> ((yside ? S_YLO : S_XLO) + (high ? 1 : 0)) & 1u)) return;
     const DFLoadT<T> P{pin};
     const int lo = yside ? (w.xl ? -1 : w.ox) : w.oy, hi = yside ? (w.xh ? nx + 1 : w.wx1) : w.wy1;
     const int side = high ? (yside ? ny : nx) : -1;
@@ -298,7 +298,7 @@ struct SideLane {
     // depend on the other side's parity (cz).
     static constexpr bool hx = kHigh, hy = kY ? kHigh : !kHigh;
     bool on, plain, neum;      // the window holds the side; its ghosts follow from three rows; a Neumann side
-    bool all_plain, corner;    // so do every side's; the window holds the corner and it is to update
+    bool all_plain, any_plain, corner;   // so do every side's, some side's; the window holds the corner and it is to update
     int cz[4];
     bool ok[2], in[2];         // the lane's cells: edge cells to update, cells of the window
     int base;
@@ -314,7 +314,10 @@ struct SideLane {
         on = kY ? (kHigh ? w.yh : w.yl) : (kHigh ? w.xh : w.xl);
         const Per pr = periodic_of(b);
         const bool periodic = kY ? (kHigh ? pr.yh : pr.yl) : (kHigh ? pr.xh : pr.xl);
-        plain = side_plain(b, homog, sd);
+        const unsigned sides = plain_sides(b, homog);
+        plain = sides >> sd & 1u;
+        all_plain = sides == 15u;
+        any_plain = sides != 0u;
         neum = b.type[sd] == T_NEUM;
         const int ot = kY ? w.ox : w.oy, et = kY ? w.wx1 : w.wy1, nt = kY ? nx : ny;
         const int m = kHigh ? ((kY ? ny - w.oy : nx - w.ox) - 1) >> 1 : 0;   // the side's block, 0 at the low end
@@ -326,9 +329,6 @@ struct SideLane {
             ok[c] = in[c] && !periodic && t >= lo && t < hi;
         }
         base = C::P + 1 + (kY ? lane + m * C::P : lane * C::P + m);
-        all_plain = true;
-#pragma unroll
-        for (int s = 0; s < 4; ++s) all_plain = all_plain && side_plain(b, homog, s);
         corner = lane == 0 && (hx ? w.xh && !pr.xh : w.xl && !pr.xl) && (hy ? w.yh && !pr.yh : w.yl && !pr.yl);
 #pragma unroll
         for (int r = 0; r < 4; ++r)   // the direction along the side: the other sides' terms
@@ -661,7 +661,7 @@ __device__ __forceinline__ void sweep_window(T* s, T* strips, const DFT<T>& pin,
     Window w;
     w.set(2 * (bx * hx / gx), min(nx, 2 * ((bx + 1) * hx / gx)), 2 * (by * hy / gy), min(ny, 2 * ((by + 1) * hy / gy)),
           4 * K + 2, 4 * K, 4 * K + 2, 4 * K + 2, nx, ny);
-    const bool any_side = w.any(), grabs = any_side && any_plain(b, homog);
+    const bool any_side = w.any();
     const T idx = T(g.idx), idy = T(g.idy), om = T(omega), om1 = T(1.0 - omega);
     if (warp >= C::NI) {   // the counterpart of the blocks' loop below, with the same CTA barriers
         with_side<C>(warp - C::NI, w, nx, ny, [&](auto L) {
@@ -671,7 +671,7 @@ __device__ __forceinline__ void sweep_window(T* s, T* strips, const DFT<T>& pin,
                 start_ghosts<C>(s, w, pin, b, homog, nx, ny, warp - C::NI);
             }
             cta_sync();   // phi, the strips and these ghosts are in place
-            if (grabs) {
+            if (any_side && L.any_plain) {
                 L.grab(s);
                 cta_sync();
             }
@@ -738,6 +738,7 @@ __device__ __forceinline__ void sweep_window(T* s, T* strips, const DFT<T>& pin,
             k.xy[r][2] = c;
         }
     }
+    const bool grabs = any_side && plain_sides(b, homog) != 0u;   // (not before the loads are on their way)
     const unsigned mask = settle<C, false>(k, s, strips, w, kbx, kby, idx, idy, om, b, nx, ny);
     cta_sync();
     if (grabs) cta_sync();   // 2. the sides' warps have read what the first sweep's ghosts are made of
